@@ -221,12 +221,15 @@ std::vector<float> twiddles(int len) {
 }
 }  // namespace
 
+// Before set_variant or autotune: the patch kernel where it covers the geometry.
+constexpr int kAutoVariant = -1;
+
 struct risa_gb_backprojection {
    Geometry g;
    Params p;
    DevBuf a, b, ad, bd, t0;
    float norm = 0.f;
-   int variant = 0;
+   int variant = kAutoVariant;
    // asynchronous variants: pair-sinogram padding without / with the fused
    // mask's tile skipping, the pair buffer (grown outside stream capture) and
    // the device error flag of their bounded waits
@@ -235,6 +238,8 @@ struct risa_gb_backprojection {
    DevBuf rowbase, colbase;  // adjoint: (hi, lo) line starts [Pp][N]
    DevBuf adj;               // adjoint: slice-interleaved image copies (reserve_adjoint)
    DevBuf tile_win;          // staged variants: window start + origin per tile and angle
+   BPPatchPlan patch;        // the patch variant's angle order
+   DevBuf patch_angles;
    std::vector<float> a_host, b_host;  // the staged variants' kernel-parameter copies of a and b
    BPCfg cfg(bool fused_mask) const {
       BPCfg c;
@@ -258,6 +263,8 @@ struct risa_gb_backprojection {
       c.rowbase = rowbase.as<float2>();
       c.colbase = colbase.as<float2>();
       c.tile_win = tile_win.as<int2>();
+      c.patch = &patch;
+      c.patch_angles = patch_angles.as<BPPatchAngle>();
       c.adj_scratch = adj.p;
       c.adj_scratch_bytes = adj.bytes;
       return c;
@@ -268,13 +275,15 @@ struct risa_gb_backprojection {
    risa_gb_status reserve(int batch) {
       size_t need = 0;
       for (int v = 0; v < bp_variant_count(); ++v)
-         need = std::max(need, bp_pairs_bytes(v, batch, g.Pp, std::max(win_len[0], win_len[1])));
+         need = std::max(need, bp_pairs_bytes(v, batch, g.Pp, g.Dp, std::max(win_len[0], win_len[1])));
       if (need <= pairs.bytes) return RISA_GB_OK;
       RG_CUDA(cudaDeviceSynchronize());
       return pairs.alloc(need);
    }
    int variant_for(int batch, bool fused_mask) const {
-      return bp_pairs_bytes(variant, batch, g.Pp, win_len[fused_mask ? 1 : 0]) > pairs.bytes ? 0 : variant;
+      const int v = variant == kAutoVariant ? bp_patch_variant() : variant;
+      if (v == bp_patch_variant() && patch.angles.empty()) return 0;  // outside its range of angles or bins per pixel
+      return bp_pairs_bytes(v, batch, g.Pp, g.Dp, win_len[fused_mask ? 1 : 0]) > pairs.bytes ? 0 : v;
    }
 };
 
@@ -815,6 +824,11 @@ risa_gb_status risa_gb_backprojection_create(const risa_gb_geometry* gi, const r
       if (tiles * (size_t)h->g.Pp * sizeof(int2) <= ((size_t)256 << 20))
          RG_TRY(h->tile_win.upload(bp_tile_windows(t.a.data(), t.b.data(), t.ad.data(), t.bd.data(), t.t0.data(),
                                                    h->g.Pp, h->g.N)));
+      if (bp_patch_plan(t.a.data(), t.b.data(), t.ad.data(), t.bd.data(), t.t0.data(), h->g.Pp, scale, &h->patch))
+         RG_TRY(h->patch_angles.upload(h->patch.angles));
+      // frame-by-frame callers need no reserve(): one slice quad (16 MB at 1024 x 1024)
+      const size_t quad = bp_quads_bytes(4, h->g.Pp, h->g.Dp);
+      if (!h->patch.angles.empty() && quad <= ((size_t)64 << 20)) RG_TRY(h->pairs.alloc(quad));
       RG_TRY(h->rowbase.upload(bp_line_starts(t.t0.data(), t.bd.data(), h->g.Pp, h->g.N)));
       RG_TRY(h->colbase.upload(bp_line_starts(t.t0.data(), t.ad.data(), h->g.Pp, h->g.N)));
    }
@@ -1067,10 +1081,9 @@ static cudaError_t engine_filter_bp(risa_gb_fbp* h, float* par, float* img, int 
    const FilterCfg fc = h->filt->cfg();
    const int v = h->bp->variant_for(batch, fused);
    BPCfg c = h->bp->cfg(fused);
-   const int slices = bp_variant_pair_slices(v);
    cudaError_t e;
-   if (slices > 0 && filter_pairs_supported(fc)) {
-      e = launch_filter_pairs(par, batch, fc, PairsOut{c.pairs, slices, c.win_lo, c.win_len}, st);
+   if (bp_variant_layout(v) != kLayoutNone && filter_pairs_supported(fc)) {
+      e = launch_filter_pairs(par, batch, fc, PairsOut{c.pairs, bp_variant_pair_slices(v), c.win_lo, c.win_len}, st);
       c.prefilled = true;
    } else {
       e = launch_filter(par, batch, fc, st);
@@ -1107,7 +1120,7 @@ static cudaError_t engine_streaming(risa_gb_fbp* h, const uint16_t* raw, int pla
 static bool two_lanes(const risa_gb_fbp* h, int batch) {
    if (h->lanes < 2 || h->p.normalize || h->p.interp != RISA_GB_INTERP_LINEAR) return false;
    const bool fused = h->p.masking && !h->p.normalize;
-   return bp_variant_pair_slices(h->bp->variant_for(batch, fused)) > 0 && filter_pairs_supported(h->filt->cfg());
+   return bp_variant_layout(h->bp->variant_for(batch, fused)) != kLayoutNone && filter_pairs_supported(h->filt->cfg());
 }
 
 // The second pair buffer, the capture lane (highest stream priority) and its

@@ -28,7 +28,7 @@ namespace {
 
 // Linear interpolation variants: kernel kind, slices per CTA and angles per
 // chunk. The nearest-neighbour modes always use the plain tile kernel.
-enum VariantKind { kTile, kPairs, kAsync, kAsyncPacked };
+enum VariantKind { kTile, kPairs, kAsync, kAsyncPacked, kPatch };
 struct BPVariant {
    int kind, slices, achunk, ppt;  // ppt: pixels per thread of the staged kernels
    const char* name;
@@ -57,6 +57,7 @@ constexpr BPVariant kVariants[] = {
     {kAsync, 4, 8, 4, "staged_cp_s4_a8_p4", true},
     {kAsync, 4, 16, 4, "staged_cp_s4_a16_p4", true},
     {kAsync, 2, 16, 4, "staged_cp_s2_a16_p4", true},
+    {kPatch, 0, 8, 4, "patch_2x2"},
 };
 constexpr int kNumVariants = sizeof(kVariants) / sizeof(kVariants[0]);
 
@@ -1010,6 +1011,12 @@ size_t bp_adjoint_scratch_bytes(int batch, int N) {
    return batch <= 0 ? 0 : sizeof(float) * 2 * 8 * (size_t)((batch + 7) / 8) * N * N;
 }
 
+int bp_patch_variant() {
+   int v = 0;
+   while (kVariants[v].kind != kPatch) ++v;
+   return v;
+}
+
 int bp_variant_count() { return kNumVariants; }
 const char* bp_variant_name(int v) {
    return (v >= 0 && v < kNumVariants) ? kVariants[v].name : "invalid";
@@ -1021,9 +1028,16 @@ int bp_variant_pair_slices(int variant) {
    return (v.kind == kAsync || v.kind == kAsyncPacked) ? v.slices : 0;
 }
 
-size_t bp_pairs_bytes(int variant, int batch, int Pp, int win_len) {
+BPLayout bp_variant_layout(int variant) {
+   if (variant < 0 || variant >= kNumVariants) return kLayoutNone;
+   const int k = kVariants[variant].kind;
+   return k == kPatch ? kLayoutQuads : k == kAsync || k == kAsyncPacked ? kLayoutPairs : kLayoutNone;
+}
+
+size_t bp_pairs_bytes(int variant, int batch, int Pp, int Dp, int win_len) {
    if (variant < 0 || variant >= kNumVariants || batch <= 0) return 0;
    const BPVariant& v = kVariants[variant];
+   if (v.kind == kPatch) return bp_quads_bytes(batch, Pp, Dp);
    if (v.kind != kAsync && v.kind != kAsyncPacked) return 0;
    const size_t groups = (size_t)(batch + v.slices - 1) / v.slices;
    return groups * v.slices * (size_t)Pp * (size_t)win_len * sizeof(float2);
@@ -1100,7 +1114,7 @@ cudaError_t launch_backprojection(const float* sino, float* img, int batch, cons
                                   int variant, cudaStream_t st) {
    if (batch <= 0) return cudaSuccess;
    const bool staged = cfg.interp == RISA_GB_INTERP_LINEAR && variant >= 0 && variant < kNumVariants &&
-                       (kVariants[variant].kind == kAsync || kVariants[variant].kind == kAsyncPacked);
+                       bp_variant_layout(variant) != kLayoutNone;
    if (!staged && cfg.mid_event) {  // no staging pass: it takes no time
       cudaError_t e = cudaEventRecord(cfg.mid_event, st);
       if (e != cudaSuccess) return e;
@@ -1109,6 +1123,7 @@ cudaError_t launch_backprojection(const float* sino, float* img, int batch, cons
        kVariants[variant].kind == kTile)
       return launch_interp<32, 32, 4, 32>(sino, img, batch, cfg, st);
    const BPVariant& v = kVariants[variant];
+   if (v.kind == kPatch) return launch_bp_patch(sino, img, batch, cfg, st);
    if (v.kind == kAsync || v.kind == kAsyncPacked) {
       const bool pk = v.kind == kAsyncPacked;
       const int ach = v.achunk;

@@ -1,0 +1,558 @@
+// Linear pixel-driven backprojection of slice batches, 2 x 2 pixel patches per
+// thread (the batch form of backProjectLinear, Backprojection.cu:238-271).
+//
+// What bounds a linear backprojection is the shared-memory data path: a
+// (midpoint, difference) record per pixel, angle and slice is 8 B of every
+// 128 B/clk (bp_linear_async, k_bp.cu: 23.8 ms per 512 slices of 1024 x 1024
+// -> 512^2, 0.90 of that bound). Here a thread owns a 2 x 2 pixel patch of 4
+// (or 8) slices and reads each detector bin its patch touches once: with
+// A = |a|, B = |b| (bins per pixel along x and y) the patch spans A + B bins,
+// so floor(A + B) + 3 bins serve 4 pixels -- 5 loads of 16 B at 2 bins per
+// pixel and 4 at 1, where the records took 8.
+//
+//   * A pixel at offset o from the patch's lowest coordinate k + g (g in [0, 1])
+//     reads the three bins m .. m + 2 around g + o, m = floor(o), with the hat
+//     weights of linear interpolation max(0, 1 - |g + o - m - 1 -+ 1|) and
+//     1 - |g + o - m - 1|; one of the outer two is 0. m is the same for every
+//     thread of an angle, so the bins are registers with compile-time indices:
+//     the angles are sorted by (sign of a, sign of b, m of the three offset
+//     pixels) and every chunk of angles runs the loop instantiated for its class.
+//     A negative a or b mirrors the patch: the accumulators are exchanged once,
+//     where the sign changes.
+//   * The rows are staged as they are, four slices to a 16-byte entry
+//     ([slice quad][angle][bin][4]): no (mid, diff) pairs, so half the bytes in
+//     global memory and in the staging copies, and no padding: bins outside the
+//     detector are the zeros a tensor-map copy fills in.
+//   * A warp is QL slice quads x 32 / QL patches. With QL = 8 the 8 lanes of a
+//     128-bit load phase read one bin of 8 quads, whose rows lie an odd number
+//     of entries apart: conflict-free whatever the bins per pixel.
+//
+// One warp of the CTA forms the windows and fills NST shared-memory stages of
+// ACH angles with cp.async.bulk.tensor (one box per angle: the tile's bins of
+// all the CTA's quads), each completing on its stage's `full` mbarrier; the other
+// warps release a stage on its `empty` mbarrier. With the refill done by one of
+// the working warps, as in bp_linear_async, the same loop took 18.0 ms instead
+// of 15.8 (512 slices of 1024 x 1024 -> 512^2). Waits are bounded; on timeout the
+// CTA records the error and leaves without output.
+#include <cuda.h>
+
+#include <algorithm>
+#include <cmath>
+#include <cstring>
+
+#include "async_copy.h"
+#include "f32x2.cuh"
+#include "kernels.h"
+#include "risa_gb300.h"
+
+namespace risa_gb {
+
+namespace {
+constexpr int kTile = 16;  // pixels per tile side
+constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23
+constexpr int kMagicBits = 0x4B400000;
+
+struct PatchArgs {
+   const BPPatchAngle* ang;  // [Pp] in plan order
+   const int* nonfinite;     // per slice quad, or nullptr
+   const float4* quads;      // [quad][angle][bin] (the rows the tensor map covers)
+   float* img;
+   int* err;
+   int N, Pp, Dp, batch, n_quads, wlen;
+   float norm, mask_value;
+   int masking;
+};
+struct PatchPlanParam {
+   float A[kPatchAngles], B[kPatchAngles];
+   uint32_t seg[kPatchMaxSegs];
+   int n_segs;
+};
+
+typedef unsigned long long u64;
+
+__device__ __forceinline__ ulonglong2 lds_quad(uint32_t addr) {
+   ulonglong2 v;
+   asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(addr));
+   return v;
+}
+
+// The same load for the lanes with r > 0, zeros elsewhere: a load phase whose
+// lanes all skip it costs no wavefront.
+__device__ __forceinline__ ulonglong2 lds_quad_if(uint32_t addr, float r) {
+   ulonglong2 v;
+   asm volatile(
+       "{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %3, 0f00000000;\n\tmov.u64 %0, 0;\n\tmov.u64 %1, 0;\n\t"
+       "@p ld.shared.v2.u64 {%0, %1}, [%2];\n\t}"
+       : "=&l"(v.x), "=&l"(v.y)
+       : "r"(addr), "f"(r));
+   return v;
+}
+
+__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z) {
+   asm volatile(
+       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];" ::
+           "r"(async::smem_u32(dst)),
+       "l"(map), "r"(async::smem_u32(bar)), "r"(x), "r"(y), "r"(z)
+       : "memory");
+}
+
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(async::smem_u32(bar)) : "memory");
+}
+
+// One angle of one patch: addr is the shared address of bin k of this thread's
+// first quad, f = g - 1/2.
+template <int MA, int MB, int MAB, int SQ, bool PRED>
+__device__ __forceinline__ void patch_angle(uint32_t addr, uint32_t qstep, float f, float A, float B,
+                                            u64 (&acc)[SQ][2][4]) {
+   constexpr int m[4] = {0, MA, MB, MAB};
+   // coordinate of each pixel relative to its middle bin m + 1, in [-1, 1]
+   const float r1 = (f + A) - (MA + 0.5f), r2 = (f + B) - (MB + 0.5f), r3 = (f + (A + B)) - (MAB + 0.5f);
+   const float r[4] = {0.f, r1, r2, r3};
+   float w[4][3];
+   w[0][0] = 0.5f - f;  // the lowest pixel lies between bins 0 and 1
+   w[0][1] = 0.5f + f;
+   w[0][2] = 0.f;
+#pragma unroll
+   for (int p = 1; p < 4; ++p) {
+      w[p][0] = __saturatef(-r[p]);
+      w[p][1] = 1.f - fabsf(r[p]);
+      w[p][2] = __saturatef(r[p]);
+   }
+#pragma unroll
+   for (int e = 0; e < MAB + 3; ++e) {
+      ulonglong2 q[SQ];
+#pragma unroll
+      for (int s = 0; s < SQ; ++s) {
+         const uint32_t at = addr + (uint32_t)s * qstep + (uint32_t)e * 16u;
+         q[s] = PRED && e == MAB + 2 ? lds_quad_if(at, r3) : lds_quad(at);
+      }
+#pragma unroll
+      for (int p = 0; p < 4; ++p) {
+         const int d = e - m[p];
+         if (d < 0 || d > (p == 0 ? 1 : 2)) continue;
+         const u64 w2 = f2_pack(w[p][d], w[p][d]);
+#pragma unroll
+         for (int s = 0; s < SQ; ++s) {
+            acc[s][0][p] = f2_fma(w2, q[s].x, acc[s][0][p]);
+            acc[s][1][p] = f2_fma(w2, q[s].y, acc[s][1][p]);
+         }
+      }
+   }
+}
+
+template <int SQ>
+__device__ __forceinline__ void flip(u64 (&acc)[SQ][2][4], bool x, bool y) {
+#pragma unroll
+   for (int s = 0; s < SQ; ++s)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+         u64* v = acc[s][h];
+         u64 t;
+         if (x) t = v[0], v[0] = v[1], v[1] = t, t = v[2], v[2] = v[3], v[3] = t;
+         if (y) t = v[0], v[0] = v[2], v[2] = t, t = v[1], v[1] = v[3], v[3] = t;
+      }
+}
+
+// The tile of a CTA whose rows hold an infinity or a NaN, by the general two-bin
+// rule (the patches above also multiply a third bin by a zero weight, which
+// would carry it one pixel further): one pixel per thread and step, straight
+// from global memory.
+template <int Q>
+__device__ __noinline__ void patch_general_tile(const PatchArgs& g, int q0, int n_threads) {
+   const int N = g.N, x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile;
+   const float c = 0.5f * (float)(N - 1), lim = (float)N * (float)N * 0.25f;
+   for (int i = threadIdx.x; i < kTile * kTile * Q; i += n_threads) {
+      const int x = x0 + i % kTile, y = y0 + (i / kTile) % kTile, q = q0 + i / (kTile * kTile);
+      if (x >= N || y >= N || q >= g.n_quads) continue;
+      const float dx = (float)x - c, dy = (float)y - c;
+      const bool out = g.masking && dx * dx + dy * dy > lim;
+      float acc[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int a = 0; a < g.Pp && !out; ++a) {
+         const BPPatchAngle t = g.ang[a];
+         const double s = t.t0 + (double)x * t.a + (double)y * t.b;
+         const double fl = floor(s);
+         const float f = (float)(s - fl) - 0.5f;
+         const int k = (int)fl;
+         const float4* row = g.quads + ((size_t)q * g.Pp + t.index) * g.Dp;
+         const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+         const float4 u = k >= 0 && k < g.Dp ? __ldg(row + k) : z, v = k + 1 >= 0 && k + 1 < g.Dp ? __ldg(row + k + 1) : z;
+         acc[0] = fmaf(f, v.x - u.x, acc[0] + 0.5f * (u.x + v.x));
+         acc[1] = fmaf(f, v.y - u.y, acc[1] + 0.5f * (u.y + v.y));
+         acc[2] = fmaf(f, v.z - u.z, acc[2] + 0.5f * (u.z + v.z));
+         acc[3] = fmaf(f, v.w - u.w, acc[3] + 0.5f * (u.w + v.w));
+      }
+      for (int j = 0; j < 4; ++j)
+         if (4 * q + j < g.batch)
+            g.img[((size_t)(4 * q + j) * N + y) * N + x] = out ? g.mask_value : acc[j] * g.norm;
+   }
+}
+
+template <int SQ, int QL, int ACH, int NST, int MINB, bool PRED>
+__global__ void __launch_bounds__(64 * QL + 32, MINB)
+    bp_patch(const __grid_constant__ CUtensorMap map, const __grid_constant__ PatchArgs g, const __grid_constant__ PatchPlanParam pp) {
+   constexpr int NW = 2 * QL, Q = QL * SQ;  // consumer warps, slice quads of the CTA
+   extern __shared__ __align__(128) unsigned char smem_raw[];
+   __shared__ uint64_t full[NST], empty[NST];
+   __shared__ float4 s_rel[NST][ACH / 4];
+   __shared__ volatile int s_fail;
+
+   const int N = g.N;
+   const int x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile, q0 = blockIdx.z * Q;
+   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+   if (g.nonfinite) {
+      bool bad = false;
+#pragma unroll 1
+      for (int i = q0; i < min(q0 + Q, g.n_quads); ++i) bad |= __ldg(g.nonfinite + i) != 0;
+      if (bad) {
+         patch_general_tile<Q>(g, q0, (NW + 1) * 32);
+         return;
+      }
+   }
+   const float c = 0.5f * (float)(N - 1);
+   const float lim = (float)N * (float)N * 0.25f;
+   // whether some pixel of the block lies inside the circle (exact, as in bp_linear_async)
+   auto inside = [&](int xa, int ya, int w, int h) {
+      const float nx = fminf(fmaxf(c, (float)xa), (float)(xa + w - 1)) - c;
+      const float ny = fminf(fmaxf(c, (float)ya), (float)(ya + h - 1)) - c;
+      return !g.masking || nx * nx + ny * ny <= lim;
+   };
+   // a consumer warp's pixel block in the tile
+   constexpr int BW = QL == 8 ? 4 : QL == 1 ? 16 : 8, BH = 128 / QL / BW;
+   auto block_x = [](int w) { return w % (kTile / BW) * BW; };
+   auto block_y = [](int w) { return w / (kTile / BW) * BH; };
+
+   const bool tile_live = inside(x0, y0, kTile, kTile);
+   const uint32_t pitch = (uint32_t)g.wlen * 16u;     // bytes between the rows of two quads
+   const uint32_t angle_bytes = pitch * (uint32_t)Q;  // one angle's box
+   if (threadIdx.x == 0) {
+      int live_warps = 0;
+      for (int w = 0; w < NW; ++w) live_warps += inside(x0 + block_x(w), y0 + block_y(w), BW, BH);
+      for (int i = 0; i < NST; ++i) {
+         async::mbar_init(&full[i], 1);
+         async::mbar_init(&empty[i], max(live_warps, 1));
+      }
+      s_fail = 0;
+      async::mbar_init_fence();
+   }
+   __syncthreads();
+
+   if (warp == NW) {
+      // ---- producer: windows and copies of every chunk
+      int st = 0;
+      uint32_t round = 0;
+      for (int si = 0; tile_live && si < pp.n_segs && !s_fail; ++si) {
+         const uint32_t d = pp.seg[si];
+         const int pos = (int)(d & 0xFFFu), n = (int)((d >> 12) & 0xFFFu);
+         const int cx = x0 + ((d >> 28) & 1u ? kTile - 1 : 0), cy = y0 + ((d >> 29) & 1u ? kTile - 1 : 0);
+         for (int a0 = 0; a0 < n; a0 += ACH) {
+            const int na = min(ACH, n - a0);
+            float rel = 0.f;
+            int w0 = 0, ang = 0;
+            if (lane < na) {
+               // the lowest coordinate of the tile's pixels
+               const BPPatchAngle t = g.ang[pos + a0 + lane];
+               const double base = t.t0 + (double)cx * t.a + (double)cy * t.b;
+               const double fl = floor(base);
+               w0 = (int)fl;
+               rel = (float)(base - fl);
+               ang = t.index;
+            }
+            if (round > 0 && !__all_sync(~0u, async::mbar_wait(&empty[st], (round - 1) & 1u, g.err, 5))) {
+               s_fail = 1;
+               break;
+            }
+            if (lane < ACH) reinterpret_cast<float*>(&s_rel[st][0])[lane] = rel - 0.5f;
+            __syncwarp();
+            if (lane == 0) async::mbar_arrive_expect_tx(&full[st], (uint32_t)na * angle_bytes);
+            __syncwarp();
+            if (lane < na)
+               tma_load_3d(smem_raw + (size_t)(st * ACH + lane) * angle_bytes, &map, &full[st], 4 * w0, ang, q0);
+            if (++st == NST) st = 0, ++round;
+         }
+      }
+      // the copies still in flight land before the CTA ends
+      for (int i = 0; i < NST; ++i) {
+         const uint32_t issued = round + (i < st ? 1u : 0u);
+         if (issued > 0) async::mbar_wait_quiet(&full[i], (issued - 1) & 1u);
+      }
+      __syncthreads();
+      return;
+   }
+
+   // ---- consumers
+   const int ql = lane % QL, pl = lane / QL;
+   // this thread's patch in the warp's block: the patches of a load phase are neighbours
+   int px, py;
+   if (QL == 8) px = pl & 1, py = pl >> 1;
+   else if (QL == 4) px = pl & 3, py = pl >> 2;
+   else if (QL == 2) px = (pl & 1) + ((pl >> 1) & 2), py = ((pl >> 1) & 1) + ((pl >> 2) & 2);
+   else px = (pl & 3) + ((pl >> 1) & 4), py = ((pl >> 2) & 1) + ((pl >> 3) & 2);
+   const int xp = block_x(warp) + 2 * px, yp = block_y(warp) + 2 * py;  // patch origin in the tile
+
+   u64 acc[SQ][2][4];
+#pragma unroll
+   for (int s = 0; s < SQ; ++s)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+         for (int p = 0; p < 4; ++p) acc[s][h][p] = 0ull;
+
+   const uint32_t sbase = async::smem_u32(smem_raw) + (uint32_t)ql * pitch - ((uint32_t)kMagicBits << 4);
+   if (tile_live && inside(x0 + block_x(warp), y0 + block_y(warp), BW, BH)) {
+      uint32_t signs = 0;  // bit 0: x mirrored, bit 1: y mirrored
+      int st = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int si = 0; si < pp.n_segs && ok; ++si) {
+         const uint32_t d = pp.seg[si];
+         const int pos = (int)(d & 0xFFFu), n = (int)((d >> 12) & 0xFFFu);
+         const uint32_t sg = d >> 28;
+         if (sg != signs) {
+            flip<SQ>(acc, (sg ^ signs) & 1u, ((sg ^ signs) >> 1) & 1u);
+            signs = sg;
+         }
+         const float fx = (float)((sg & 1u) ? kTile - 2 - xp : xp), fy = (float)((sg & 2u) ? kTile - 2 - yp : yp);
+         auto run = [&](auto cls) {
+            constexpr int CL = decltype(cls)::value;
+#pragma unroll 1
+            for (int a0 = 0; a0 < n; a0 += ACH) {
+               if (!async::mbar_wait(&full[st], phase, g.err, 5)) {
+                  ok = false;
+                  break;
+               }
+               const uint32_t stage = sbase + (uint32_t)(st * ACH) * angle_bytes;
+               auto angle = [&](int ai, float rel) {
+                  const float A = pp.A[pos + a0 + ai], B = pp.B[pos + a0 + ai];
+                  const float tm = fmaf(fy, B, fmaf(fx, A, rel));
+                  const float v = tm + kMagic;
+                  const float f = tm - (v - kMagic);
+                  const uint32_t addr = stage + (uint32_t)ai * angle_bytes + ((uint32_t)__float_as_int(v) << 4);
+                  patch_angle<(CL >> 4) & 1, (CL >> 3) & 1, CL & 3, SQ, PRED>(addr, pitch * QL, f, A, B, acc);
+               };
+               if (n - a0 >= ACH) {
+#pragma unroll 1
+                  for (int a4 = 0; a4 < ACH; a4 += 4) {
+                     const float4 r4 = s_rel[st][a4 >> 2];
+                     angle(a4, r4.x);
+                     angle(a4 + 1, r4.y);
+                     angle(a4 + 2, r4.z);
+                     angle(a4 + 3, r4.w);
+                  }
+               } else {
+#pragma unroll 1
+                  for (int ai = 0; ai < n - a0; ++ai) angle(ai, reinterpret_cast<const float*>(&s_rel[st][0])[ai]);
+               }
+               __syncwarp();
+               if (lane == 0) mbar_arrive(&empty[st]);
+               if (++st == NST) st = 0, phase ^= 1u;
+            }
+         };
+         switch ((d >> 24) & 15u) {  // bits of the class: MA << 4 | MB << 3 | MAB
+            case 0: run(std::integral_constant<int, 0>{}); break;
+            case 1: run(std::integral_constant<int, 1>{}); break;
+            case 2: run(std::integral_constant<int, 8 + 1>{}); break;
+            case 3: run(std::integral_constant<int, 8 + 2>{}); break;
+            case 4: run(std::integral_constant<int, 16 + 1>{}); break;
+            case 5: run(std::integral_constant<int, 16 + 2>{}); break;
+            default: run(std::integral_constant<int, 16 + 8 + 2>{}); break;
+         }
+      }
+      if (!ok) s_fail = 1;
+      flip<SQ>(acc, signs & 1u, (signs >> 1) & 1u);
+   }
+   __syncthreads();
+   if (s_fail) return;  // a wait gave up (recorded in g.err): no output
+#pragma unroll
+   for (int s = 0; s < SQ; ++s)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+         for (int p = 0; p < 4; ++p) {
+            float v[2];
+            f2_unpack(acc[s][h][p], v[0], v[1]);
+            const int x = x0 + xp + (p & 1), y = y0 + yp + (p >> 1);
+            if (x >= N || y >= N) continue;
+            bool out = false;
+            if (g.masking) {
+               const float dx = (float)x - c, dy = (float)y - c;
+               out = dx * dx + dy * dy > lim;
+            }
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+               const int sl = 4 * (q0 + s * QL + ql) + 2 * h + j;
+               if (sl < g.batch) g.img[((size_t)sl * N + y) * N + x] = out ? g.mask_value : v[j] * g.norm;
+            }
+         }
+}
+
+// Staged rows from a plain sinogram: quads[q][angle][bin] = slices 4q .. 4q + 3
+// of the bin, 0 past the batch. nonfinite[q] (zero before the launch) is set
+// where a row of the quad holds an infinity or a NaN.
+__global__ void __launch_bounds__(256) bp_quads_fill(const float* __restrict__ sino, float4* __restrict__ quads,
+                                                     int* __restrict__ nonfinite, int batch, int Pp, int Dp) {
+   const int k = blockIdx.x * 256 + threadIdx.x;
+   if (k >= Dp) return;
+   const int ang = blockIdx.y, q = blockIdx.z;
+   float v[4];
+#pragma unroll
+   for (int j = 0; j < 4; ++j)
+      v[j] = 4 * q + j < batch ? __ldg(sino + ((size_t)(4 * q + j) * Pp + ang) * Dp + k) : 0.f;
+   quads[((size_t)q * Pp + ang) * Dp + k] = make_float4(v[0], v[1], v[2], v[3]);
+   if (!(isfinite(v[0]) && isfinite(v[1]) && isfinite(v[2]) && isfinite(v[3]))) nonfinite[q] = 1;
+}
+
+using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+EncodeTiled encode_fn() {
+   static const EncodeTiled fn = [] {
+      void* p = nullptr;
+      cudaDriverEntryPointQueryResult q;
+      if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
+              cudaSuccess &&
+          q == cudaDriverEntryPointSuccess)
+         return reinterpret_cast<EncodeTiled>(p);
+      return EncodeTiled(nullptr);
+   }();
+   return fn;
+}
+
+// Staged row of one angle and quad, in 16-byte entries: the bins a 16-pixel
+// tile reaches, rounded up so that the rows of the QL quads of a load phase
+// start in different banks (QL rows 8 / QL entries apart modulo a bank row) and
+// an angle's box is a multiple of 128 bytes.
+int patch_wlen(float scale, int ql) {
+   const int need = (int)std::floor((kTile - 2) * 1.41421357 * (double)scale + 1.01) + 3 +
+                    std::min(2, (int)std::floor(1.41421357 * (double)scale));
+   const int step = 8 / ql;  // 1, 2, 4, 8
+   int w = need;
+   if (step == 8) return (need + 7) / 8 * 8;
+   while (w % step || (w / step) % 2 == 0) ++w;  // an odd multiple of step
+   return w;
+}
+
+size_t patch_smem(int sq, int ql, int ach, int nst, int wlen) {
+   return (size_t)nst * ach * sq * ql * wlen * 16;
+}
+
+template <int SQ, int QL, int MINB, bool PRED = false>
+cudaError_t launch_patch(const PatchArgs& args, const PatchPlanParam& pp, float scale, cudaStream_t st) {
+   constexpr int ACH = 8, NST = 2;
+   PatchArgs a = args;
+   a.wlen = patch_wlen(scale, QL);
+   const size_t smem = patch_smem(SQ, QL, ACH, NST, a.wlen);
+   if (4 * a.wlen > 256 || smem > 220 * 1024) return cudaErrorInvalidConfiguration;
+   EncodeTiled enc = encode_fn();
+   if (!enc) return cudaErrorNotSupported;
+   CUtensorMap map;
+   const cuuint64_t dims[3] = {(cuuint64_t)a.Dp * 4, (cuuint64_t)a.Pp, (cuuint64_t)a.n_quads};
+   const cuuint64_t strides[2] = {(cuuint64_t)a.Dp * 16, (cuuint64_t)a.Pp * a.Dp * 16};
+   const cuuint32_t box[3] = {(cuuint32_t)a.wlen * 4, 1, (cuuint32_t)(SQ * QL)};
+   const cuuint32_t estr[3] = {1, 1, 1};
+   if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float4*>(a.quads), dims, strides, box, estr,
+           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return cudaErrorInvalidValue;
+   auto kern = bp_patch<SQ, QL, ACH, NST, MINB, PRED>;
+   if (smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+   }
+   const int t = (a.N + kTile - 1) / kTile;
+   kern<<<dim3(t, t, (a.n_quads + SQ * QL - 1) / (SQ * QL)), 64 * QL + 32, smem, st>>>(map, a, pp);
+   return cudaGetLastError();
+}
+}  // namespace
+
+bool bp_patch_plan(const float* a, const float* b, const double* ad, const double* bd, const double* t0, int Pp,
+                   float scale, BPPatchPlan* plan) {
+   plan->angles.clear();
+   if (Pp < 1 || Pp > kPatchAngles || !(scale > 0.f) || scale > 2.f) return false;
+   struct Key {
+      int group, index;
+   };
+   std::vector<Key> keys(Pp);
+   for (int i = 0; i < Pp; ++i) {
+      const float A = std::fabs(a[i]), B = std::fabs(b[i]);
+      if (!(A <= 2.f && B <= 2.f && A + B < 3.f) || !std::isfinite(t0[i])) return false;
+      const int ma = A >= 1.f, mb = B >= 1.f;
+      // the offset lies in [m, m + 1]; at an integer either end serves
+      const int mab = std::min({(int)(A + B), 2, ma + mb + 1});
+      if (A + B - (float)mab > 1.f) return false;
+      const int cls = ma == 0 && mb == 0 ? mab : 1 + ma * 2 + mb + (ma + mb == 1 ? (ma ? 1 : 0) + (mab - 1) : 2);
+      keys[i] = {((a[i] < 0.f ? 1 : 0) + (b[i] < 0.f ? 2 : 0)) * 16 + cls, i};
+   }
+   std::stable_sort(keys.begin(), keys.end(), [](const Key& x, const Key& y) { return x.group < y.group; });
+   for (int i = 0; i < Pp;) {
+      int n = 1;
+      while (i + n < Pp && keys[i + n].group == keys[i].group) ++n;
+      plan->segs.push_back((uint32_t)i | (uint32_t)n << 12 | (uint32_t)(keys[i].group & 15) << 24 |
+                           (uint32_t)(keys[i].group >> 4) << 28);
+      i += n;
+   }
+   for (const Key& k : keys) {
+      plan->angles.push_back(BPPatchAngle{t0[k.index], ad[k.index], bd[k.index], k.index, 0});
+      plan->A.push_back(std::fabs(a[k.index]));
+      plan->B.push_back(std::fabs(b[k.index]));
+   }
+   return true;
+}
+
+// The rows, then one non-finite flag per quad.
+size_t bp_quads_bytes(int batch, int Pp, int Dp) {
+   if (batch <= 0) return 0;
+   const size_t quads = (size_t)((batch + 3) / 4);
+   return sizeof(float4) * quads * Pp * Dp + sizeof(int) * quads;
+}
+
+cudaError_t launch_bp_patch(const float* sino, float* img, int batch, const BPCfg& cfg, cudaStream_t st) {
+   if (!cfg.patch || cfg.patch->angles.empty() || !cfg.patch_angles || !cfg.err) return cudaErrorInvalidConfiguration;
+   if (!cfg.pairs || bp_quads_bytes(batch, cfg.Pp, cfg.Dp) > cfg.pairs_bytes) return cudaErrorInvalidValue;
+   const int nq = (batch + 3) / 4;
+   float4* quads = static_cast<float4*>(cfg.pairs);
+   int* flags = reinterpret_cast<int*>(quads + (size_t)nq * cfg.Pp * cfg.Dp);
+   PatchArgs a;
+   a.ang = cfg.patch_angles;
+   a.nonfinite = cfg.prefilled ? nullptr : flags;  // the engine's rows are finite: logarithms of clamped counts
+   a.quads = quads;
+   a.img = img;
+   a.err = cfg.err;
+   a.N = cfg.N;
+   a.Pp = cfg.Pp;
+   a.Dp = cfg.Dp;
+   a.batch = batch;
+   a.n_quads = nq;
+   a.norm = cfg.norm;
+   a.mask_value = cfg.mask_value;
+   a.masking = cfg.masking;
+   PatchPlanParam pp;
+   std::memcpy(pp.A, cfg.patch->A.data(), sizeof(float) * cfg.Pp);
+   std::memcpy(pp.B, cfg.patch->B.data(), sizeof(float) * cfg.Pp);
+   std::memcpy(pp.seg, cfg.patch->segs.data(), sizeof(uint32_t) * cfg.patch->segs.size());
+   pp.n_segs = (int)cfg.patch->segs.size();
+   cudaError_t e = cudaSuccess;
+   if (!cfg.prefilled) {
+      if ((e = cudaMemsetAsync(flags, 0, sizeof(int) * nq, st)) != cudaSuccess) return e;
+      bp_quads_fill<<<dim3((cfg.Dp + 255) / 256, cfg.Pp, nq), 256, 0, st>>>(sino, quads, flags, batch, cfg.Pp, cfg.Dp);
+      if ((e = cudaGetLastError()) != cudaSuccess) return e;
+   }
+   if (cfg.mid_event && (e = cudaEventRecord(cfg.mid_event, st)) != cudaSuccess) return e;
+   // Slice quads per thread (SQ) and per load phase (QL) by the batch and the
+   // bins per pixel. Up to 1.25 bins per pixel the neighbouring patches of a
+   // phase fall in different banks as they are, so few quads per phase do as
+   // well as eight and leave smaller CTAs: 16 slices of 1024^2 at 1 bin per pixel
+   // 2.19 ms with (2, 2), 2.77 with (1, 4). Above, patches collide (64 slices at
+   // 1.5: (2, 2) 2.35 ms, (2, 8) 1.72) and a phase takes as many quads as the
+   // batch has. All forms add the same terms in the same order: same bits.
+   if (nq == 1) return launch_patch<1, 1, 10>(a, pp, cfg.scale, st);
+   if (nq == 2) return launch_patch<1, 2, 6>(a, pp, cfg.scale, st);
+   if (cfg.scale <= 1.25f) return launch_patch<2, 2, 3>(a, pp, cfg.scale, st);
+   if (nq <= 4) return launch_patch<1, 4, 3>(a, pp, cfg.scale, st);
+   // 16 quads per CTA share a pixel's weights between twice the slices: 1.69
+   // times the time of 8 quads (2.11 against 1.25 ms, 512^2 x 1024 angles)
+   if (169 * ((nq + 15) / 16) <= 100 * ((nq + 7) / 8)) return launch_patch<2, 8, 1, true>(a, pp, cfg.scale, st);
+   return launch_patch<1, 8, 1>(a, pp, cfg.scale, st);
+}
+}  // namespace risa_gb

@@ -382,6 +382,61 @@ __global__ void __launch_bounds__(r16_threads<LEN>(), 512 / r16_threads<LEN>())
    }
 }
 
+// As filter_rows_r16_pairs, writing the filtered rows of two slices into the
+// patch backprojection's slice quads, quads[s / 4][angle][bin][s % 4]: the
+// values go straight from the last pass's registers (8 bytes per bin; the two
+// row pairs of a quad and angle are neighbouring groups, whose halves of each
+// entry meet in L2).
+template <int LEN, bool HALF>
+__global__ void __launch_bounds__(r16_threads<LEN>(), 512 / r16_threads<LEN>())
+    filter_rows_r16_quads(const float* __restrict__ sino, int batch, FilterCfg cfg, float* __restrict__ quads) {
+   constexpr int TPF = LEN / 16, FPB = r16_threads<LEN>() / TPF, PL = LEN + LEN / 16;
+   using P = R16Plan<LEN>;
+   extern __shared__ float2 sm[];
+   const int local = threadIdx.x / TPF, lt = threadIdx.x % TPF;
+   const int Pp = cfg.rows, Dp = cfg.Dp;
+   const int pair = blockIdx.x * FPB + local;  // (quad, angle, half)
+   const int qa = pair >> 1, quad = qa / Pp, ang = qa - quad * Pp;
+   const int s0 = 4 * quad + 2 * (pair & 1);
+   const bool has_a = s0 < batch, has_b = s0 + 1 < batch;
+   const float* row_a = sino + ((size_t)(has_a ? s0 : 0) * Pp + ang) * Dp;
+   const float* row_b = sino + ((size_t)(has_b ? s0 + 1 : 0) * Pp + ang) * Dp;
+   float2* buf = sm + local * PL;
+   float2 v[16];
+#pragma unroll
+   for (int r = 0; r < (HALF ? 8 : 16); ++r) {
+      const int n = lt + r * TPF;
+      v[r] = make_float2((has_a && n < Dp) ? row_a[n] : 0.f, (has_b && n < Dp) ? row_b[n] : 0.f);
+   }
+   r16_filter_core<LEN, HALF>(v, buf, lt, cfg.twp, cfg.h, cfg.adjoint != 0);
+   if (!has_a) return;
+   float* out = quads + (((size_t)quad * Pp + ang) * Dp) * 4 + 2 * (pair & 1);
+#pragma unroll
+   for (int b = 0; b < 16 / P::R3; ++b)
+#pragma unroll
+      for (int r = 0; r < P::R3; ++r) {
+         if (HALF && out_slot<P::R3>(r) >= P::R3 / 2) continue;  // time index LEN / 2 or more
+         const int n = r16_time_index<LEN>(lt, b, r);
+         if (n < Dp)
+            *reinterpret_cast<float2*>(out + 4 * (size_t)n) =
+                make_float2(v[b * P::R3 + r].x, has_b ? -v[b * P::R3 + r].y : 0.f);
+      }
+}
+
+template <int LEN, bool HALF>
+cudaError_t launch_r16_quads_as(const float* sino, int batch, const FilterCfg& cfg, float* quads, cudaStream_t st) {
+   constexpr int TPF = LEN / 16, FPB = r16_threads<LEN>() / TPF;
+   const size_t smem = sizeof(float2) * (size_t)FPB * (LEN + LEN / 16);
+   if (smem > 48 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(filter_rows_r16_quads<LEN, HALF>,
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+   }
+   const int pairs = (batch + 3) / 4 * cfg.rows * 2;
+   filter_rows_r16_quads<LEN, HALF><<<(pairs + FPB - 1) / FPB, r16_threads<LEN>(), smem, st>>>(sino, batch, cfg, quads);
+   return cudaGetLastError();
+}
+
 template <int LEN, bool HALF>
 cudaError_t launch_r16_pairs_as(const float* sino, int batch, const FilterCfg& cfg, const PairsOut& po,
                                 cudaStream_t st) {
@@ -400,6 +455,11 @@ cudaError_t launch_r16_pairs_as(const float* sino, int batch, const FilterCfg& c
 template <int LEN>
 cudaError_t launch_r16_pairs(const float* sino, int batch, const FilterCfg& cfg, const PairsOut& po,
                              cudaStream_t st) {
+   if (po.S == 0) {
+      float* quads = static_cast<float*>(po.pairs);
+      return 2 * cfg.Dp <= LEN ? launch_r16_quads_as<LEN, true>(sino, batch, cfg, quads, st)
+                               : launch_r16_quads_as<LEN, false>(sino, batch, cfg, quads, st);
+   }
    return 2 * cfg.Dp <= LEN ? launch_r16_pairs_as<LEN, true>(sino, batch, cfg, po, st)
                             : launch_r16_pairs_as<LEN, false>(sino, batch, cfg, po, st);
 }
@@ -499,7 +559,7 @@ bool filter_pairs_supported(const FilterCfg& cfg) {
 cudaError_t launch_filter_pairs(const float* sino, int batch, const FilterCfg& cfg, const PairsOut& po,
                                 cudaStream_t st) {
    if (batch <= 0) return cudaSuccess;
-   if (!po.pairs || po.S < 2 || po.S % 2 || po.wp <= 0) return cudaErrorInvalidValue;
+   if (!po.pairs || po.S % 2 || po.S < 0 || (po.S > 0 && po.wp <= 0)) return cudaErrorInvalidValue;
    switch (filter_pairs_supported(cfg) ? cfg.len : 0) {
       case 512: return launch_r16_pairs<512>(sino, batch, cfg, po, st);
       case 1024: return launch_r16_pairs<1024>(sino, batch, cfg, po, st);

@@ -223,6 +223,7 @@ cudaError_t launch_filter(float* sino, int batch, const FilterCfg& cfg, cudaStre
 // Destination of the fused filter + backprojection staging pass: the padded
 // pair sinogram of a staged backprojection variant with S slices per group
 // (window bins u = k + win_lo, u in [0, wp)).
+// S = 0: plain rows in slice quads, [quad][angle][bin][4], no padding.
 struct PairsOut {
    void* pairs;  // float4 records
    int S, win_lo, wp;
@@ -243,6 +244,24 @@ cudaError_t launch_filter_taps_grad(const float* x, const float* g, int batch, c
 
 // ---------------------------------------------------------------- backprojection
 constexpr int kCPAngles = 2048;  // angles the backprojection can take from its kernel parameters
+// The patch kernel's angle plan (k_bp_patch.cu): angles sorted by the signs of
+// a and b and by their bin-offset class, cut into runs of one class each.
+constexpr int kPatchAngles = 2048;
+constexpr int kPatchMaxSegs = 32;  // at most 7 classes for each of the 4 sign pairs
+struct BPPatchAngle {
+   double t0, a, b;
+   int index, pad;  // the angle's row
+};
+struct BPPatchPlan {
+   std::vector<BPPatchAngle> angles;  // in plan order; empty: the geometry is outside the kernel's range
+   std::vector<float> A, B;           // |a|, |b|
+   std::vector<uint32_t> segs;        // runs of one class: first | n << 12 | class << 24 | signs << 28
+};
+bool bp_patch_plan(const float* a, const float* b, const double* ad, const double* bd, const double* t0, int Pp,
+                   float scale, BPPatchPlan* plan);
+// Device bytes of the staged rows [quad of slices][angle][bin][4] of `batch` slices
+// and the quads' non-finite flags.
+size_t bp_quads_bytes(int batch, int Pp, int Dp);
 struct BPCfg {
    int Pp, Dp, N;
    const float* a;      // [Pp]
@@ -269,6 +288,8 @@ struct BPCfg {
    const float* b_host = nullptr;  // coefficients, at most kCPAngles angles)
    const int2* tile_win = nullptr;  // staged variants: per tile and angle (window start, bits of the float
                                     // coordinate of the tile origin in it), bp_tile_windows; else FP64 on device
+   const BPPatchPlan* patch = nullptr;  // host side
+   const BPPatchAngle* patch_angles = nullptr;
    void* adj_scratch = nullptr;  // adjoint: slice-interleaved image copies (bp_adjoint_scratch_bytes)
    size_t adj_scratch_bytes = 0;
    // adjoint: FP64 line starts split as (hi, lo) floats, [Pp][N]:
@@ -287,7 +308,7 @@ int bp_variant_count();
 const char* bp_variant_name(int v);
 // Device bytes of the pair sinogram that `variant` needs for `batch` slices
 // (0 for variants that stage windows from the sinogram itself).
-size_t bp_pairs_bytes(int variant, int batch, int Pp, int win_len);
+size_t bp_pairs_bytes(int variant, int batch, int Pp, int Dp, int win_len);
 // Slices per group of a staged variant (the S of its pair records), 0 for the others.
 int bp_variant_pair_slices(int variant);
 // Padding of the pair sinogram: the bin range covering every window that a
@@ -295,6 +316,12 @@ int bp_variant_pair_slices(int variant);
 // when `masking`), computed with the kernel's own arithmetic.
 void bp_window_extent(const float* a, const float* b, const double* ad, const double* bd, const double* t0,
                       int Pp, int N, float scale, bool masking, int* win_lo, int* win_len);
+// How a variant's staged rows are laid out: (mid, diff) pair records, or plain
+// slice quads; kLayoutNone for the variants that read the sinogram itself.
+enum BPLayout { kLayoutNone, kLayoutPairs, kLayoutQuads };
+BPLayout bp_variant_layout(int variant);
+cudaError_t launch_bp_patch(const float* sino, float* img, int batch, const BPCfg& cfg, cudaStream_t st);
+int bp_patch_variant();  // its place in the variant list
 cudaError_t launch_backprojection(const float* sino, float* img, int batch, const BPCfg& cfg,
                                   int variant, cudaStream_t st);
 cudaError_t launch_backprojection_adjoint(const float* img, float* sino, int batch,
