@@ -904,12 +904,12 @@ __global__ void __launch_bounds__(128) bp_adjoint(const float* __restrict__ img,
    for (int s = 0; s < SB; ++s)
       if (s0 + s < batch) sino[((size_t)(s0 + s) * cfg.Pp + i) * cfg.Dp + k] = acc[s] * cfg.norm;
 }
-// Slice-interleaved copies of the image for the adjoint: P[g][y][x][8] and
-// its transpose PT[g][x][y][8] hold slices 8g..8g+7 (zero past the batch), so
-// a ray walking rows of P (angles with |a| >= |b|) or rows of PT (the others)
-// reads the 8 slices of a pixel with two 16-byte loads from consecutive
-// addresses across the warp. One CTA transposes a 32 x 32 pixel tile of all 8
-// slices of a group through shared memory.
+// Slice-interleaved copies of the image for the adjoint: P[g][h][y][x][4] and
+// its transpose PT[g][h][x][y][4] hold slices 8g + 4h .. 8g + 4h + 3 (zero past
+// the batch), so a ray walking rows of P (angles with |a| >= |b|) or rows of PT
+// (the others) reads 4 slices of a pixel with one 16-byte load, and the lanes of
+// a warp (consecutive bins) read consecutive 16-byte entries. One CTA transposes
+// a 32 x 32 pixel tile of all 8 slices of a group through shared memory.
 __global__ void __launch_bounds__(256) bp_adjoint_layout(const float* __restrict__ img, float4* __restrict__ P,
                                                          float4* __restrict__ PT, int N, int batch) {
    __shared__ float tile[8][32][33];
@@ -930,80 +930,192 @@ __global__ void __launch_bounds__(256) bp_adjoint_layout(const float* __restrict
    for (int yy = ty; yy < 32; yy += 8) {
       const int y = y0 + yy, x = x0 + tx;
       if (y < N && x < N) {  // pixel (y, x): row y of P
-         const size_t o = ((size_t)y * N + x) * 2;
+         const size_t o = (size_t)y * N + x;
          Pg[o] = make_float4(tile[0][yy][tx], tile[1][yy][tx], tile[2][yy][tx], tile[3][yy][tx]);
-         Pg[o + 1] = make_float4(tile[4][yy][tx], tile[5][yy][tx], tile[6][yy][tx], tile[7][yy][tx]);
+         Pg[plane + o] = make_float4(tile[4][yy][tx], tile[5][yy][tx], tile[6][yy][tx], tile[7][yy][tx]);
       }
       const int xt = x0 + yy, yt = y0 + tx;  // pixel (yt, xt): row xt of PT
       if (xt < N && yt < N) {
-         const size_t o = ((size_t)xt * N + yt) * 2;
+         const size_t o = (size_t)xt * N + yt;
          PTg[o] = make_float4(tile[0][tx][yy], tile[1][tx][yy], tile[2][tx][yy], tile[3][tx][yy]);
-         PTg[o + 1] = make_float4(tile[4][tx][yy], tile[5][tx][yy], tile[6][tx][yy], tile[7][tx][yy]);
+         PTg[plane + o] = make_float4(tile[4][tx][yy], tile[5][tx][yy], tile[6][tx][yy], tile[7][tx][yy]);
       }
    }
 }
 
-// The adjoint over the interleaved layout: as bp_adjoint with 8 slices per
-// thread, the ray always walking rows (of P, or of PT for steep angles), and
-// the visited pixel range [floor(ja), ceil(jb)]: the range ends carry an
-// error of ~1e-6 * N / |step| pixels (< 1e-3), far below one pixel, and every
-// visited pixel is still tested exactly (|t' - k| < 1).
-__global__ void __launch_bounds__(128) bp_adjoint_rows(const float4* __restrict__ P, const float4* __restrict__ PT,
-                                                       float* __restrict__ sino, BPCfg cfg, int batch) {
-   extern __shared__ float2 s_line[];  // this angle's line starts [N]
-   const int k = blockIdx.x * blockDim.x + threadIdx.x;
-   const int i = blockIdx.y;
-   const int g = blockIdx.z;
-   const int N = cfg.N;
-   const float a = __ldg(cfg.a + i), b = __ldg(cfg.b + i);
-   const bool along_x = fabsf(a) >= fabsf(b);
-   const float2* line = (along_x ? cfg.rowbase : cfg.colbase) + (size_t)i * N;
-   for (int r = threadIdx.x; r < N; r += blockDim.x) s_line[r] = __ldg(line + r);
+// 16 bytes from global memory where `p`, zeros (and no access) elsewhere.
+__device__ __forceinline__ ulonglong2 ldg_if(const ulonglong2* ptr, bool p) {
+   ulonglong2 v;
+   asm("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\tmov.u64 %0, 0;\n\tmov.u64 %1, 0;\n\t"
+       "@q ld.global.nc.v2.u64 {%0, %1}, [%2];\n\t}"
+       : "=&l"(v.x), "=&l"(v.y)
+       : "l"(ptr), "r"((int)p));
+   return v;
+}
+
+// The adjoint over the interleaved layout: as bp_adjoint with up to 8 slices
+// per thread (NH 16-byte halves), the ray always walking rows (of P, or of PT
+// for steep angles). A warp is 32 consecutive bins of one angle; the warps of a
+// CTA are `apc` consecutive angles over the same bins, whose rays cross a row at
+// nearly the same pixels, so the image passes from L2 to L1 once per CTA and not
+// once per angle; `rs` warps share an angle's rows where the bins alone leave
+// the GPU idle, and their sums are added in a fixed order.
+// What bounds it is L1 wavefronts: per row and warp, two candidate pixels of NH
+// 16-byte loads (4.5 wavefronts each; 82% of the data path). 16 slices of 512^2
+// -> 720 x 768: 1.77 ms with 32-byte pixel records and one angle per CTA (7
+// wavefronts a load, 6.8 TB/s from L2), 1.24 ms in this layout, 1.13 ms with the
+// loads of two rows issued before their multiply-adds (four rows: 1.16).
+template <int NH>
+__global__ void __launch_bounds__(256) bp_adjoint_rows(const float4* __restrict__ P, const float4* __restrict__ PT,
+                                                       float* __restrict__ sino, BPCfg cfg, int batch, int apc,
+                                                       int rs) {
+   extern __shared__ float2 s_line[];  // the angles' line starts [apc][N]; then the partial sums
+   const int N = cfg.N, Dp = cfg.Dp;
+   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+   const int sub = warp % apc, part = warp / apc;  // angle of the CTA, share of the rows
+   const int k = blockIdx.x * 32 + lane;
+   const int i = blockIdx.y * apc + sub, g = blockIdx.z;
+   for (int w = warp; w < apc; w += apc * rs) {
+      const int iw = blockIdx.y * apc + w;
+      if (iw >= cfg.Pp) continue;
+      const bool ax = fabsf(__ldg(cfg.a + iw)) >= fabsf(__ldg(cfg.b + iw));
+      const float2* line = (ax ? cfg.rowbase : cfg.colbase) + (size_t)iw * N;
+      for (int r = lane; r < N; r += 32) s_line[w * N + r] = __ldg(line + r);
+   }
    __syncthreads();
-   if (k >= cfg.Dp) return;
-   const float s_hi = along_x ? a : b;
-   const float s_lo = (float)((along_x ? __ldg(cfg.ad + i) : __ldg(cfg.bd + i)) - (double)s_hi);
-   const float inv = 1.0f / s_hi;  // |s_hi| >= scale / sqrt(2) > 0
-   const float4* im = (along_x ? P : PT) + (size_t)g * N * N * 2;
-   const float kf = (float)k;
-   // The pixels of a row within one bin of k lie in the open interval from
-   // jlo = (-/+1 - t0) / s of length 2 / |s|; the candidates are the
-   // ncand consecutive integers from ceil(jlo - 1e-3) (1e-3 pixel covers the
-   // FP32 error of jlo, ~1e-4 at these sizes), each then tested exactly.
-   const float lo_num = s_hi > 0.f ? -1.f : 1.f;
-   const int ncand = (int)floorf(2.f * fabsf(inv) + 0.002f) + 1;
-   // the 8 slices of a pixel as four f32x2 pairs: one fma.rn.f32x2 per pair
-   // (each lane rounded like fmaf)
-   unsigned long long acc2[4] = {0ull, 0ull, 0ull, 0ull};
-   const ulonglong2* imp = reinterpret_cast<const ulonglong2*>(im);
-   for (int r = 0; r < N; ++r) {
-      const float2 hb = s_line[r];
-      const float t_hi = hb.x - kf, t_lo = hb.y;
-      const float jlo = (lo_num - (t_hi + t_lo)) * inv;
-      const int j1 = (int)ceilf(jlo - 1e-3f);
-      const ulonglong2* row = imp + (size_t)r * N * 2;
-      for (int c = 0; c < ncand; ++c) {
-         const int j = j1 + c;
-         if ((unsigned)j >= (unsigned)N) continue;
-         const float jf = (float)j;
-         const float d = fabsf(fmaf(jf, s_hi, t_hi) + fmaf(jf, s_lo, t_lo));
-         if (d < 1.f) {
-            const float w = 1.f - d;
-            const unsigned long long w2 = f2_pack(w, w);
-            const ulonglong2 v0 = __ldg(row + 2 * j), v1 = __ldg(row + 2 * j + 1);
-            acc2[0] = f2_fma(w2, v0.x, acc2[0]);
-            acc2[1] = f2_fma(w2, v0.y, acc2[1]);
-            acc2[2] = f2_fma(w2, v1.x, acc2[2]);
-            acc2[3] = f2_fma(w2, v1.y, acc2[3]);
+   unsigned long long acc2[2 * NH];
+#pragma unroll
+   for (int q = 0; q < 2 * NH; ++q) acc2[q] = 0ull;
+   if (i < cfg.Pp) {
+      const float a = __ldg(cfg.a + i), b = __ldg(cfg.b + i);
+      const bool along_x = fabsf(a) >= fabsf(b);
+      const float s_hi = along_x ? a : b, cross = along_x ? b : a;
+      const float s_lo = (float)((along_x ? __ldg(cfg.ad + i) : __ldg(cfg.bd + i)) - (double)s_hi);
+      const float inv = 1.0f / s_hi;  // |s_hi| >= scale / sqrt(2) > 0
+      const size_t plane = (size_t)N * N;
+      const ulonglong2* im = reinterpret_cast<const ulonglong2*>((along_x ? P : PT) + (size_t)g * plane * 2);
+      const float2* lines = s_line + sub * N;
+      const float kf = (float)k;
+      // Rows whose candidates can lie in the image, for any bin of the warp: the
+      // ray of bin k crosses row r near j = c0 + slope r (margin 3 pixels, the
+      // FP32 error is below 1e-2)
+      int r0 = 0, r1 = N;
+      {
+         const float c0 = (kf - (lines[0].x + lines[0].y)) * inv, slope = -cross * inv;
+         const float lo = -(fabsf(inv) + 3.f), hi = (float)N + fabsf(inv) + 3.f;
+         if (fabsf(slope) * (float)N < 0.5f) {
+            if (c0 < lo - 1.f || c0 > hi + 1.f) r1 = 0;
+         } else {
+            const float ra = (lo - c0) / slope, rb = (hi - c0) / slope;
+            r0 = (int)fminf(fmaxf(floorf(fminf(ra, rb)) - 1.f, 0.f), (float)N);
+            r1 = (int)fminf(fmaxf(ceilf(fmaxf(ra, rb)) + 1.f, 0.f), (float)N);
+         }
+         if (k >= Dp || r1 <= r0) r0 = N, r1 = 0;
+         r0 = __reduce_min_sync(~0u, r0);
+         r1 = __reduce_max_sync(~0u, r1);
+      }
+      if (rs > 1 && r1 > r0) {
+         const int len = (r1 - r0 + rs - 1) / rs, first = r0 + part * len;
+         r1 = min(r1, first + len);
+         r0 = first;
+      }
+      // The pixels of a row within one bin of k lie in the open interval from
+      // jlo = (-/+1 - t0) / s of length 2 / |s|; the candidates are the
+      // ncand consecutive integers from ceil(jlo - 1e-3) (1e-3 pixel covers the
+      // FP32 error of jlo, ~1e-4 at these sizes), each then tested exactly. The
+      // integer comes from rounding jlo - 1e-3 + 1/2 with the magic constant.
+      const float lo_num = s_hi > 0.f ? -1.f : 1.f;
+      const int ncand = (int)floorf(2.f * fabsf(inv) + 0.002f) + 1;
+      const float vbias = 0.5f - 1e-3f;
+      // R rows at a time: every candidate's test first, then all their loads
+      // (predicated on the test, zeros elsewhere: no read outside the image or
+      // of a pixel the ray misses), then the multiply-adds
+      auto rows = [&](int r, auto rc, auto ncc) {
+         constexpr int R = decltype(rc)::value, NC = decltype(ncc)::value;
+         float w[R][NC];
+         ulonglong2 v[R][NC][NH];
+#pragma unroll
+         for (int u = 0; u < R; ++u) {
+            const float2 hb = lines[r + u];
+            const float t_hi = hb.x - kf, t_lo = hb.y;
+            const float m = fmaf(lo_num - (t_hi + t_lo), inv, vbias) + kMagic;
+            const float j1 = m - kMagic;
+            const int j1i = __float_as_int(m) - kMagicBits;
+            const ulonglong2* rowp = im + (size_t)(r + u) * N + j1i;
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+               const float jf = j1 + (float)c;
+               const float d = fabsf(fmaf(jf, s_hi, t_hi) + fmaf(jf, s_lo, t_lo));
+               const bool hit = d < 1.f && (unsigned)(j1i + c) < (unsigned)N;
+               w[u][c] = 1.f - d;
+#pragma unroll
+               for (int h = 0; h < NH; ++h) v[u][c][h] = ldg_if(rowp + c + (h ? plane : 0), hit);
+               if (!hit) w[u][c] = 0.f;
+            }
+         }
+#pragma unroll
+         for (int u = 0; u < R; ++u)
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+               const unsigned long long w2 = f2_pack(w[u][c], w[u][c]);
+#pragma unroll
+               for (int h = 0; h < NH; ++h) {
+                  acc2[2 * h] = f2_fma(w2, v[u][c][h].x, acc2[2 * h]);
+                  acc2[2 * h + 1] = f2_fma(w2, v[u][c][h].y, acc2[2 * h + 1]);
+               }
+            }
+      };
+      auto walk = [&](auto rc, auto ncc) {
+         constexpr int R = decltype(rc)::value;
+         int r = r0;
+         for (; r + R <= r1; r += R) rows(r, rc, ncc);
+         for (; r < r1; ++r) rows(r, std::integral_constant<int, 1>{}, ncc);
+      };
+      using std::integral_constant;
+      if (ncand <= 2) walk(integral_constant<int, 2>{}, integral_constant<int, 2>{});
+      else if (ncand == 3) walk(integral_constant<int, 2>{}, integral_constant<int, 3>{});
+      else {
+         // fewer than one bin per pixel: any number of candidates, one at a time
+         for (int r = r0; r < r1; ++r) {
+            const float2 hb = lines[r];
+            const float t_hi = hb.x - kf, t_lo = hb.y;
+            const float m = fmaf(lo_num - (t_hi + t_lo), inv, vbias) + kMagic;
+            const float j1 = m - kMagic;
+            const int j1i = __float_as_int(m) - kMagicBits;
+            for (int c = 0; c < ncand; ++c) {
+               const float jf = j1 + (float)c;
+               const float d = fabsf(fmaf(jf, s_hi, t_hi) + fmaf(jf, s_lo, t_lo));
+               if (!(d < 1.f && (unsigned)(j1i + c) < (unsigned)N)) continue;
+               const unsigned long long w2 = f2_pack(1.f - d, 1.f - d);
+#pragma unroll
+               for (int h = 0; h < NH; ++h) {
+                  const ulonglong2 v = __ldg(im + (size_t)r * N + j1i + c + (h ? plane : 0));
+                  acc2[2 * h] = f2_fma(w2, v.x, acc2[2 * h]);
+                  acc2[2 * h + 1] = f2_fma(w2, v.y, acc2[2 * h + 1]);
+               }
+            }
          }
       }
    }
-   float acc[8];
+   if (rs > 1) {  // sum the row shares of an angle in their order
+      __syncthreads();
+      unsigned long long* part_sums = reinterpret_cast<unsigned long long*>(s_line);  // [warp][2 NH][32]
 #pragma unroll
-   for (int q = 0; q < 4; ++q) f2_unpack(acc2[q], acc[2 * q], acc[2 * q + 1]);
+      for (int q = 0; q < 2 * NH; ++q) part_sums[(warp * 2 * NH + q) * 32 + lane] = acc2[q];
+      __syncthreads();
+      if (part > 0) return;
+      for (int p = 1; p < rs; ++p)
 #pragma unroll
-   for (int s = 0; s < 8; ++s)
-      if (8 * g + s < batch) sino[((size_t)(8 * g + s) * cfg.Pp + i) * cfg.Dp + k] = acc[s] * cfg.norm;
+         for (int q = 0; q < 2 * NH; ++q)
+            acc2[q] = f2_add(acc2[q], part_sums[((p * apc + sub) * 2 * NH + q) * 32 + lane]);
+   }
+   if (i >= cfg.Pp || k >= Dp) return;
+   float acc[4 * NH];
+#pragma unroll
+   for (int q = 0; q < 2 * NH; ++q) f2_unpack(acc2[q], acc[2 * q], acc[2 * q + 1]);
+#pragma unroll
+   for (int s = 0; s < 4 * NH; ++s)
+      if (8 * g + s < batch) sino[((size_t)(8 * g + s) * cfg.Pp + i) * Dp + k] = acc[s] * cfg.norm;
 }
 }  // namespace
 
@@ -1167,8 +1279,18 @@ cudaError_t launch_backprojection_adjoint(const float* img, float* sino, int bat
       float4* PT = P + (size_t)groups * cfg.N * cfg.N * 2;
       dim3 lg((cfg.N + 31) / 32, (cfg.N + 31) / 32, groups);
       bp_adjoint_layout<<<lg, 256, 0, st>>>(img, P, PT, cfg.N, batch);
-      dim3 grid((cfg.Dp + 127) / 128, cfg.Pp, groups);
-      bp_adjoint_rows<<<grid, 128, smem, st>>>(P, PT, sino, cfg, batch);
+      // 8 warps per CTA; row shares so that small geometries still fill the GPU
+      // (about 32 warps on each of 152 SMs)
+      const long warps = (long)((cfg.Dp + 31) / 32) * cfg.Pp * groups;
+      const int rs = warps >= 4864 ? 1 : warps >= 2432 ? 2 : 4;
+      int apc = 8 / rs;
+      while (apc > 1 && sizeof(float2) * (size_t)apc * cfg.N > 48 * 1024) apc /= 2;
+      const bool one = batch <= 4;
+      const size_t sums = rs > 1 ? sizeof(float2) * 32 * (one ? 2 : 4) * (size_t)(apc * rs) : 0;
+      const size_t lines = std::max(sizeof(float2) * (size_t)apc * cfg.N, sums);
+      dim3 grid((cfg.Dp + 31) / 32, (cfg.Pp + apc - 1) / apc, groups);
+      if (one) bp_adjoint_rows<1><<<grid, 32 * apc * rs, lines, st>>>(P, PT, sino, cfg, batch, apc, rs);
+      else bp_adjoint_rows<2><<<grid, 32 * apc * rs, lines, st>>>(P, PT, sino, cfg, batch, apc, rs);
       return cudaGetLastError();
    }
    if (batch >= 8) {
