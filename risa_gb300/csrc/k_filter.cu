@@ -170,11 +170,18 @@ __global__ void __launch_bounds__(kThreads) filter_grad_partial(const float* __r
 template <int LEN>
 __host__ __device__ constexpr int r16_threads() { return LEN / 16 >= 128 ? LEN / 16 : 128; }
 
-// filter_grad_partial on the radix-16 path (LEN 512..4096): the forward
-// transforms of a row pair of x and of g run in registers (three passes each),
-// the spectra go to shared memory in natural order, and the pair's G conj(X)
-// is added to the CTA's accumulator in the same fixed order as above.
-template <int LEN>
+// filter_grad_partial on the radix-16 path (LEN 512..4096). The two rows of a
+// pair are not separated: with Z = X_a + i X_b for x and for g,
+// Zg conj(Zx) = S + i T, S = G_a conj(X_a) + G_b conj(X_b) the wanted sum and T =
+// G_b conj(X_a) - G_a conj(X_b), both Hermitian (the rows are real), so the
+// inverse transform of S is the real part of that of the product. The forward
+// transforms of x and g leave the same frequencies in the same registers, so a
+// CTA adds its pairs' products in registers, in their order, and writes one
+// partial spectrum at the end. Bound by FFT issue: 11,520 rows of 768 in 2048
+// (x and g, 71 MB) take 56 us; separating the spectra through shared memory
+// took 104.
+// HALF: Dp <= LEN / 2, the upper half of the padded rows is not transformed.
+template <int LEN, bool HALF>
 __global__ void __launch_bounds__(r16_threads<LEN>(), 384 / r16_threads<LEN>())
     filter_grad_partial_r16(const float* __restrict__ x, const float* __restrict__ g, int total_rows, FilterCfg cfg,
                             float2* __restrict__ partial, int groups) {
@@ -182,88 +189,118 @@ __global__ void __launch_bounds__(r16_threads<LEN>(), 384 / r16_threads<LEN>())
    using P = R16Plan<LEN>;
    extern __shared__ float2 sm[];
    const int local = threadIdx.x / TPF, lt = threadIdx.x % TPF;
-   float2* bx = sm + (size_t)local * 2 * PL;  // X spectrum, padded index
-   float2* bg = bx + PL;                     // transform scratch, then the G spectrum
-   float2* acc = sm + (size_t)FPB * 2 * PL;  // [LEN], shared by the CTA's pairs
+   float2* buf = sm + (size_t)local * PL;
    const int Dp = cfg.Dp;
-   for (int k = threadIdx.x; k < LEN; k += blockDim.x) acc[k] = make_float2(0.f, 0.f);
+   float2 acc[16];
+#pragma unroll
+   for (int r = 0; r < 16; ++r) acc[r] = make_float2(0.f, 0.f);
    for (int grp = blockIdx.x; grp < groups; grp += gridDim.x) {
-      const int pair = grp * FPB + local;
-      const int ra = 2 * pair, rb = 2 * pair + 1;
+      const int ra = 2 * (grp * FPB + local), rb = ra + 1;
       const bool has_a = ra < total_rows, has_b = rb < total_rows;
-      float2 v[16];
-      __syncthreads();  // the previous group's spectra have been read
+      float2 vx[16], v[16];
+      auto load = [&](const float* rows, float2 (&u)[16]) {
 #pragma unroll
-      for (int r = 0; r < 16; ++r) {
-         const int n = lt + r * TPF;
-         v[r] = make_float2((has_a && n < Dp) ? x[(size_t)ra * Dp + n] : 0.f,
-                            (has_b && n < Dp) ? x[(size_t)rb * Dp + n] : 0.f);
-      }
-      r16_forward<LEN>(v, bg, lt, cfg.twp);
-#pragma unroll
-      for (int b = 0; b < 16 / P::R3; ++b)
-#pragma unroll
-         for (int r = 0; r < P::R3; ++r) bx[pad16(r16_time_index<LEN>(lt, b, r))] = v[b * P::R3 + r];
-#pragma unroll
-      for (int r = 0; r < 16; ++r) {
-         const int n = lt + r * TPF;
-         v[r] = make_float2((has_a && n < Dp) ? g[(size_t)ra * Dp + n] : 0.f,
-                            (has_b && n < Dp) ? g[(size_t)rb * Dp + n] : 0.f);
-      }
-      r16_forward<LEN>(v, bg, lt, cfg.twp);
-#pragma unroll
-      for (int b = 0; b < 16 / P::R3; ++b)
-#pragma unroll
-         for (int r = 0; r < P::R3; ++r) bg[pad16(r16_time_index<LEN>(lt, b, r))] = v[b * P::R3 + r];
-      __syncthreads();
-      for (int p = 0; p < FPB; ++p) {  // pairs of the CTA add in a fixed order
-         if (local == p) {
-            for (int k = lt; k < LEN; k += TPF) {
-               const int nk = (LEN - k) & (LEN - 1);
-               const float2 zk = bx[pad16(k)], zn = bx[pad16(nk)], gk = bg[pad16(k)], gn = bg[pad16(nk)];
-               // X_a = (zk + conj zn)/2, X_b = (zk - conj zn)/(2i); same for G
-               const float2 xa = make_float2(0.5f * (zk.x + zn.x), 0.5f * (zk.y - zn.y));
-               const float2 xb = make_float2(0.5f * (zk.y + zn.y), -0.5f * (zk.x - zn.x));
-               const float2 ga = make_float2(0.5f * (gk.x + gn.x), 0.5f * (gk.y - gn.y));
-               const float2 gb = make_float2(0.5f * (gk.y + gn.y), -0.5f * (gk.x - gn.x));
-               // G conj(X)
-               const float2 pa = make_float2(ga.x * xa.x + ga.y * xa.y, ga.y * xa.x - ga.x * xa.y);
-               const float2 pb = make_float2(gb.x * xb.x + gb.y * xb.y, gb.y * xb.x - gb.x * xb.y);
-               acc[k].x += pa.x + pb.x;
-               acc[k].y += pa.y + pb.y;
-            }
+         for (int r = 0; r < (HALF ? 8 : 16); ++r) {
+            const int n = lt + r * TPF;
+            u[r] = make_float2((has_a && n < Dp) ? __ldg(rows + (size_t)ra * Dp + n) : 0.f,
+                               (has_b && n < Dp) ? __ldg(rows + (size_t)rb * Dp + n) : 0.f);
          }
-         __syncthreads();
+      };
+      load(x, vx);
+      load(g, v);
+      r16_forward<LEN, HALF>(vx, buf, lt, cfg.twp);
+      r16_forward<LEN, HALF>(v, buf, lt, cfg.twp);
+#pragma unroll
+      for (int r = 0; r < 16; ++r) {  // += Zg conj(Zx)
+         acc[r].x = fmaf(v[r].x, vx[r].x, fmaf(v[r].y, vx[r].y, acc[r].x));
+         acc[r].y = fmaf(v[r].y, vx[r].x, fmaf(-v[r].x, vx[r].y, acc[r].y));
       }
    }
-   for (int k = threadIdx.x; k < LEN; k += blockDim.x) partial[(size_t)blockIdx.x * LEN + k] = acc[k];
+   // the CTA's pairs in a fixed order, then its partial spectrum
+   for (int p = 0; p < FPB; ++p) {
+      if (local == p) {
+#pragma unroll
+         for (int b = 0; b < 16 / P::R3; ++b)
+#pragma unroll
+            for (int r = 0; r < P::R3; ++r) {
+               const int k = r16_time_index<LEN>(lt, b, r);
+               const float2 t = acc[b * P::R3 + r];
+               const float2 s = p > 0 ? sm[k] : make_float2(0.f, 0.f);
+               const float2 sum = make_float2(s.x + t.x, s.y + t.y);
+               if (p + 1 < FPB) sm[k] = sum;
+               else partial[(size_t)blockIdx.x * LEN + k] = sum;
+            }
+      }
+      if (p + 1 < FPB) __syncthreads();
+   }
 }
 
 template <int LEN>
 cudaError_t launch_grad_partial_r16(const float* x, const float* g, int total_rows, const FilterCfg& cfg,
                                     float2* partial, int groups, int blocks, cudaStream_t st) {
    constexpr int TPF = LEN / 16, FPB = r16_threads<LEN>() / TPF;
-   const size_t smem = sizeof(float2) * ((size_t)FPB * 2 * (LEN + LEN / 16) + LEN);
-   cudaError_t e =
-       cudaFuncSetAttribute(filter_grad_partial_r16<LEN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-   if (e != cudaSuccess) return e;
-   filter_grad_partial_r16<LEN><<<blocks, r16_threads<LEN>(), smem, st>>>(x, g, total_rows, cfg, partial, groups);
+   const size_t smem = sizeof(float2) * (size_t)FPB * (LEN + LEN / 16);
+   if (2 * cfg.Dp <= LEN)
+      filter_grad_partial_r16<LEN, true><<<blocks, r16_threads<LEN>(), smem, st>>>(x, g, total_rows, cfg, partial, groups);
+   else
+      filter_grad_partial_r16<LEN, false><<<blocks, r16_threads<LEN>(), smem, st>>>(x, g, total_rows, cfg, partial, groups);
    return cudaGetLastError();
 }
 
-// Sum of the partial spectra in block order, one frequency per thread;
-// spec receives the conjugate (the finish kernel inverts by conj(FFT(conj))).
+// Sum of the partial spectra: a CTA takes 32 frequencies, its 8 warps eight
+// consecutive shares of the blocks, added in their order (fixed by the number
+// of blocks). spec receives the conjugate (the finish kernel inverts by
+// conj(FFT(conj))). 512 blocks of 2048: 8 us (46 with one thread per
+// frequency walking all blocks).
 __global__ void __launch_bounds__(kThreads) filter_grad_sum(const float2* __restrict__ partial, int blocks, int len,
                                                             float2* __restrict__ spec) {
-   const int k = blockIdx.x * kThreads + threadIdx.x;
-   if (k >= len) return;
+   __shared__ float2 s_sum[kThreads / 32][32];
+   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, k = blockIdx.x * 32 + lane;  // len is a multiple of 32
+   const int share = (blocks + kThreads / 32 - 1) / (kThreads / 32);
+   const int j1 = min(blocks, (warp + 1) * share);
    float sx = 0.f, sy = 0.f;
-   for (int j = 0; j < blocks; ++j) {
-      const float2 v = partial[(size_t)j * len + k];
+#pragma unroll 8
+   for (int j = warp * share; j < j1; ++j) {
+      const float2 v = __ldg(partial + (size_t)j * len + k);
       sx += v.x;
       sy += v.y;
    }
+   s_sum[warp][lane] = make_float2(sx, sy);
+   __syncthreads();
+   if (warp > 0) return;
+   for (int w = 1; w < kThreads / 32; ++w) {
+      sx += s_sum[w][lane].x;
+      sy += s_sum[w][lane].y;
+   }
    spec[k] = make_float2(sx, -sy);
+}
+
+// One CTA on the radix-16 path: invert the summed (conjugated) spectrum, scale
+// by 1/len, map lags to taps (see filter_grad_finish).
+template <int LEN>
+__global__ void __launch_bounds__(LEN / 16) filter_grad_finish_r16(const float2* __restrict__ spec, FilterCfg cfg,
+                                                                   int n_taps, int center, float* __restrict__ grad) {
+   using P = R16Plan<LEN>;
+   extern __shared__ float2 sm[];
+   const int lt = threadIdx.x;
+   float2 v[16];
+#pragma unroll
+   for (int r = 0; r < 16; ++r) v[r] = spec[lt + r * (LEN / 16)];
+   r16_forward<LEN>(v, sm, lt, cfg.twp);
+#pragma unroll
+   for (int b = 0; b < 16 / P::R3; ++b)
+#pragma unroll
+      for (int r = 0; r < P::R3; ++r) {
+         const int j = (r16_time_index<LEN>(lt, b, r) + center) & (LEN - 1);  // tap j sits at lag (j - center) mod len
+         if (j < n_taps) grad[j] = v[b * P::R3 + r].x * (1.0f / (float)LEN);
+      }
+}
+
+template <int LEN>
+cudaError_t launch_grad_finish_r16(const float2* spec, const FilterCfg& cfg, int n_taps, int center, float* grad,
+                                   cudaStream_t st) {
+   filter_grad_finish_r16<LEN><<<1, LEN / 16, sizeof(float2) * (LEN + LEN / 16), st>>>(spec, cfg, n_taps, center, grad);
+   return cudaGetLastError();
 }
 
 
@@ -528,7 +565,14 @@ cudaError_t launch_filter_taps_grad(const float* x, const float* g, int batch, c
    }
    if (e != cudaSuccess) return e;
    float2* spec = workspace + (size_t)gp.blocks * cfg.len;
-   filter_grad_sum<<<(cfg.len + kThreads - 1) / kThreads, kThreads, 0, st>>>(workspace, gp.blocks, cfg.len, spec);
+   filter_grad_sum<<<cfg.len / 32, kThreads, 0, st>>>(workspace, gp.blocks, cfg.len, spec);
+   switch (cfg.twp ? cfg.len : 0) {
+      case 512: return launch_grad_finish_r16<512>(spec, cfg, n_taps, center, grad_taps, st);
+      case 1024: return launch_grad_finish_r16<1024>(spec, cfg, n_taps, center, grad_taps, st);
+      case 2048: return launch_grad_finish_r16<2048>(spec, cfg, n_taps, center, grad_taps, st);
+      case 4096: return launch_grad_finish_r16<4096>(spec, cfg, n_taps, center, grad_taps, st);
+      default: break;
+   }
    const size_t smem2 = sizeof(float2) * 2 * (size_t)cfg.len;
    e = cudaFuncSetAttribute(filter_grad_finish, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
    if (e != cudaSuccess) return e;
