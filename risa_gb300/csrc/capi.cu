@@ -264,6 +264,7 @@ struct risa_gb_backprojection {
       c.colbase = colbase.as<float2>();
       c.tile_win = tile_win.as<int2>();
       c.patch = &patch;
+      c.few = reserved_batch <= 2;
       c.patch_angles = patch_angles.as<BPPatchAngle>();
       c.adj_scratch = adj.p;
       c.adj_scratch_bytes = adj.bytes;
@@ -272,7 +273,12 @@ struct risa_gb_backprojection {
    // Pair buffer for `batch` slices under every variant. Only set-up calls
    // (create of the engine, reserve, autotune) allocate; an enqueue whose
    // batch exceeds the reservation runs a variant that needs no pair buffer.
+   // The largest reservation also says how the handle is used: up to two slices
+   // take the patch kernel's form for single frames, whatever a call's batch, so
+   // that the calls of one handle give the same bits however a job is cut.
+   int reserved_batch = 0;
    risa_gb_status reserve(int batch) {
+      reserved_batch = std::max(reserved_batch, batch);
       size_t need = 0;
       for (int v = 0; v < bp_variant_count(); ++v)
          need = std::max(need, bp_pairs_bytes(v, batch, g.Pp, g.Dp, std::max(win_len[0], win_len[1])));
@@ -1082,7 +1088,8 @@ static cudaError_t engine_filter_bp(risa_gb_fbp* h, float* par, float* img, int 
    const int v = h->bp->variant_for(batch, fused);
    BPCfg c = h->bp->cfg(fused);
    cudaError_t e;
-   if (bp_variant_layout(v) != kLayoutNone && filter_pairs_supported(fc)) {
+   const bool rows = v == bp_patch_variant() && bp_patch_rows_ok(c, par, batch);
+   if (!rows && bp_variant_layout(v) != kLayoutNone && filter_pairs_supported(fc)) {
       e = launch_filter_pairs(par, batch, fc, PairsOut{c.pairs, bp_variant_pair_slices(v), c.win_lo, c.win_len}, st);
       c.prefilled = true;
    } else {
@@ -1120,7 +1127,9 @@ static cudaError_t engine_streaming(risa_gb_fbp* h, const uint16_t* raw, int pla
 static bool two_lanes(const risa_gb_fbp* h, int batch) {
    if (h->lanes < 2 || h->p.normalize || h->p.interp != RISA_GB_INTERP_LINEAR) return false;
    const bool fused = h->p.masking && !h->p.normalize;
-   return bp_variant_layout(h->bp->variant_for(batch, fused)) != kLayoutNone && filter_pairs_supported(h->filt->cfg());
+   const int v = h->bp->variant_for(batch, fused);
+   if (v == bp_patch_variant() && bp_patch_rows_ok(h->bp->cfg(fused), h->par.as<float>(), batch)) return false;
+   return bp_variant_layout(v) != kLayoutNone && filter_pairs_supported(h->filt->cfg());
 }
 
 // The second pair buffer, the capture lane (highest stream priority) and its

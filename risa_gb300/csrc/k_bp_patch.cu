@@ -39,6 +39,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 
 #include "async_copy.h"
 #include "f32x2.cuh"
@@ -62,10 +63,12 @@ struct PatchArgs {
    float norm, mask_value;
    int masking;
 };
-struct PatchPlanParam {
-   float A[kPatchAngles], B[kPatchAngles];
+struct PatchSegs {
    uint32_t seg[kPatchMaxSegs];
    int n_segs;
+};
+struct PatchPlanParam : PatchSegs {
+   float A[kPatchAngles], B[kPatchAngles];
 };
 
 typedef unsigned long long u64;
@@ -94,6 +97,25 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
            "r"(async::smem_u32(dst)),
        "l"(map), "r"(async::smem_u32(bar)), "r"(x), "r"(y), "r"(z)
        : "memory");
+}
+
+// Window of an angle for a tile whose lowest coordinate is at pixel (cx, cy):
+// its first bin w0 (a multiple of ALIGN) and the lowest coordinate relative to
+// it, t0 + cx a + cy b - w0 >= 0. Error-free FP32 sums and products of the (hi,
+// lo) coefficients keep ~2^-40 of a bin; FP64 has few units per SM (one slice of
+// 1024 x 1024 -> 512^2: 148 us with FP64 windows, 142 with these).
+template <int ALIGN>
+__device__ __forceinline__ void patch_window(const BPPatchAngle& t, int cx, int cy, int* w0, float* rel) {
+   const float x = (float)cx, y = (float)cy;
+   const float p = __fmul_rn(x, t.a_hi), q = __fmul_rn(y, t.b_hi);
+   const float pe = fmaf(x, t.a_lo, fmaf(x, t.a_hi, -p)), qe = fmaf(y, t.b_lo, fmaf(y, t.b_hi, -q));
+   const float s = __fadd_rn(t.t0_hi, p), sv = __fsub_rn(s, t.t0_hi);
+   const float se = __fadd_rn(__fsub_rn(t.t0_hi, __fsub_rn(s, sv)), __fsub_rn(p, sv));
+   const float u = __fadd_rn(s, q), uv = __fsub_rn(u, s);
+   const float ue = __fadd_rn(__fsub_rn(s, __fsub_rn(u, uv)), __fsub_rn(q, uv));
+   const float lo = __fadd_rn(__fadd_rn(se, ue), __fadd_rn(__fadd_rn(pe, qe), t.t0_lo));
+   *w0 = (int)floorf(__fadd_rn(u, lo)) & ~(ALIGN - 1);
+   *rel = fmaxf(__fadd_rn(__fsub_rn(u, (float)*w0), lo), 0.f);
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -170,7 +192,8 @@ __device__ __noinline__ void patch_general_tile(const PatchArgs& g, int q0, int 
       float acc[4] = {0.f, 0.f, 0.f, 0.f};
       for (int a = 0; a < g.Pp && !out; ++a) {
          const BPPatchAngle t = g.ang[a];
-         const double s = t.t0 + (double)x * t.a + (double)y * t.b;
+         const double s = ((double)t.t0_hi + (double)t.t0_lo) + (double)x * ((double)t.a_hi + (double)t.a_lo) +
+                          (double)y * ((double)t.b_hi + (double)t.b_lo);
          const double fl = floor(s);
          const float f = (float)(s - fl) - 0.5f;
          const int k = (int)fl;
@@ -250,12 +273,8 @@ __global__ void __launch_bounds__(64 * QL + 32, MINB)
             float rel = 0.f;
             int w0 = 0, ang = 0;
             if (lane < na) {
-               // the lowest coordinate of the tile's pixels
                const BPPatchAngle t = g.ang[pos + a0 + lane];
-               const double base = t.t0 + (double)cx * t.a + (double)cy * t.b;
-               const double fl = floor(base);
-               w0 = (int)fl;
-               rel = (float)(base - fl);
+               patch_window<1>(t, cx, cy, &w0, &rel);
                ang = t.index;
             }
             if (round > 0 && !__all_sync(~0u, async::mbar_wait(&empty[st], (round - 1) & 1u, g.err, 5))) {
@@ -328,7 +347,7 @@ __global__ void __launch_bounds__(64 * QL + 32, MINB)
                   const float v = tm + kMagic;
                   const float f = tm - (v - kMagic);
                   const uint32_t addr = stage + (uint32_t)ai * angle_bytes + ((uint32_t)__float_as_int(v) << 4);
-                  patch_angle<(CL >> 4) & 1, (CL >> 3) & 1, CL & 3, SQ, PRED>(addr, pitch * QL, f, A, B, acc);
+                  patch_angle<(CL >> 3), (CL >> 2) & 1, CL & 3, SQ, PRED>(addr, pitch * QL, f, A, B, acc);
                };
                if (n - a0 >= ACH) {
 #pragma unroll 1
@@ -348,14 +367,14 @@ __global__ void __launch_bounds__(64 * QL + 32, MINB)
                if (++st == NST) st = 0, phase ^= 1u;
             }
          };
-         switch ((d >> 24) & 15u) {  // bits of the class: MA << 4 | MB << 3 | MAB
+         switch ((d >> 24) & 15u) {  // class: MA << 3 | MB << 2 | MAB
             case 0: run(std::integral_constant<int, 0>{}); break;
             case 1: run(std::integral_constant<int, 1>{}); break;
-            case 2: run(std::integral_constant<int, 8 + 1>{}); break;
-            case 3: run(std::integral_constant<int, 8 + 2>{}); break;
-            case 4: run(std::integral_constant<int, 16 + 1>{}); break;
-            case 5: run(std::integral_constant<int, 16 + 2>{}); break;
-            default: run(std::integral_constant<int, 16 + 8 + 2>{}); break;
+            case 5: run(std::integral_constant<int, 5>{}); break;
+            case 6: run(std::integral_constant<int, 6>{}); break;
+            case 9: run(std::integral_constant<int, 9>{}); break;
+            case 10: run(std::integral_constant<int, 10>{}); break;
+            default: run(std::integral_constant<int, 14>{}); break;
          }
       }
       if (!ok) s_fail = 1;
@@ -384,6 +403,234 @@ __global__ void __launch_bounds__(64 * QL + 32, MINB)
                if (sl < g.batch) g.img[((size_t)sl * N + y) * N + x] = out ? g.mask_value : v[j] * g.norm;
             }
          }
+}
+
+// ---- one or two slices: the same patches over the sinogram itself ------------
+// A frame at a time there are no slices to share a pixel's weights and a 16 x 16
+// tile is 64 patches, too few warps to hide the shared-memory latency. Here the
+// G groups of a CTA take the angles of a chunk in turn over the same patches and
+// add their sums in group order at the end, the rows come straight from the
+// sinogram (no staging pass; windows start at a multiple of 4 bins, as the copy
+// needs), and a pixel reads its two bins by selecting the outer one, so
+// infinities and NaN stay where the general kernel leaves them.
+// A stage is refilled by all working warps: with one producer warp as
+// in bp_patch the same loop took 141 us, with 16-byte cp.async pieces instead of a
+// box per angle 134. One slice of 1024 x 1024 -> 512^2: 119 us (quads 263,
+// pairs_s1_a32 229); 512 x 256 -> 256^2: 28 us (66, 80). Bound by issue: about 40
+// instructions per patch and angle.
+constexpr int kRowsACH = 64;
+
+struct RowsArgs {
+   const BPPatchAngle* ang;
+   const float* sino;
+   float* img;
+   int* err;
+   int N, Pp, Dp, wlen;
+   float norm, mask_value;
+   int masking;
+};
+
+__device__ __forceinline__ float lds_f32(uint32_t addr) {
+   float v;
+   asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+   return v;
+}
+
+// off: the offset pixels' coordinates relative to their middle bins at f = 0.
+template <int MA, int MB, int MAB, int S>
+__device__ __forceinline__ void rows_angle(uint32_t addr, uint32_t sstep, float f, float4 off, float (&acc)[S][4]) {
+   constexpr int m[4] = {0, MA, MB, MAB};
+   const float r[4] = {0.f, f + off.x, f + off.y, f + off.z};
+#pragma unroll
+   for (int s = 0; s < S; ++s) {
+      float q[MAB + 3];
+#pragma unroll
+      for (int e = 0; e < MAB + 3; ++e) q[e] = lds_f32(addr + (uint32_t)s * sstep + (uint32_t)e * 4u);
+      acc[s][0] = fmaf(0.5f - f, q[0], acc[s][0]);
+      acc[s][0] = fmaf(0.5f + f, q[1], acc[s][0]);
+#pragma unroll
+      for (int p = 1; p < 4; ++p) {
+         const float outer = r[p] < 0.f ? q[m[p]] : q[m[p] + 2];
+         acc[s][p] = fmaf(1.f - fabsf(r[p]), q[m[p] + 1], acc[s][p]);
+         acc[s][p] = fmaf(fabsf(r[p]), outer, acc[s][p]);
+      }
+   }
+}
+
+template <int S, int G>
+__global__ void __launch_bounds__(64 * G)
+    bp_patch_rows(const __grid_constant__ CUtensorMap map, const __grid_constant__ RowsArgs g,
+                  const __grid_constant__ PatchSegs pp) {
+   constexpr int ACH = kRowsACH;
+   extern __shared__ __align__(128) unsigned char smem_raw[];
+   __shared__ uint64_t full[2], empty[2];
+   // per angle: (|a|, |b|, window-relative coordinate - 1/2), then rows_angle's offsets
+   __shared__ float4 s_par[2][ACH][2];
+   __shared__ volatile int s_fail;
+
+   const int N = g.N;
+   const int x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile;
+   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+   const float c = 0.5f * (float)(N - 1);
+   const float lim = (float)N * (float)N * 0.25f;
+   auto inside = [&](int xa, int ya, int w, int h) {
+      const float nx = fminf(fmaxf(c, (float)xa), (float)(xa + w - 1)) - c;
+      const float ny = fminf(fmaxf(c, (float)ya), (float)(ya + h - 1)) - c;
+      return !g.masking || nx * nx + ny * ny <= lim;
+   };
+   // a group's two warps cover 16 x 8 pixels each; halves outside the circle are left out
+   const bool live0 = inside(x0, y0, kTile, kTile / 2), live1 = inside(x0, y0 + kTile / 2, kTile, kTile / 2);
+   const int halves = (int)live0 + (int)live1, L = G * halves;  // working warps
+   const uint32_t row_bytes = (uint32_t)g.wlen * 4u, angle_bytes = row_bytes * S;
+   if (threadIdx.x == 0) {
+      for (int i = 0; i < 2; ++i) {
+         async::mbar_init(&full[i], max(L, 1));
+         async::mbar_init(&empty[i], max(L, 1));
+      }
+      s_fail = 0;
+      async::mbar_init_fence();
+   }
+   __syncthreads();
+
+   float acc[S][4];
+#pragma unroll
+   for (int s = 0; s < S; ++s)
+#pragma unroll
+      for (int p = 0; p < 4; ++p) acc[s][p] = 0.f;
+   const int group = warp >> 1;
+   const int xp = 2 * ((lane & 3) + ((lane >> 1) & 4));
+   const int yp = (warp & 1) * 8 + 2 * (((lane >> 2) & 1) + ((lane >> 3) & 2));
+
+   if ((warp & 1) ? live1 : live0) {
+      const int rank = halves == 2 ? warp : group;
+      // Refill of a stage with one chunk (angles a0 .. a0 + ACH - 1 of run `d`):
+      // every working warp forms the windows of its angles (rank + j L, one per
+      // lane) and issues their copies.
+      auto refill = [&](uint32_t d, int a0, int st) {
+         const int pos = (int)(d & 0xFFFu), na = min(ACH, (int)((d >> 12) & 0xFFFu) - a0);
+         const int mine = na > rank ? (na - rank + L - 1) / L : 0;
+         int w0 = 0, row = 0;
+         if (lane < mine) {
+            const int a = rank + lane * L;
+            const BPPatchAngle t = g.ang[pos + a0 + a];
+            float rel;
+            patch_window<4>(t, x0 + ((d >> 28) & 1u ? kTile - 1 : 0), y0 + ((d >> 29) & 1u ? kTile - 1 : 0), &w0, &rel);
+            row = t.index;
+            const float A = fabsf(t.a_hi), B = fabsf(t.b_hi);
+            const uint32_t cls = (d >> 24) & 15u;
+            s_par[st][a][0] = make_float4(A, B, rel - 0.5f, 0.f);
+            s_par[st][a][1] = make_float4(A - ((float)(cls >> 3) + 0.5f), B - ((float)((cls >> 2) & 1u) + 0.5f),
+                                          (A + B) - ((float)(cls & 3u) + 0.5f), 0.f);
+         }
+         __syncwarp();
+         if (lane == 0) async::mbar_arrive_expect_tx(&full[st], (uint32_t)mine * angle_bytes);
+         __syncwarp();
+         if (lane < mine)
+            tma_load_3d(smem_raw + (size_t)(st * ACH + rank + lane * L) * angle_bytes, &map, &full[st], w0, row, 0);
+      };
+      const uint32_t sbase = async::smem_u32(smem_raw) - ((uint32_t)kMagicBits << 2);
+      uint32_t signs = 0;
+      auto flip1 = [&](uint32_t f) {
+#pragma unroll
+         for (int s = 0; s < S; ++s) {
+            float* v = acc[s];
+            float t;
+            if (f & 1u) t = v[0], v[0] = v[1], v[1] = t, t = v[2], v[2] = v[3], v[3] = t;
+            if (f & 2u) t = v[0], v[0] = v[2], v[2] = t, t = v[1], v[1] = v[3], v[3] = t;
+         }
+      };
+      refill(pp.seg[0], 0, 0);
+      int ch = 0;  // chunks done
+      bool ok = true;
+      for (int si = 0; si < pp.n_segs && ok; ++si) {
+         const uint32_t d = pp.seg[si];
+         const int n = (int)((d >> 12) & 0xFFFu);
+         const uint32_t sg = (d >> 28) & 3u;
+         flip1(sg ^ signs);
+         signs = sg;
+         const float fx = (float)((sg & 1u) ? kTile - 2 - xp : xp), fy = (float)((sg & 2u) ? kTile - 2 - yp : yp);
+         auto run = [&](auto cls) {
+            constexpr int CL = decltype(cls)::value;
+#pragma unroll 1
+            for (int a0 = 0; a0 < n; a0 += ACH, ++ch) {
+               const int st = ch & 1;
+               // the next chunk into the other stage, once every warp has left it
+               const bool more = a0 + ACH < n;
+               if (more || si + 1 < pp.n_segs) {
+                  if (ch > 0 && !async::mbar_wait(&empty[st ^ 1], (uint32_t)((ch - 1) >> 1) & 1u, g.err, 5)) {
+                     ok = false;
+                     break;
+                  }
+                  refill(more ? d : pp.seg[si + 1], more ? a0 + ACH : 0, st ^ 1);
+               }
+               if (!async::mbar_wait(&full[st], (uint32_t)(ch >> 1) & 1u, g.err, 5)) {
+                  ok = false;
+                  break;
+               }
+               const uint32_t stage = sbase + (uint32_t)(st * ACH) * angle_bytes;
+               auto angle = [&](int ai) {
+                  const float4 q = s_par[st][ai][0], off = s_par[st][ai][1];
+                  const float tm = fmaf(fy, q.y, fmaf(fx, q.x, q.z));
+                  const float v = tm + kMagic;
+                  const float f = tm - (v - kMagic);
+                  const uint32_t addr = stage + (uint32_t)ai * angle_bytes + ((uint32_t)__float_as_int(v) << 2);
+                  rows_angle<(CL >> 3), (CL >> 2) & 1, CL & 3, S>(addr, row_bytes, f, off, acc);
+               };
+               const int na = min(ACH, n - a0);
+               int ai = group;
+#pragma unroll 1
+               for (; ai + 3 * G < na; ai += 4 * G) {
+                  angle(ai);
+                  angle(ai + G);
+                  angle(ai + 2 * G);
+                  angle(ai + 3 * G);
+               }
+#pragma unroll 1
+               for (; ai < na; ai += G) angle(ai);
+               __syncwarp();
+               if (lane == 0) mbar_arrive(&empty[st]);
+            }
+         };
+         switch ((d >> 24) & 15u) {  // as in bp_patch
+            case 0: run(std::integral_constant<int, 0>{}); break;
+            case 1: run(std::integral_constant<int, 1>{}); break;
+            case 5: run(std::integral_constant<int, 5>{}); break;
+            case 6: run(std::integral_constant<int, 6>{}); break;
+            case 9: run(std::integral_constant<int, 9>{}); break;
+            case 10: run(std::integral_constant<int, 10>{}); break;
+            default: run(std::integral_constant<int, 14>{}); break;
+         }
+      }
+      if (!ok) s_fail = 1;
+      flip1(signs);
+   }
+   __syncthreads();  // the stages are no longer read
+   if (s_fail) {  // a wait gave up: let the copies in flight land, leave without output
+      if (threadIdx.x == 0 && L > 0)
+         for (int i = 0; i < 2; ++i)
+            for (uint32_t ph = 0; ph < 2; ++ph) async::mbar_wait_quiet(&full[i], ph);
+      return;
+   }
+   float* sums = reinterpret_cast<float*>(smem_raw);  // [group][slice][pixel of the tile]
+#pragma unroll
+   for (int s = 0; s < S; ++s)
+#pragma unroll
+      for (int p = 0; p < 4; ++p)
+         sums[(group * S + s) * kTile * kTile + (yp + (p >> 1)) * kTile + xp + (p & 1)] = acc[s][p];
+   __syncthreads();
+   for (int i = threadIdx.x; i < S * kTile * kTile; i += 64 * G) {
+      float v = sums[i];
+#pragma unroll
+      for (int k = 1; k < G; ++k) v += sums[k * S * kTile * kTile + i];
+      const int s = i / (kTile * kTile), x = x0 + i % kTile, y = y0 + (i / kTile) % kTile;
+      if (x >= N || y >= N) continue;
+      v *= g.norm;
+      if (g.masking) {
+         const float dx = (float)x - c, dy = (float)y - c;
+         if (dx * dx + dy * dy > lim) v = g.mask_value;
+      }
+      g.img[((size_t)s * N + y) * N + x] = v;
+   }
 }
 
 // Staged rows from a plain sinogram: quads[q][angle][bin] = slices 4q .. 4q + 3
@@ -456,12 +703,42 @@ cudaError_t launch_patch(const PatchArgs& args, const PatchPlanParam& pp, float 
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return cudaErrorInvalidValue;
    auto kern = bp_patch<SQ, QL, ACH, NST, MINB, PRED>;
-   if (smem > 48 * 1024) {
+   if (smem > 47 * 1024) {  // with the kernel's static shared memory
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
    }
    const int t = (a.N + kTile - 1) / kTile;
    kern<<<dim3(t, t, (a.n_quads + SQ * QL - 1) / (SQ * QL)), 64 * QL + 32, smem, st>>>(map, a, pp);
+   return cudaGetLastError();
+}
+
+template <int S, int G>
+cudaError_t launch_rows(const RowsArgs& args, const PatchSegs& pp, const BPCfg& cfg,
+                        cudaStream_t st) {
+   RowsArgs a = args;
+   const int need = (int)std::floor((kTile - 2) * 1.41421357 * (double)cfg.scale + 4.01) + 3 +
+                    std::min(2, (int)std::floor(1.41421357 * (double)cfg.scale));
+   a.wlen = need <= 32 ? 32 : 64;
+   const size_t smem = std::max((size_t)2 * kRowsACH * S * a.wlen * 4, (size_t)G * S * kTile * kTile * 4);
+   if (need > 64 || smem > 220 * 1024) return cudaErrorInvalidConfiguration;
+   EncodeTiled enc = encode_fn();
+   if (!enc) return cudaErrorNotSupported;
+   CUtensorMap map;
+   const cuuint64_t dims[3] = {(cuuint64_t)a.Dp, (cuuint64_t)a.Pp, (cuuint64_t)S};
+   const cuuint64_t strides[2] = {(cuuint64_t)a.Dp * 4, (cuuint64_t)a.Pp * a.Dp * 4};
+   const cuuint32_t box[3] = {(cuuint32_t)a.wlen, 1, (cuuint32_t)S};
+   const cuuint32_t estr[3] = {1, 1, 1};
+   if (enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, const_cast<float*>(a.sino), dims, strides, box, estr,
+           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+      return cudaErrorInvalidValue;
+   auto kern = bp_patch_rows<S, G>;
+   if (smem > 47 * 1024) {  // with the kernel's static shared memory
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+   }
+   const int t = (a.N + kTile - 1) / kTile;
+   kern<<<dim3(t, t), 64 * G, smem, st>>>(map, a, pp);
    return cudaGetLastError();
 }
 }  // namespace
@@ -473,6 +750,10 @@ bool bp_patch_plan(const float* a, const float* b, const double* ad, const doubl
    struct Key {
       int group, index;
    };
+   auto split = [](double v, float* hi, float* lo) {
+      *hi = (float)v;
+      *lo = (float)(v - (double)*hi);
+   };
    std::vector<Key> keys(Pp);
    for (int i = 0; i < Pp; ++i) {
       const float A = std::fabs(a[i]), B = std::fabs(b[i]);
@@ -481,7 +762,7 @@ bool bp_patch_plan(const float* a, const float* b, const double* ad, const doubl
       // the offset lies in [m, m + 1]; at an integer either end serves
       const int mab = std::min({(int)(A + B), 2, ma + mb + 1});
       if (A + B - (float)mab > 1.f) return false;
-      const int cls = ma == 0 && mb == 0 ? mab : 1 + ma * 2 + mb + (ma + mb == 1 ? (ma ? 1 : 0) + (mab - 1) : 2);
+      const int cls = ma << 3 | mb << 2 | mab;
       keys[i] = {((a[i] < 0.f ? 1 : 0) + (b[i] < 0.f ? 2 : 0)) * 16 + cls, i};
    }
    std::stable_sort(keys.begin(), keys.end(), [](const Key& x, const Key& y) { return x.group < y.group; });
@@ -493,7 +774,13 @@ bool bp_patch_plan(const float* a, const float* b, const double* ad, const doubl
       i += n;
    }
    for (const Key& k : keys) {
-      plan->angles.push_back(BPPatchAngle{t0[k.index], ad[k.index], bd[k.index], k.index, 0});
+      BPPatchAngle t;
+      split(t0[k.index], &t.t0_hi, &t.t0_lo);
+      split(ad[k.index], &t.a_hi, &t.a_lo);
+      split(bd[k.index], &t.b_hi, &t.b_lo);
+      t.index = k.index;
+      t.pad = 0;
+      plan->angles.push_back(t);
       plan->A.push_back(std::fabs(a[k.index]));
       plan->B.push_back(std::fabs(b[k.index]));
    }
@@ -507,9 +794,31 @@ size_t bp_quads_bytes(int batch, int Pp, int Dp) {
    return sizeof(float4) * quads * Pp * Dp + sizeof(int) * quads;
 }
 
+bool bp_patch_rows_ok(const BPCfg& cfg, const float* sino, int batch) {
+   return cfg.few && batch <= 2 && cfg.patch && !cfg.patch->angles.empty() && cfg.Dp % 4 == 0 &&
+          (reinterpret_cast<uintptr_t>(sino) & 15) == 0;
+}
+
 cudaError_t launch_bp_patch(const float* sino, float* img, int batch, const BPCfg& cfg, cudaStream_t st) {
    if (!cfg.patch || cfg.patch->angles.empty() || !cfg.patch_angles || !cfg.err) return cudaErrorInvalidConfiguration;
+   PatchPlanParam pp;
+   std::memcpy(pp.seg, cfg.patch->segs.data(), sizeof(uint32_t) * cfg.patch->segs.size());
+   pp.n_segs = (int)cfg.patch->segs.size();
+   cudaError_t e = cudaSuccess;
+   if (!cfg.prefilled && bp_patch_rows_ok(cfg, sino, batch)) {
+      if (cfg.mid_event && (e = cudaEventRecord(cfg.mid_event, st)) != cudaSuccess) return e;
+      const RowsArgs r{cfg.patch_angles, sino, img, cfg.err, cfg.N, cfg.Pp, cfg.Dp, 0, cfg.norm, cfg.mask_value, cfg.masking};
+      // Groups of angles per CTA: two keep a chunk's refill small beside its work;
+      // four where the tiles alone are too few warps (one slice, groups of 2 / 4 /
+      // 8: 512^2 119 / 130 / 145 us, 256^2 36 / 28 / 30).
+      const long tiles = (long)((cfg.N + kTile - 1) / kTile) * ((cfg.N + kTile - 1) / kTile);
+      if (tiles >= 600)
+         return batch == 1 ? launch_rows<1, 2>(r, pp, cfg, st) : launch_rows<2, 2>(r, pp, cfg, st);
+      return batch == 1 ? launch_rows<1, 4>(r, pp, cfg, st) : launch_rows<2, 4>(r, pp, cfg, st);
+   }
    if (!cfg.pairs || bp_quads_bytes(batch, cfg.Pp, cfg.Dp) > cfg.pairs_bytes) return cudaErrorInvalidValue;
+   std::memcpy(pp.A, cfg.patch->A.data(), sizeof(float) * cfg.Pp);
+   std::memcpy(pp.B, cfg.patch->B.data(), sizeof(float) * cfg.Pp);
    const int nq = (batch + 3) / 4;
    float4* quads = static_cast<float4*>(cfg.pairs);
    int* flags = reinterpret_cast<int*>(quads + (size_t)nq * cfg.Pp * cfg.Dp);
@@ -527,12 +836,6 @@ cudaError_t launch_bp_patch(const float* sino, float* img, int batch, const BPCf
    a.norm = cfg.norm;
    a.mask_value = cfg.mask_value;
    a.masking = cfg.masking;
-   PatchPlanParam pp;
-   std::memcpy(pp.A, cfg.patch->A.data(), sizeof(float) * cfg.Pp);
-   std::memcpy(pp.B, cfg.patch->B.data(), sizeof(float) * cfg.Pp);
-   std::memcpy(pp.seg, cfg.patch->segs.data(), sizeof(uint32_t) * cfg.patch->segs.size());
-   pp.n_segs = (int)cfg.patch->segs.size();
-   cudaError_t e = cudaSuccess;
    if (!cfg.prefilled) {
       if ((e = cudaMemsetAsync(flags, 0, sizeof(int) * nq, st)) != cudaSuccess) return e;
       bp_quads_fill<<<dim3((cfg.Dp + 255) / 256, cfg.Pp, nq), 256, 0, st>>>(sino, quads, flags, batch, cfg.Pp, cfg.Dp);

@@ -249,7 +249,8 @@ constexpr int kCPAngles = 2048;  // angles the backprojection can take from its 
 constexpr int kPatchAngles = 2048;
 constexpr int kPatchMaxSegs = 32;  // at most 7 classes for each of the 4 sign pairs
 struct BPPatchAngle {
-   double t0, a, b;
+   // t = t0 + x a + y b, each coefficient the sum of two floats (48 bits)
+   float t0_hi, t0_lo, a_hi, a_lo, b_hi, b_lo;
    int index, pad;  // the angle's row
 };
 struct BPPatchPlan {
@@ -289,6 +290,7 @@ struct BPCfg {
    const int2* tile_win = nullptr;  // staged variants: per tile and angle (window start, bits of the float
                                     // coordinate of the tile origin in it), bp_tile_windows; else FP64 on device
    const BPPatchPlan* patch = nullptr;  // host side
+   bool few = false;  // a caller of one or two slices at a time: the patch kernel over the sinogram itself
    const BPPatchAngle* patch_angles = nullptr;
    void* adj_scratch = nullptr;  // adjoint: slice-interleaved image copies (bp_adjoint_scratch_bytes)
    size_t adj_scratch_bytes = 0;
@@ -322,6 +324,8 @@ enum BPLayout { kLayoutNone, kLayoutPairs, kLayoutQuads };
 BPLayout bp_variant_layout(int variant);
 cudaError_t launch_bp_patch(const float* sino, float* img, int batch, const BPCfg& cfg, cudaStream_t st);
 int bp_patch_variant();  // its place in the variant list
+// Whether the patch kernel reads this sinogram itself (no staged rows).
+bool bp_patch_rows_ok(const BPCfg& cfg, const float* sino, int batch);
 cudaError_t launch_backprojection(const float* sino, float* img, int batch, const BPCfg& cfg,
                                   int variant, cudaStream_t st);
 cudaError_t launch_backprojection_adjoint(const float* img, float* sino, int batch,

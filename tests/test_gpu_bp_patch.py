@@ -90,6 +90,31 @@ def test_patch_angle_limits():
         assert mr < MAX_REL, (Pp, Dp, N, mr)
 
 
+@pytest.mark.parametrize("N,Dp,Pp", [(97, 96, 150), (97, 132, 97), (64, 128, 130), (33, 12, 65), (400, 400, 70),
+                                     (41, 41, 20)])
+def test_patch_single_frames(N, Dp, Pp):
+    """Handles that were never reserved for more than two slices read the
+    sinogram itself (four and two groups of angles; chunks of 64 angles with
+    partial ones; Dp % 4 != 0 takes the staged quads): the oracle's values, and
+    the same bits for two slices at once and one by one."""
+    for rot in (0.0, 143.0):
+        g = rg.make_geometry(n_par_proj=Pp, n_par_det=Dp, n_pixels=N, rotation_offset=rot)
+        bp = rg.Backprojection(g, rg.make_params(masking=True, masking_value=2.0))
+        sino, _ = phantom.parallel_sinograms(2, Pp, Dp, 200.0, seed=Pp)
+        t = torch.from_numpy(sino).cuda()
+        got = _run(bp, t, N, 2)
+        for b in range(2):
+            mr, _ = rel_err(got[b], oracle.mask(oracle.backproject(sino[b], N, rot), 2.0))
+            assert mr < MAX_REL, (rot, b, mr)
+            one = _run(bp, t[b:b + 1].contiguous(), N, 1)
+            np.testing.assert_array_equal(one[0].view(np.uint32), got[b].view(np.uint32))
+        # an unaligned sinogram takes the staged quads
+        shifted = torch.empty(sino.size + 1, dtype=torch.float32, device="cuda")[1:].view(sino.shape)
+        shifted.copy_(t)
+        mr, _ = rel_err(_run(bp, shifted, N, 2)[1], got[1])
+        assert mr < MAX_REL, mr
+
+
 @pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan])
 @pytest.mark.parametrize("n", [1, 6, 40])
 def test_patch_nonfinite_rows(value, n):
