@@ -233,7 +233,17 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
                atomicCAS(A.err, 0, 4);
                u0 = min(max(u0, 0), I.win_len - W) & ~1;
             }
-            S.par[st][l] = make_float4(a, b, rel, 0.f);
+            // The angle loop indexes the window without a bounds test: every
+            // coordinate of the tile lies well inside it (host-built windows
+            // keep a margin of two bins either side), or the angle is recorded
+            // as an error and reads entry 0.
+            const float lo = rel + fminf(0.f, 31.f * a) + fminf(0.f, 31.f * b);
+            const float hi = rel + fmaxf(0.f, 31.f * a) + fmaxf(0.f, 31.f * b);
+            if (!(lo >= 0.25f && hi <= (float)W - 1.25f)) {
+               atomicCAS(A.err, 0, 4);
+               a = b = rel = 0.f;
+            }
+            S.par[st][l] = make_float4(a, b, rel, 2.f * (float)RS * b);
             async::bulk_load(wsm + (size_t)(st * ACH + l) * W, prow + (size_t)ang * I.win_len + u0,
                              win_bytes, &full[st]);
          }
@@ -247,7 +257,6 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
 #pragma unroll
       for (int r = 0; r < PPT; ++r) acc[r] = 0.f;
       const uint32_t wbase = async::smem_u32(wsm);
-      const unsigned wmax = (unsigned)(W - 1);
       const unsigned long long magic2 = f2_pack(kSweepMagic, kSweepMagic);
       bool failed = false;
       // Bit r: the warp's 8 x 4 pixel block of step r lies (partly) in the
@@ -271,18 +280,19 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
          if (!async::mbar_wait(&full[st], uses[st] & 1u, A.err, 5)) S.fail = 1;
          ++uses[st];
          const int na = live ? min(ACH, Pp - ch * ACH) : 0;
+         // the rounded coordinate's bits less the magic constant's are the entry
+         const uint32_t cbase = wbase + (uint32_t)(st * ACH * W) * (uint32_t)sizeof(float2) -
+                                ((uint32_t)kSweepMagicBits << 3);
 #pragma unroll 8
          for (int ai = 0; ai < na; ++ai) {
             const float4 q = S.par[st][ai];  // one broadcast load per angle
             const float a = q.x, b = q.y;
             const float tm = q.z + (float)xo * a + (float)yo * b;
-            const float step = (float)RS * b;
-            const uint32_t abase = wbase + (uint32_t)((st * ACH + ai) * W) * (uint32_t)sizeof(float2);
+            const uint32_t abase = cbase + (uint32_t)(ai * W) * (uint32_t)sizeof(float2);
             // pixel steps (r, r + 1) as one f32x2 pair: the ray coordinate,
             // its rounding and the fraction take one instruction per pair
-            unsigned long long t2 = f2_pack(tm, tm + step);
-            const float step2 = 2.f * step;
-            const unsigned long long dt2 = f2_pack(step2, step2);
+            unsigned long long t2 = f2_pack(tm, fmaf((float)RS, b, tm));
+            const unsigned long long dt2 = f2_pack(q.w, q.w);
 #pragma unroll
             for (int r = 0; r < PPT; r += 2) {
                const unsigned long long v2 = f2_add(t2, magic2);
@@ -290,10 +300,8 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
                float v0, v1, f0, f1;
                f2_unpack(v2, v0, v1);
                f2_unpack(fr2, f0, f1);
-               const unsigned k0 = min((unsigned)(__float_as_int(v0) - kSweepMagicBits), wmax);
-               const unsigned k1 = min((unsigned)(__float_as_int(v1) - kSweepMagicBits), wmax);
-               const float2 p0 = lds64(abase + k0 * (uint32_t)sizeof(float2));
-               const float2 p1 = lds64(abase + k1 * (uint32_t)sizeof(float2));
+               const float2 p0 = lds64(abase + ((uint32_t)__float_as_int(v0) << 3));
+               const float2 p1 = lds64(abase + ((uint32_t)__float_as_int(v1) << 3));
                acc[r] = fmaf(f0, p0.y, acc[r] + p0.x);
                acc[r + 1] = fmaf(f1, p1.y, acc[r + 1] + p1.x);
                t2 = f2_add(t2, dt2);
@@ -336,7 +344,11 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
    return true;
 }
 
-__global__ void __launch_bounds__(kNT, 2) sweep_persistent(SweepArgs A) {
+// Three CTAs per SM: the row items' FFT spills at 80 registers (about 140 B a
+// thread), which costs less than the third CTA gives the tiles, whose loop is
+// latency-bound with 16 warps (64 instances 4.96 -> 4.58 ms; four CTAs and 32
+// angles per chunk 4.91).
+__global__ void __launch_bounds__(kNT, 3) sweep_persistent(SweepArgs A) {
    extern __shared__ float4 sm4[];
    float2* sm = reinterpret_cast<float2*>(sm4);
    __shared__ uint64_t full[2];
