@@ -239,7 +239,7 @@ struct risa_gb_backprojection {
    DevBuf adj;               // adjoint: slice-interleaved image copies (reserve_adjoint)
    DevBuf tile_win;          // staged variants: window start + origin per tile and angle
    BPPatchPlan patch;        // the patch variant's angle order
-   DevBuf patch_angles;
+   DevBuf patch_angles, part;
    std::vector<float> a_host, b_host;  // the staged variants' kernel-parameter copies of a and b
    BPCfg cfg(bool fused_mask) const {
       BPCfg c;
@@ -265,6 +265,7 @@ struct risa_gb_backprojection {
       c.tile_win = tile_win.as<int2>();
       c.patch = &patch;
       c.few = reserved_batch <= 2;
+      c.part = part.as<float>();
       c.patch_angles = patch_angles.as<BPPatchAngle>();
       c.adj_scratch = adj.p;
       c.adj_scratch_bytes = adj.bytes;
@@ -830,8 +831,15 @@ risa_gb_status risa_gb_backprojection_create(const risa_gb_geometry* gi, const r
       if (tiles * (size_t)h->g.Pp * sizeof(int2) <= ((size_t)256 << 20))
          RG_TRY(h->tile_win.upload(bp_tile_windows(t.a.data(), t.b.data(), t.ad.data(), t.bd.data(), t.t0.data(),
                                                    h->g.Pp, h->g.N)));
-      if (bp_patch_plan(t.a.data(), t.b.data(), t.ad.data(), t.bd.data(), t.t0.data(), h->g.Pp, scale, &h->patch))
-         RG_TRY(h->patch_angles.upload(h->patch.angles));
+      const bool unrotated = h->p.quirks == RISA_GB_QUIRKS_NONE && h->g.rotation_offset == 0.0;
+      if (bp_patch_plan(t.a.data(), t.b.data(), t.ad.data(), t.bd.data(), t.t0.data(), h->g.Pp, scale, unrotated,
+                        &h->patch)) {
+         std::vector<BPPatchAngle> all = h->patch.angles;
+         all.insert(all.end(), h->patch.sym_angles.begin(), h->patch.sym_angles.end());
+         RG_TRY(h->patch_angles.upload(all));
+         const size_t part = bp_part_bytes(2, h->g.N);  // single frames (8 MB at 512^2)
+         if (!h->patch.sym_angles.empty() && part <= ((size_t)64 << 20)) RG_TRY(h->part.alloc(part));
+      }
       // frame-by-frame callers need no reserve(): one slice quad (16 MB at 1024 x 1024)
       const size_t quad = bp_quads_bytes(4, h->g.Pp, h->g.Dp);
       if (!h->patch.angles.empty() && quad <= ((size_t)64 << 20)) RG_TRY(h->pairs.alloc(quad));

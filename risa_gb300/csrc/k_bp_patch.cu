@@ -44,6 +44,7 @@
 #include "async_copy.h"
 #include "f32x2.cuh"
 #include "kernels.h"
+#include "patch_window.cuh"
 #include "risa_gb300.h"
 
 namespace risa_gb {
@@ -97,25 +98,6 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, u
            "r"(async::smem_u32(dst)),
        "l"(map), "r"(async::smem_u32(bar)), "r"(x), "r"(y), "r"(z)
        : "memory");
-}
-
-// Window of an angle for a tile whose lowest coordinate is at pixel (cx, cy):
-// its first bin w0 (a multiple of ALIGN) and the lowest coordinate relative to
-// it, t0 + cx a + cy b - w0 >= 0. Error-free FP32 sums and products of the (hi,
-// lo) coefficients keep ~2^-40 of a bin; FP64 has few units per SM (one slice of
-// 1024 x 1024 -> 512^2: 148 us with FP64 windows, 142 with these).
-template <int ALIGN>
-__device__ __forceinline__ void patch_window(const BPPatchAngle& t, int cx, int cy, int* w0, float* rel) {
-   const float x = (float)cx, y = (float)cy;
-   const float p = __fmul_rn(x, t.a_hi), q = __fmul_rn(y, t.b_hi);
-   const float pe = fmaf(x, t.a_lo, fmaf(x, t.a_hi, -p)), qe = fmaf(y, t.b_lo, fmaf(y, t.b_hi, -q));
-   const float s = __fadd_rn(t.t0_hi, p), sv = __fsub_rn(s, t.t0_hi);
-   const float se = __fadd_rn(__fsub_rn(t.t0_hi, __fsub_rn(s, sv)), __fsub_rn(p, sv));
-   const float u = __fadd_rn(s, q), uv = __fsub_rn(u, s);
-   const float ue = __fadd_rn(__fsub_rn(s, __fsub_rn(u, uv)), __fsub_rn(q, uv));
-   const float lo = __fadd_rn(__fadd_rn(se, ue), __fadd_rn(__fadd_rn(pe, qe), t.t0_lo));
-   *w0 = (int)floorf(__fadd_rn(u, lo)) & ~(ALIGN - 1);
-   *rel = fmaxf(__fadd_rn(__fsub_rn(u, (float)*w0), lo), 0.f);
 }
 
 __device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
@@ -415,15 +397,16 @@ __global__ void __launch_bounds__(64 * QL + 32, MINB)
 // infinities and NaN stay where the general kernel leaves them.
 // A stage is refilled by all working warps: with one producer warp as
 // in bp_patch the same loop took 141 us, with 16-byte cp.async pieces instead of a
-// box per angle 134. One slice of 1024 x 1024 -> 512^2: 119 us (quads 263,
-// pairs_s1_a32 229); 512 x 256 -> 256^2: 28 us (66, 80). Bound by issue: about 40
-// instructions per patch and angle.
-constexpr int kRowsACH = 64;
+// box per angle 134. One slice of 1024 x 1024 -> 512^2: 119 us, 91 with symmetric
+// sets (quads 263, pairs_s1_a32 229); 512 x 256 -> 256^2: 28 and 27 us (66, 80).
+// Bound by issue (70%), half of it on the integer and select pipe.
+template <int R>
+constexpr int kRowsACH = 64 / R;  // angles per chunk, R rows each
 
 struct RowsArgs {
    const BPPatchAngle* ang;
    const float* sino;
-   float* img;
+   float* img;   // SYM: the partial images [4][S][N][N]
    int* err;
    int N, Pp, Dp, wlen;
    float norm, mask_value;
@@ -437,12 +420,12 @@ __device__ __forceinline__ float lds_f32(uint32_t addr) {
 }
 
 // off: the offset pixels' coordinates relative to their middle bins at f = 0.
-template <int MA, int MB, int MAB, int S>
-__device__ __forceinline__ void rows_angle(uint32_t addr, uint32_t sstep, float f, float4 off, float (&acc)[S][4]) {
+template <int MA, int MB, int MAB, int R>
+__device__ __forceinline__ void rows_angle(uint32_t addr, uint32_t sstep, float f, float4 off, float (&acc)[R][4]) {
    constexpr int m[4] = {0, MA, MB, MAB};
    const float r[4] = {0.f, f + off.x, f + off.y, f + off.z};
 #pragma unroll
-   for (int s = 0; s < S; ++s) {
+   for (int s = 0; s < R; ++s) {
       float q[MAB + 3];
 #pragma unroll
       for (int e = 0; e < MAB + 3; ++e) q[e] = lds_f32(addr + (uint32_t)s * sstep + (uint32_t)e * 4u);
@@ -457,11 +440,19 @@ __device__ __forceinline__ void rows_angle(uint32_t addr, uint32_t sstep, float 
    }
 }
 
-template <int S, int G>
+// SYM: the rows of four angles at once. With the angles i pi / Pp of an unrotated
+// scan, theta, pi - theta, pi/2 + theta and pi/2 - theta (rows i, Pp - i, Pp/2 + i,
+// Pp/2 - i) see a pixel, its x mirror, its quarter turn and its transpose at the
+// same ray coordinate, so the bin index and the weights of a patch serve four
+// rows, as they serve the slices of a quad in bp_patch. The sums go to four
+// partial images (pixel = where that row's contribution belongs), which
+// bp_patch_combine adds with the angles that are not in a set of four (0, Pp/2 and,
+// where Pp is a multiple of 4, Pp/4 and 3 Pp/4).
+template <int S, int G, bool SYM>
 __global__ void __launch_bounds__(64 * G)
     bp_patch_rows(const __grid_constant__ CUtensorMap map, const __grid_constant__ RowsArgs g,
                   const __grid_constant__ PatchSegs pp) {
-   constexpr int ACH = kRowsACH;
+   constexpr int R = SYM ? 4 * S : S, ACH = kRowsACH<R>;  // rows per angle, angles per chunk
    extern __shared__ __align__(128) unsigned char smem_raw[];
    __shared__ uint64_t full[2], empty[2];
    // per angle: (|a|, |b|, window-relative coordinate - 1/2), then rows_angle's offsets
@@ -481,7 +472,7 @@ __global__ void __launch_bounds__(64 * G)
    // a group's two warps cover 16 x 8 pixels each; halves outside the circle are left out
    const bool live0 = inside(x0, y0, kTile, kTile / 2), live1 = inside(x0, y0 + kTile / 2, kTile, kTile / 2);
    const int halves = (int)live0 + (int)live1, L = G * halves;  // working warps
-   const uint32_t row_bytes = (uint32_t)g.wlen * 4u, angle_bytes = row_bytes * S;
+   const uint32_t row_bytes = (uint32_t)g.wlen * 4u, angle_bytes = row_bytes * R;
    if (threadIdx.x == 0) {
       for (int i = 0; i < 2; ++i) {
          async::mbar_init(&full[i], max(L, 1));
@@ -492,9 +483,9 @@ __global__ void __launch_bounds__(64 * G)
    }
    __syncthreads();
 
-   float acc[S][4];
+   float acc[R][4];
 #pragma unroll
-   for (int s = 0; s < S; ++s)
+   for (int s = 0; s < R; ++s)
 #pragma unroll
       for (int p = 0; p < 4; ++p) acc[s][p] = 0.f;
    const int group = warp >> 1;
@@ -525,14 +516,22 @@ __global__ void __launch_bounds__(64 * G)
          __syncwarp();
          if (lane == 0) async::mbar_arrive_expect_tx(&full[st], (uint32_t)mine * angle_bytes);
          __syncwarp();
-         if (lane < mine)
-            tma_load_3d(smem_raw + (size_t)(st * ACH + rank + lane * L) * angle_bytes, &map, &full[st], w0, row, 0);
+         if (lane < mine) {
+            unsigned char* dst = smem_raw + (size_t)(st * ACH + rank + lane * L) * angle_bytes;
+            tma_load_3d(dst, &map, &full[st], w0, row, 0);
+            if (SYM) {
+               const uint32_t step = row_bytes * S;
+               tma_load_3d(dst + step, &map, &full[st], w0, g.Pp - row, 0);
+               tma_load_3d(dst + 2 * step, &map, &full[st], w0, g.Pp / 2 + row, 0);
+               tma_load_3d(dst + 3 * step, &map, &full[st], w0, g.Pp / 2 - row, 0);
+            }
+         }
       };
       const uint32_t sbase = async::smem_u32(smem_raw) - ((uint32_t)kMagicBits << 2);
       uint32_t signs = 0;
       auto flip1 = [&](uint32_t f) {
 #pragma unroll
-         for (int s = 0; s < S; ++s) {
+         for (int s = 0; s < R; ++s) {
             float* v = acc[s];
             float t;
             if (f & 1u) t = v[0], v[0] = v[1], v[1] = t, t = v[2], v[2] = v[3], v[3] = t;
@@ -574,7 +573,7 @@ __global__ void __launch_bounds__(64 * G)
                   const float v = tm + kMagic;
                   const float f = tm - (v - kMagic);
                   const uint32_t addr = stage + (uint32_t)ai * angle_bytes + ((uint32_t)__float_as_int(v) << 2);
-                  rows_angle<(CL >> 3), (CL >> 2) & 1, CL & 3, S>(addr, row_bytes, f, off, acc);
+                  rows_angle<(CL >> 3), (CL >> 2) & 1, CL & 3, R>(addr, row_bytes, f, off, acc);
                };
                const int na = min(ACH, n - a0);
                int ai = group;
@@ -611,26 +610,81 @@ __global__ void __launch_bounds__(64 * G)
             for (uint32_t ph = 0; ph < 2; ++ph) async::mbar_wait_quiet(&full[i], ph);
       return;
    }
-   float* sums = reinterpret_cast<float*>(smem_raw);  // [group][slice][pixel of the tile]
+   float* sums = reinterpret_cast<float*>(smem_raw);  // [group][row][pixel of the tile]
 #pragma unroll
-   for (int s = 0; s < S; ++s)
+   for (int s = 0; s < R; ++s)
 #pragma unroll
       for (int p = 0; p < 4; ++p)
-         sums[(group * S + s) * kTile * kTile + (yp + (p >> 1)) * kTile + xp + (p & 1)] = acc[s][p];
+         sums[(group * R + s) * kTile * kTile + (yp + (p >> 1)) * kTile + xp + (p & 1)] = acc[s][p];
    __syncthreads();
-   for (int i = threadIdx.x; i < S * kTile * kTile; i += 64 * G) {
-      float v = sums[i];
-#pragma unroll
-      for (int k = 1; k < G; ++k) v += sums[k * S * kTile * kTile + i];
-      const int s = i / (kTile * kTile), x = x0 + i % kTile, y = y0 + (i / kTile) % kTile;
+   for (int i = threadIdx.x; i < R * kTile * kTile; i += 64 * G) {
+      const int r = i / (kTile * kTile), e = i % (kTile * kTile);
+      // rows 2 and 3 of SYM are transposed: consecutive threads take consecutive y
+      const bool turned = SYM && r >= 2 * S;
+      const int tx = turned ? e / kTile : e % kTile, ty = turned ? e % kTile : e / kTile;
+      const int x = x0 + tx, y = y0 + ty;
       if (x >= N || y >= N) continue;
+      float v = 0.f;
+#pragma unroll
+      for (int k = 0; k < G; ++k) v += sums[(k * R + r) * kTile * kTile + ty * kTile + tx];
+      if (SYM) {
+         const int j = r / S;
+         const int X = j == 0 ? x : j == 1 ? N - 1 - x : j == 2 ? N - 1 - y : y, Y = j < 2 ? y : x;
+         g.img[((size_t)r * N + Y) * N + X] = v;
+         continue;
+      }
       v *= g.norm;
       if (g.masking) {
          const float dx = (float)x - c, dy = (float)y - c;
          if (dx * dx + dy * dy > lim) v = g.mask_value;
       }
-      g.img[((size_t)s * N + y) * N + x] = v;
+      g.img[((size_t)r * N + y) * N + x] = v;
    }
+}
+
+// Sum of the four partial images and of the angles outside the symmetric sets
+// (given by their coefficients), scaled and masked.
+struct CombineArgs {
+   const float* part;
+   const float* sino;
+   float* img;
+   BPPatchAngle extra[4];
+   int n_extra, N, Pp, Dp;
+   float norm, mask_value;
+   int masking;
+};
+template <int S>
+__global__ void __launch_bounds__(256) bp_patch_combine(const __grid_constant__ CombineArgs g) {
+   const int x = blockIdx.x * 32 + (threadIdx.x & 31), y = blockIdx.y * 8 + (threadIdx.x >> 5);
+   const int N = g.N;
+   if (x >= N || y >= N) return;
+   const size_t at = (size_t)y * N + x, plane = (size_t)N * N;
+   const float c = 0.5f * (float)(N - 1), dx = (float)x - c, dy = (float)y - c;
+   const bool out = g.masking && dx * dx + dy * dy > (float)N * (float)N * 0.25f;
+   float v[S];
+#pragma unroll
+   for (int s = 0; s < S; ++s) v[s] = 0.f;
+   if (!out) {
+#pragma unroll
+      for (int s = 0; s < S; ++s) {
+         const float* p = g.part + s * plane + at;
+         v[s] = (p[0] + p[S * plane]) + (p[2 * S * plane] + p[3 * S * plane]);
+      }
+      for (int i = 0; i < g.n_extra; ++i) {
+         int k;
+         float f;
+         patch_window<1>(g.extra[i], x, y, &k, &f);
+         const bool in0 = (unsigned)k < (unsigned)g.Dp, in1 = (unsigned)(k + 1) < (unsigned)g.Dp;
+#pragma unroll
+         for (int s = 0; s < S; ++s) {
+            const float* row = g.sino + ((size_t)s * g.Pp + g.extra[i].index) * g.Dp + k;
+            const float q0 = in0 ? __ldg(row) : 0.f, q1 = in1 ? __ldg(row + 1) : 0.f;
+            v[s] = fmaf(f - 0.5f, q1 - q0, v[s] + 0.5f * (q0 + q1));
+         }
+      }
+   }
+#pragma unroll
+   for (int s = 0; s < S; ++s) g.img[s * plane + at] = out ? g.mask_value : v[s] * g.norm;
 }
 
 // Staged rows from a plain sinogram: quads[q][angle][bin] = slices 4q .. 4q + 3
@@ -712,14 +766,15 @@ cudaError_t launch_patch(const PatchArgs& args, const PatchPlanParam& pp, float 
    return cudaGetLastError();
 }
 
-template <int S, int G>
+template <int S, int G, bool SYM>
 cudaError_t launch_rows(const RowsArgs& args, const PatchSegs& pp, const BPCfg& cfg,
                         cudaStream_t st) {
    RowsArgs a = args;
    const int need = (int)std::floor((kTile - 2) * 1.41421357 * (double)cfg.scale + 4.01) + 3 +
                     std::min(2, (int)std::floor(1.41421357 * (double)cfg.scale));
    a.wlen = need <= 32 ? 32 : 64;
-   const size_t smem = std::max((size_t)2 * kRowsACH * S * a.wlen * 4, (size_t)G * S * kTile * kTile * 4);
+   constexpr int R = SYM ? 4 * S : S;
+   const size_t smem = std::max((size_t)2 * kRowsACH<R> * R * a.wlen * 4, (size_t)G * R * kTile * kTile * 4);
    if (need > 64 || smem > 220 * 1024) return cudaErrorInvalidConfiguration;
    EncodeTiled enc = encode_fn();
    if (!enc) return cudaErrorNotSupported;
@@ -732,7 +787,7 @@ cudaError_t launch_rows(const RowsArgs& args, const PatchSegs& pp, const BPCfg& 
            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return cudaErrorInvalidValue;
-   auto kern = bp_patch_rows<S, G>;
+   auto kern = bp_patch_rows<S, G, SYM>;
    if (smem > 47 * 1024) {  // with the kernel's static shared memory
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
@@ -743,46 +798,79 @@ cudaError_t launch_rows(const RowsArgs& args, const PatchSegs& pp, const BPCfg& 
 }
 }  // namespace
 
-bool bp_patch_plan(const float* a, const float* b, const double* ad, const double* bd, const double* t0, int Pp,
-                   float scale, BPPatchPlan* plan) {
-   plan->angles.clear();
-   if (Pp < 1 || Pp > kPatchAngles || !(scale > 0.f) || scale > 2.f) return false;
-   struct Key {
-      int group, index;
-   };
-   auto split = [](double v, float* hi, float* lo) {
-      *hi = (float)v;
-      *lo = (float)(v - (double)*hi);
-   };
-   std::vector<Key> keys(Pp);
-   for (int i = 0; i < Pp; ++i) {
-      const float A = std::fabs(a[i]), B = std::fabs(b[i]);
-      if (!(A <= 2.f && B <= 2.f && A + B < 3.f) || !std::isfinite(t0[i])) return false;
-      const int ma = A >= 1.f, mb = B >= 1.f;
-      // the offset lies in [m, m + 1]; at an integer either end serves
-      const int mab = std::min({(int)(A + B), 2, ma + mb + 1});
-      if (A + B - (float)mab > 1.f) return false;
-      const int cls = ma << 3 | mb << 2 | mab;
-      keys[i] = {((a[i] < 0.f ? 1 : 0) + (b[i] < 0.f ? 2 : 0)) * 16 + cls, i};
-   }
-   std::stable_sort(keys.begin(), keys.end(), [](const Key& x, const Key& y) { return x.group < y.group; });
-   for (int i = 0; i < Pp;) {
-      int n = 1;
-      while (i + n < Pp && keys[i + n].group == keys[i].group) ++n;
-      plan->segs.push_back((uint32_t)i | (uint32_t)n << 12 | (uint32_t)(keys[i].group & 15) << 24 |
-                           (uint32_t)(keys[i].group >> 4) << 28);
+namespace {
+void split(double v, float* hi, float* lo) {
+   *hi = (float)v;
+   *lo = (float)(v - (double)*hi);
+}
+// Class and signs of an angle: MA << 3 | MB << 2 | MAB, then (a < 0) | (b < 0) << 1
+// in bits 4 and 5; -1 outside the kernel's range.
+int patch_group(float a, float b) {
+   const float A = std::fabs(a), B = std::fabs(b);
+   if (!(A <= 2.f && B <= 2.f && A + B < 3.f)) return -1;
+   const int ma = A >= 1.f, mb = B >= 1.f;
+   // the offset lies in [m, m + 1]; at an integer either end serves
+   const int mab = std::min({(int)(A + B), 2, ma + mb + 1});
+   if (A + B - (float)mab > 1.f) return -1;
+   return ((a < 0.f ? 1 : 0) | (b < 0.f ? 2 : 0)) << 4 | ma << 3 | mb << 2 | mab;
+}
+BPPatchAngle patch_angle_of(const double* ad, const double* bd, const double* t0, int i) {
+   BPPatchAngle t;
+   split(t0[i], &t.t0_hi, &t.t0_lo);
+   split(ad[i], &t.a_hi, &t.a_lo);
+   split(bd[i], &t.b_hi, &t.b_lo);
+   t.index = i;
+   t.pad = 0;
+   return t;
+}
+// Runs of equal groups: first | n << 12 | class << 24 | signs << 28.
+std::vector<uint32_t> patch_runs(const std::vector<int>& groups) {
+   std::vector<uint32_t> segs;
+   for (size_t i = 0; i < groups.size();) {
+      size_t n = 1;
+      while (i + n < groups.size() && groups[i + n] == groups[i]) ++n;
+      segs.push_back((uint32_t)i | (uint32_t)n << 12 | (uint32_t)(groups[i] & 15) << 24 |
+                     (uint32_t)(groups[i] >> 4) << 28);
       i += n;
    }
-   for (const Key& k : keys) {
-      BPPatchAngle t;
-      split(t0[k.index], &t.t0_hi, &t.t0_lo);
-      split(ad[k.index], &t.a_hi, &t.a_lo);
-      split(bd[k.index], &t.b_hi, &t.b_lo);
-      t.index = k.index;
-      t.pad = 0;
-      plan->angles.push_back(t);
-      plan->A.push_back(std::fabs(a[k.index]));
-      plan->B.push_back(std::fabs(b[k.index]));
+   return segs;
+}
+}  // namespace
+
+bool bp_patch_plan(const float* a, const float* b, const double* ad, const double* bd, const double* t0, int Pp,
+                   float scale, bool unrotated, BPPatchPlan* plan) {
+   *plan = BPPatchPlan();
+   if (Pp < 1 || Pp > kPatchAngles || !(scale > 0.f) || scale > 2.f) return false;
+   std::vector<std::pair<int, int>> keys(Pp);  // (group, angle)
+   for (int i = 0; i < Pp; ++i) {
+      keys[i] = {patch_group(a[i], b[i]), i};
+      if (keys[i].first < 0 || !std::isfinite(t0[i])) return false;
+   }
+   std::sort(keys.begin(), keys.end());
+   std::vector<int> groups;
+   for (const auto& k : keys) {
+      groups.push_back(k.first);
+      plan->angles.push_back(patch_angle_of(ad, bd, t0, k.second));
+      plan->A.push_back(std::fabs(a[k.second]));
+      plan->B.push_back(std::fabs(b[k.second]));
+   }
+   plan->segs = patch_runs(groups);
+   if (plan->segs.size() > kPatchMaxSegs) return false;
+   // symmetric sets: angles i pi / Pp with 0 < i < Pp / 4 stand for four rows each
+   if (unrotated && Pp % 2 == 0 && Pp >= 8) {
+      groups.clear();
+      for (int i = 1; 4 * i < Pp; ++i) {
+         groups.push_back(patch_group(a[i], b[i]));
+         plan->sym_angles.push_back(patch_angle_of(ad, bd, t0, i));
+      }
+      plan->sym_segs = patch_runs(groups);
+      plan->sym_extra.push_back(patch_angle_of(ad, bd, t0, 0));
+      plan->sym_extra.push_back(patch_angle_of(ad, bd, t0, Pp / 2));
+      if (Pp % 4 == 0) {  // and its mirror image
+         plan->sym_extra.push_back(patch_angle_of(ad, bd, t0, Pp / 4));
+         plan->sym_extra.push_back(patch_angle_of(ad, bd, t0, 3 * Pp / 4));
+      }
+      if (plan->sym_segs.size() > kPatchMaxSegs) plan->sym_angles.clear();
    }
    return true;
 }
@@ -807,14 +895,41 @@ cudaError_t launch_bp_patch(const float* sino, float* img, int batch, const BPCf
    cudaError_t e = cudaSuccess;
    if (!cfg.prefilled && bp_patch_rows_ok(cfg, sino, batch)) {
       if (cfg.mid_event && (e = cudaEventRecord(cfg.mid_event, st)) != cudaSuccess) return e;
-      const RowsArgs r{cfg.patch_angles, sino, img, cfg.err, cfg.N, cfg.Pp, cfg.Dp, 0, cfg.norm, cfg.mask_value, cfg.masking};
+      RowsArgs r{cfg.patch_angles, sino, img, cfg.err, cfg.N, cfg.Pp, cfg.Dp, 0, cfg.norm, cfg.mask_value, cfg.masking};
       // Groups of angles per CTA: two keep a chunk's refill small beside its work;
       // four where the tiles alone are too few warps (one slice, groups of 2 / 4 /
-      // 8: 512^2 119 / 130 / 145 us, 256^2 36 / 28 / 30).
-      const long tiles = (long)((cfg.N + kTile - 1) / kTile) * ((cfg.N + kTile - 1) / kTile);
-      if (tiles >= 600)
-         return batch == 1 ? launch_rows<1, 2>(r, pp, cfg, st) : launch_rows<2, 2>(r, pp, cfg, st);
-      return batch == 1 ? launch_rows<1, 4>(r, pp, cfg, st) : launch_rows<2, 4>(r, pp, cfg, st);
+      // 8: 512^2 119 / 130 / 145 us, 256^2 36 / 28 / 30; with symmetric sets 91 /
+      // 99 / 131 and 30 / 27 / 30).
+      const bool many = (long)((cfg.N + kTile - 1) / kTile) * ((cfg.N + kTile - 1) / kTile) >= 600;
+      if (cfg.part && !cfg.patch->sym_angles.empty()) {
+         r.ang = cfg.patch_angles + cfg.patch->angles.size();  // uploaded after the plan's own
+         r.img = cfg.part;
+         PatchSegs ps;
+         std::memcpy(ps.seg, cfg.patch->sym_segs.data(), sizeof(uint32_t) * cfg.patch->sym_segs.size());
+         ps.n_segs = (int)cfg.patch->sym_segs.size();
+         e = many ? (batch == 1 ? launch_rows<1, 2, true>(r, ps, cfg, st) : launch_rows<2, 2, true>(r, ps, cfg, st))
+                  : (batch == 1 ? launch_rows<1, 4, true>(r, ps, cfg, st) : launch_rows<2, 4, true>(r, ps, cfg, st));
+         if (e != cudaSuccess) return e;
+         CombineArgs ca;
+         ca.part = cfg.part;
+         ca.sino = sino;
+         ca.img = img;
+         ca.n_extra = (int)cfg.patch->sym_extra.size();
+         for (int i = 0; i < ca.n_extra; ++i) ca.extra[i] = cfg.patch->sym_extra[i];
+         ca.N = cfg.N;
+         ca.Pp = cfg.Pp;
+         ca.Dp = cfg.Dp;
+         ca.norm = cfg.norm;
+         ca.mask_value = cfg.mask_value;
+         ca.masking = cfg.masking;
+         const dim3 grid((cfg.N + 31) / 32, (cfg.N + 7) / 8);
+         if (batch == 1) bp_patch_combine<1><<<grid, 256, 0, st>>>(ca);
+         else bp_patch_combine<2><<<grid, 256, 0, st>>>(ca);
+         return cudaGetLastError();
+      }
+      if (many)
+         return batch == 1 ? launch_rows<1, 2, false>(r, pp, cfg, st) : launch_rows<2, 2, false>(r, pp, cfg, st);
+      return batch == 1 ? launch_rows<1, 4, false>(r, pp, cfg, st) : launch_rows<2, 4, false>(r, pp, cfg, st);
    }
    if (!cfg.pairs || bp_quads_bytes(batch, cfg.Pp, cfg.Dp) > cfg.pairs_bytes) return cudaErrorInvalidValue;
    std::memcpy(pp.A, cfg.patch->A.data(), sizeof(float) * cfg.Pp);

@@ -256,10 +256,16 @@ struct BPPatchAngle {
 struct BPPatchPlan {
    std::vector<BPPatchAngle> angles;  // in plan order; empty: the geometry is outside the kernel's range
    std::vector<float> A, B;           // |a|, |b|
+   // unrotated scans of an even number of angles: the angles that stand for four
+   // rows each, their runs, and the angles left over
+   std::vector<BPPatchAngle> sym_angles, sym_extra;
+   std::vector<uint32_t> sym_segs;
    std::vector<uint32_t> segs;        // runs of one class: first | n << 12 | class << 24 | signs << 28
 };
 bool bp_patch_plan(const float* a, const float* b, const double* ad, const double* bd, const double* t0, int Pp,
-                   float scale, BPPatchPlan* plan);
+                   float scale, bool unrotated, BPPatchPlan* plan);
+// Bytes of the partial images of the symmetric form, `batch` (1 or 2) slices.
+inline size_t bp_part_bytes(int batch, int N) { return sizeof(float) * 4 * (size_t)batch * N * N; }
 // Device bytes of the staged rows [quad of slices][angle][bin][4] of `batch` slices
 // and the quads' non-finite flags.
 size_t bp_quads_bytes(int batch, int Pp, int Dp);
@@ -291,7 +297,8 @@ struct BPCfg {
                                     // coordinate of the tile origin in it), bp_tile_windows; else FP64 on device
    const BPPatchPlan* patch = nullptr;  // host side
    bool few = false;  // a caller of one or two slices at a time: the patch kernel over the sinogram itself
-   const BPPatchAngle* patch_angles = nullptr;
+   const BPPatchAngle* patch_angles = nullptr;  // the plan's angles, then its sym_angles
+   float* part = nullptr;  // partial images of the symmetric form (bp_part_bytes)
    void* adj_scratch = nullptr;  // adjoint: slice-interleaved image copies (bp_adjoint_scratch_bytes)
    size_t adj_scratch_bytes = 0;
    // adjoint: FP64 line starts split as (hi, lo) floats, [Pp][N]:
