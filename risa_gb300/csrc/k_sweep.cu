@@ -15,6 +15,7 @@
 #include "f32x2.cuh"
 #include "fft_r16.cuh"
 #include "kernels.h"
+#include "patch_window.cuh"
 #include "sweep.h"
 
 namespace risa_gb {
@@ -126,12 +127,38 @@ struct TileShared {
    int ok, fail;
 };
 
+// Waits until *count reaches `want` (every thread of the CTA calls it; bounded).
+__device__ __forceinline__ bool sweep_wait(const SweepArgs& A, const int* count, int want, TileShared& S) {
+   if (threadIdx.x == 0) {
+      int ok = 0;
+      for (uint32_t i = 0; i < kDepPolls; ++i) {
+         if (load_acquire(count) >= want) {
+            ok = 1;
+            break;
+         }
+         __nanosleep(256);
+      }
+      if (!ok) atomicCAS(A.err, 0, 7);
+      S.ok = ok;
+      S.fail = 0;
+   }
+   __syncthreads();
+   return S.ok;
+}
+
 // One 32 x 32 tile of instance `inst`. Returns false (uniformly) when a
-// bounded wait gave up; the CTA then stops taking items.
+// bounded wait gave up; the CTA then stops taking items. SYM: the angles are the
+// instance's symmetric sets, four rows (angles i, Pp - i, Pp/2 + i, Pp/2 - i) at
+// the same window and ray coordinate, added to four partial images: the
+// coordinate arithmetic (about 8 of 10 instructions per update) is shared by four
+// updates, and shared memory bounds the tile instead (8 B per update): 64
+// instances 4.58 -> 4.16 ms (75% of the shared-memory data path).
+template <bool SYM>
 __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& I, int inst, int tile, float2* wsm,
                            uint64_t* full, uint32_t (&uses)[2], TileShared& S) {
-   constexpr int T = 32, PPT = 4, RS = 8;
-   const int N = I.N, Pp = I.Pp, W = I.wlen2;
+   constexpr int T = 32, PPT = 4, RS = 8, R = SYM ? 4 : 1;
+   const int N = I.N, W = I.wlen2, first = SYM ? 1 : 0;
+   const int n_ang = SYM ? I.n_base : I.Pp;  // angles walked, from `first`
    const int x0 = (tile % I.tiles_x) * T, y0 = (tile / I.tiles_x) * T;
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
    const int xo = (warp & 3) * 8 + (lane & 3) + ((lane >> 1) & 4);
@@ -148,34 +175,20 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
    }
    if (skip) {
 #pragma unroll
-      for (int r = 0; r < PPT; ++r) {
+      for (int r = 0; r < (SYM ? 0 : PPT); ++r) {  // SYM: the combine items write the mask
          const int x = x0 + xo, y = y0 + yo + RS * r;
          if (x < N && y < N) out[(size_t)y * N + x] = I.mask_value;
       }
    } else {
       // every row item of the instance must have been written
-      if (threadIdx.x == 0) {
-         int ok = 0;
-         for (uint32_t i = 0; i < kDepPolls; ++i) {
-            if (load_acquire(A.rows_done + inst) >= I.row_items) {
-               ok = 1;
-               break;
-            }
-            __nanosleep(256);
-         }
-         if (!ok) atomicCAS(A.err, 0, 7);
-         S.ok = ok;
-         S.fail = 0;
-      }
-      __syncthreads();
-      if (!S.ok) return false;
+      if (!sweep_wait(A, A.rows_done + inst, I.row_items, S)) return false;
       // the rows were written by generic-proxy stores of other CTAs; the bulk
       // copies below (issued by every warp) read them through the async proxy
       asm volatile("fence.proxy.async.global;" ::: "memory");
       const float2* prow = A.pairs + I.pair_off;
       const uint32_t win_bytes = (uint32_t)W * (uint32_t)sizeof(float2);
-      const int ACH = A.ach;
-      const int nchunks = (Pp + ACH - 1) / ACH;
+      const int ACH = A.ach / R;  // angles per chunk
+      const int nchunks = (n_ang + ACH - 1) / ACH;
       // Every warp refills its share of a chunk: warp w's lanes 0 .. ACH/8 - 1
       // take angles w ACH/8 + lane, and each warp arrives once on the stage's
       // mbarrier (initialised for all the CTA's warps) with its own byte
@@ -186,23 +199,23 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
       const bool pre = I.tile_win != nullptr;
       const int apw = ACH / kSweepWarps, l = warp * apw + lane;  // this lane's angle slot
       auto prefetch = [&](int ch) {
-         const int na = min(ACH, Pp - ch * ACH), s = ch & 1;
+         const int na = min(ACH, n_ang - ch * ACH), s = ch & 1;
          if (lane < apw && l < na) {
             const int ang = ch * ACH + l;
-            async::cp_async<4>(&S.pre_a[s][l], I.a + ang);
-            async::cp_async<4>(&S.pre_b[s][l], I.b + ang);
-            async::cp_async<8>(&S.pre_win[s][l], I.tile_win + (size_t)tile * Pp + ang);
+            async::cp_async<4>(&S.pre_a[s][l], I.a + first + ang);
+            async::cp_async<4>(&S.pre_b[s][l], I.b + first + ang);
+            async::cp_async<8>(&S.pre_win[s][l], I.tile_win + (size_t)tile * n_ang + ang);
          }
          async::cp_async_commit();
       };
       auto issue = [&](int ch, int st, bool from_pre) {
-         const int na = min(ACH, Pp - ch * ACH);
+         const int na = min(ACH, n_ang - ch * ACH);
          const int mine = min(max(na - warp * apw, 0), apw);  // angles of this warp in the chunk
          if (from_pre) async::cp_async_wait_all();
-         if (lane == 0) async::mbar_arrive_expect_tx(&full[st], (uint32_t)mine * win_bytes);
+         if (lane == 0) async::mbar_arrive_expect_tx(&full[st], (uint32_t)(mine * R) * win_bytes);
          __syncwarp();
          if (lane < mine) {  // a lane per angle of the warp's share
-            const int ang = ch * ACH + l;
+            const int ang = first + ch * ACH + l;
             float a, b, rel;
             int w0;
             if (from_pre) {  // this lane's own prefetched entries
@@ -215,7 +228,7 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
             } else if (I.tile_win) {  // the host's table of the same FP64 arithmetic
                a = __ldg(I.a + ang);
                b = __ldg(I.b + ang);
-               const int2 e = __ldg(I.tile_win + (size_t)tile * Pp + ang);
+               const int2 e = __ldg(I.tile_win + (size_t)tile * n_ang + ang - first);
                w0 = e.x;
                rel = __int_as_float(e.y);
             } else {
@@ -244,8 +257,14 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
                a = b = rel = 0.f;
             }
             S.par[st][l] = make_float4(a, b, rel, 2.f * (float)RS * b);
-            async::bulk_load(wsm + (size_t)(st * ACH + l) * W, prow + (size_t)ang * I.win_len + u0,
-                             win_bytes, &full[st]);
+            float2* dst = wsm + (size_t)((st * ACH + l) * R) * W;
+            async::bulk_load(dst, prow + (size_t)ang * I.win_len + u0, win_bytes, &full[st]);
+            if (SYM) {
+               const int P = I.Pp;
+               async::bulk_load(dst + W, prow + (size_t)(P - ang) * I.win_len + u0, win_bytes, &full[st]);
+               async::bulk_load(dst + 2 * W, prow + (size_t)(P / 2 + ang) * I.win_len + u0, win_bytes, &full[st]);
+               async::bulk_load(dst + 3 * W, prow + (size_t)(P / 2 - ang) * I.win_len + u0, win_bytes, &full[st]);
+            }
          }
       };
       issue(0, 0, false);
@@ -253,9 +272,11 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
       if (pre && nchunks > 2) prefetch(2);
       __syncthreads();
 
-      float acc[PPT];
+      float acc[R][PPT];
 #pragma unroll
-      for (int r = 0; r < PPT; ++r) acc[r] = 0.f;
+      for (int j = 0; j < R; ++j)
+#pragma unroll
+         for (int r = 0; r < PPT; ++r) acc[j][r] = 0.f;
       const uint32_t wbase = async::smem_u32(wsm);
       const unsigned long long magic2 = f2_pack(kSweepMagic, kSweepMagic);
       bool failed = false;
@@ -279,16 +300,16 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
          const int st = ch & 1;
          if (!async::mbar_wait(&full[st], uses[st] & 1u, A.err, 5)) S.fail = 1;
          ++uses[st];
-         const int na = live ? min(ACH, Pp - ch * ACH) : 0;
+         const int na = live ? min(ACH, n_ang - ch * ACH) : 0;
          // the rounded coordinate's bits less the magic constant's are the entry
-         const uint32_t cbase = wbase + (uint32_t)(st * ACH * W) * (uint32_t)sizeof(float2) -
+         const uint32_t cbase = wbase + (uint32_t)(st * ACH * R * W) * (uint32_t)sizeof(float2) -
                                 ((uint32_t)kSweepMagicBits << 3);
-#pragma unroll 8
+#pragma unroll(SYM ? 2 : 8)
          for (int ai = 0; ai < na; ++ai) {
             const float4 q = S.par[st][ai];  // one broadcast load per angle
             const float a = q.x, b = q.y;
             const float tm = q.z + (float)xo * a + (float)yo * b;
-            const uint32_t abase = cbase + (uint32_t)(ai * W) * (uint32_t)sizeof(float2);
+            const uint32_t abase = cbase + (uint32_t)(ai * R * W) * (uint32_t)sizeof(float2);
             // pixel steps (r, r + 1) as one f32x2 pair: the ray coordinate,
             // its rounding and the fraction take one instruction per pair
             unsigned long long t2 = f2_pack(tm, fmaf((float)RS, b, tm));
@@ -300,10 +321,14 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
                float v0, v1, f0, f1;
                f2_unpack(v2, v0, v1);
                f2_unpack(fr2, f0, f1);
-               const float2 p0 = lds64(abase + ((uint32_t)__float_as_int(v0) << 3));
-               const float2 p1 = lds64(abase + ((uint32_t)__float_as_int(v1) << 3));
-               acc[r] = fmaf(f0, p0.y, acc[r] + p0.x);
-               acc[r + 1] = fmaf(f1, p1.y, acc[r + 1] + p1.x);
+               const uint32_t at0 = abase + ((uint32_t)__float_as_int(v0) << 3);
+               const uint32_t at1 = abase + ((uint32_t)__float_as_int(v1) << 3);
+#pragma unroll
+               for (int j = 0; j < R; ++j) {
+                  const float2 p0 = lds64(at0 + (uint32_t)j * win_bytes), p1 = lds64(at1 + (uint32_t)j * win_bytes);
+                  acc[j][r] = fmaf(f0, p0.y, acc[j][r] + p0.x);
+                  acc[j][r + 1] = fmaf(f1, p1.y, acc[j][r + 1] + p1.x);
+               }
                t2 = f2_add(t2, dt2);
             }
          }
@@ -325,8 +350,15 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
 #pragma unroll
       for (int r = 0; r < PPT; ++r) {
          const int x = x0 + xo, y = y0 + yo + RS * r;
-         if (x < N && y < N) {
-            float val = acc[r] * I.norm;
+         if (SYM && x < N && y < N) {
+            float* part = A.part + 4 * I.img_off;
+            const size_t plane = (size_t)N * N;
+            part[(size_t)y * N + x] = acc[0][r];
+            part[plane + (size_t)y * N + (N - 1 - x)] = acc[R > 1 ? 1 : 0][r];
+            part[2 * plane + (size_t)x * N + (N - 1 - y)] = acc[R > 1 ? 2 : 0][r];
+            part[3 * plane + (size_t)x * N + y] = acc[R > 1 ? 3 : 0][r];
+         } else if (x < N && y < N) {
+            float val = acc[0][r] * I.norm;
             if (I.masking) {
                const float dx = (float)x - c, dy = (float)y - c;
                if (dx * dx + dy * dy > lim) val = I.mask_value;
@@ -339,16 +371,67 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
    __syncthreads();
    if (threadIdx.x == 0) {
       const int done = atomicAdd(A.tiles_done + inst, 1) + 1;
-      if (done == I.tiles) A.t_done[inst] = global_ns();
+      if (!SYM && done == I.tiles) A.t_done[inst] = global_ns();
    }
    return true;
 }
 
-// Three CTAs per SM: the row items' FFT spills at 80 registers (about 140 B a
-// thread), which costs less than the third CTA gives the tiles, whose loop is
-// latency-bound with 16 warps (64 instances 4.96 -> 4.58 ms; four CTAs and 32
-// angles per chunk 4.91).
-__global__ void __launch_bounds__(kNT, 3) sweep_persistent(SweepArgs A) {
+// One run of pixels of a symmetric instance: the four partial images and the
+// angles outside the sets, scaled and masked. Returns false (uniformly) when the
+// bounded wait for the tiles gave up.
+__device__ __forceinline__ bool sweep_sum(const SweepArgs& A, const SweepInst& I, int inst, int index, TileShared& S) {
+   __shared__ BPPatchAngle extra[4];
+   if (threadIdx.x < I.n_extra) {
+      const int i = I.extra[threadIdx.x];
+      BPPatchAngle& t = extra[threadIdx.x];
+      auto split = [](double v, float* hi, float* lo) {
+         *hi = (float)v;
+         *lo = (float)(v - (double)*hi);
+      };
+      split(I.t0[i], &t.t0_hi, &t.t0_lo);
+      split(I.ad[i], &t.a_hi, &t.a_lo);
+      split(I.bd[i], &t.b_hi, &t.b_lo);
+      t.index = i;
+   }
+   if (!sweep_wait(A, A.tiles_done + inst, I.tiles, S)) return false;
+   const int N = I.N;
+   const size_t plane = (size_t)N * N;
+   const float c = 0.5f * (float)(N - 1), lim = (float)N * (float)N * 0.25f;
+   const float* part = A.part + 4 * I.img_off;
+   const float2* prow = A.pairs + I.pair_off;
+   const size_t end = min(plane, (size_t)(index + 1) * I.combine_px);
+   for (size_t at = (size_t)index * I.combine_px + threadIdx.x; at < end; at += kNT) {
+      const int y = (int)(at / N), x = (int)(at - (size_t)y * N);
+      float v = I.mask_value;
+      const float dx = (float)x - c, dy = (float)y - c;
+      if (!(I.masking && dx * dx + dy * dy > lim)) {
+         v = (__ldcg(part + at) + __ldcg(part + plane + at)) + (__ldcg(part + 2 * plane + at) + __ldcg(part + 3 * plane + at));
+         for (int i = 0; i < I.n_extra; ++i) {
+            int k;
+            float f;
+            patch_window<1>(extra[i], x, y, &k, &f);
+            const int u = min(max(k + I.win_lo, 0), I.win_len - 1);
+            const float2 p = __ldcg(prow + (size_t)extra[i].index * I.win_len + u);
+            v = fmaf(f - 0.5f, p.y, v + p.x);
+         }
+         v *= I.norm;
+      }
+      A.img[I.img_off + at] = v;
+   }
+   __threadfence();
+   __syncthreads();
+   if (threadIdx.x == 0 && atomicAdd(A.sums_done + inst, 1) + 1 == I.combine_items) A.t_done[inst] = global_ns();
+   return true;
+}
+
+// MINB CTAs per SM. With three, the row items' FFT spills at 80 registers (about
+// 140 B a thread), which costs less than the third CTA gives the tiles of a large
+// sweep, whose loop is latency-bound with 16 warps (64 instances, sides 128 ..
+// 1024: 4.96 -> 4.58 ms); four CTAs and 32 angles per chunk took 4.91. A sweep of
+// a few hundred tiles waits for its rows instead (4 instances of up to 256^2: 61 us
+// with two CTAs, 83 with three; 12 of up to 300^2 125 and 119), so it takes two.
+template <int MINB>
+__global__ void __launch_bounds__(kNT, MINB) sweep_persistent(SweepArgs A) {
    extern __shared__ float4 sm4[];
    float2* sm = reinterpret_cast<float2*>(sm4);
    __shared__ uint64_t full[2];
@@ -381,7 +464,10 @@ __global__ void __launch_bounds__(kNT, 3) sweep_persistent(SweepArgs A) {
          __threadfence();
          __syncthreads();
          if (threadIdx.x == 0) atomicAdd(A.rows_done + it.inst, 1);
-      } else if (!sweep_tile(A, I, it.inst, it.index, sm, full, uses, ts)) {
+      } else if (it.kind == kSweepSum) {
+         if (!sweep_sum(A, I, it.inst, it.index, ts)) break;
+      } else if (I.n_base > 0 ? !sweep_tile<true>(A, I, it.inst, it.index, sm, full, uses, ts)
+                              : !sweep_tile<false>(A, I, it.inst, it.index, sm, full, uses, ts)) {
          break;
       }
    }
@@ -425,13 +511,13 @@ void sweep_window_extent(const float* a, const float* b, const double* ad, const
 }
 
 void sweep_tile_windows(const float* a, const float* b, const double* ad, const double* bd, const double* t0,
-                        int Pp, int N, std::vector<int2>& out) {
+                        int first, int n, int N, std::vector<int2>& out) {
    // mirrors sweep_tile (host code is compiled without floating-point contraction)
    const int tiles_x = (N + 31) / 32;
-   out.reserve(out.size() + (size_t)tiles_x * tiles_x * Pp);
+   out.reserve(out.size() + (size_t)tiles_x * tiles_x * n);
    for (int t = 0; t < tiles_x * tiles_x; ++t) {
       const int x0 = (t % tiles_x) * 32, y0 = (t / tiles_x) * 32;
-      for (int i = 0; i < Pp; ++i) {
+      for (int i = first; i < first + n; ++i) {
          const double base = (t0[i] + (double)x0 * ad[i]) + (double)y0 * bd[i];
          const float ma = 31.f * a[i], mb = 31.f * b[i];
          const double tmin = (base + (double)std::fmin(0.f, ma)) + (double)std::fmin(0.f, mb);
@@ -450,22 +536,29 @@ size_t sweep_smem_bytes(int max_wlen2, int ach) {
    return std::max(rows, tiles);
 }
 
-cudaError_t launch_sweep(const SweepArgs& args, int max_wlen2, cudaStream_t st, int* grid_out) {
+template <int MINB>
+static cudaError_t launch_sweep_as(const SweepArgs& args, int max_wlen2, cudaStream_t st, int* grid_out) {
+   auto kern = sweep_persistent<MINB>;
    SweepArgs a = args;
    a.ach = sweep_smem_bytes(max_wlen2, kSweepACH) <= 100 * 1024 ? kSweepACH : 32;
    const size_t smem = sweep_smem_bytes(max_wlen2, a.ach);
    if (smem > 200 * 1024) return cudaErrorInvalidConfiguration;
-   cudaError_t e = cudaFuncSetAttribute(sweep_persistent, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
    if (e != cudaSuccess) return e;
    int dev = 0, sms = 0, per_sm = 0;
    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
    if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, sweep_persistent, kNT, smem)) != cudaSuccess)
+   if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kNT, smem)) != cudaSuccess)
       return e;
    const int grid = std::max(1, sms * std::max(1, per_sm));
    if (grid_out) *grid_out = grid;
-   sweep_persistent<<<grid, kNT, smem, st>>>(a);
+   kern<<<grid, kNT, smem, st>>>(a);
    return cudaGetLastError();
+}
+
+cudaError_t launch_sweep(const SweepArgs& a, int max_wlen2, cudaStream_t st, int* grid_out) {
+   return a.n_tiles >= kSweepManyTiles ? launch_sweep_as<3>(a, max_wlen2, st, grid_out)
+                                       : launch_sweep_as<2>(a, max_wlen2, st, grid_out);
 }
 
 }  // namespace risa_gb

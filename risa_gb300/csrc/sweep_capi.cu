@@ -22,14 +22,15 @@ struct risa_gb_sweep {
    std::vector<SweepInst> inst;
    std::vector<size_t> raw_off, img_off;
    size_t raw_total = 0, img_total = 0, pair_total = 0;
-   int max_wlen2 = 0, n_items = 0, grid = 0;
-   DevBuf d_inst, d_items, d_f32, d_f64, d_h, d_rep, d_pairs, d_twp[4], d_cnt, d_times;
+   int max_wlen2 = 0, n_items = 0, n_tiles = 0, grid = 0;
+   DevBuf d_inst, d_items, d_f32, d_f64, d_h, d_rep, d_pairs, d_part, d_twp[4], d_cnt, d_times;
    DevBuf d_win;  // per instance [tile][angle] window starts (sweep_tile_windows)
-   // d_cnt: [next][err][rows_done n][tiles_done n]; d_times: [t_first n][t_done n][t_launch]
+   // d_cnt: [next][err][rows_done n][tiles_done n][sums_done n]; d_times: [t_first n][t_done n][t_launch]
    int* next() const { return d_cnt.as<int>(); }
    int* err() const { return d_cnt.as<int>() + 1; }
    int* rows_done() const { return d_cnt.as<int>() + 2; }
    int* tiles_done() const { return d_cnt.as<int>() + 2 + n; }
+   int* sums_done() const { return d_cnt.as<int>() + 2 + 2 * n; }
    unsigned long long* t_first() const { return d_times.as<unsigned long long>(); }
    unsigned long long* t_done() const { return d_times.as<unsigned long long>() + n; }
    unsigned long long* t_launch() const { return d_times.as<unsigned long long>() + 2 * n; }
@@ -93,6 +94,13 @@ risa_gb_status risa_gb_sweep_create(const risa_gb_sweep_instance* in, int n, ris
    std::vector<SweepRepair> reps;
    std::vector<size_t> o_f32(n), o_f64(n), o_h(n), o_rep(n, (size_t)-1), o_win(n, (size_t)-1);
    std::vector<int2> win;
+   size_t n_tiles = 0;
+   for (int i = 0; i < n; ++i) {
+      const size_t t = in[i].n_pixels > 0 ? ((size_t)in[i].n_pixels + 31) / 32 : 0;
+      n_tiles += t * t;
+   }
+   h->n_tiles = (int)std::min<size_t>(n_tiles, 1u << 30);
+   const bool sets = h->n_tiles >= kSweepSetTiles;
    for (int i = 0; i < n; ++i) {
       const risa_gb_sweep_instance& s = in[i];
       if (s.n_pixels < 16 || s.n_par_proj < 1 || s.n_par_det < 2 || s.n_par_det > 65535 ||
@@ -145,11 +153,22 @@ risa_gb_status risa_gb_sweep_create(const risa_gb_sweep_instance* in, int n, ris
       h->raw_total += (size_t)g.Pp * g.Dp;
       h->img_total += (size_t)g.N * g.N;
       h->pair_total += (size_t)g.Pp * I.win_len;
+      I.n_base = I.combine_items = I.combine_px = I.n_extra = 0;
+      if (sets && g.rotation_offset == 0.0 && g.Pp % 2 == 0 && g.Pp >= 8) {
+         I.n_base = (g.Pp - 1) / 4;  // 0 < i < Pp / 4
+         I.extra[I.n_extra++] = 0;
+         I.extra[I.n_extra++] = g.Pp / 2;
+         if (g.Pp % 4 == 0) {
+            I.extra[I.n_extra++] = g.Pp / 4;
+            I.extra[I.n_extra++] = 3 * g.Pp / 4;
+         }
+      }
+      const int w_first = I.n_base ? 1 : 0, w_n = I.n_base ? I.n_base : g.Pp;
       // the tiles' window starts, built here once (8 B per tile and angle, up
       // to 1 GiB for the whole sweep; later instances compute them in FP64)
-      if ((win.size() + (size_t)I.tiles * g.Pp) * sizeof(int2) <= ((size_t)1 << 30)) {
+      if ((win.size() + (size_t)I.tiles * w_n) * sizeof(int2) <= ((size_t)1 << 30)) {
          o_win[i] = win.size();
-         sweep_tile_windows(t.a.data(), t.b.data(), t.ad.data(), t.bd.data(), t.t0.data(), g.Pp, g.N, win);
+         sweep_tile_windows(t.a.data(), t.b.data(), t.ad.data(), t.bd.data(), t.t0.data(), w_first, w_n, g.N, win);
       }
       o_f32[i] = f32.size();
       f32.insert(f32.end(), t.a.begin(), t.a.end());
@@ -182,8 +201,17 @@ risa_gb_status risa_gb_sweep_create(const risa_gb_sweep_instance* in, int n, ris
       I.repair = o_rep[i] == (size_t)-1 ? nullptr : h->d_rep.as<SweepRepair>() + o_rep[i];
       I.tile_win = o_win[i] == (size_t)-1 ? nullptr : h->d_win.as<int2>() + o_win[i];
    }
+   // pixels per combine item: short runs where the sums are the tail of a small
+   // sweep, long ones where thousands of items would be mostly their fetches
+   for (SweepInst& I : h->inst)
+      if (I.n_base > 0) {
+         const size_t px = (size_t)I.N * I.N;
+         I.combine_px = (int)std::min<size_t>(8192, std::max<size_t>(1024, h->img_total / 2048 / 256 * 256));
+         I.combine_items = (int)((px + I.combine_px - 1) / I.combine_px);
+      }
    RG_TRY(h->d_inst.upload(h->inst));
-   // work list: rows(0), rows(1), tiles(0), rows(2), tiles(1), ..., tiles(n-1)
+   // work list: rows(0), rows(1), tiles(0), rows(2), tiles(1), sums(0), ..., tiles(n-1),
+   // sums(n-2), sums(n-1)
    std::vector<SweepItem> items;
    auto rows = [&](int i) {
       for (int r = 0; r < h->inst[i].row_items; ++r) items.push_back(SweepItem{i, kSweepRows, r});
@@ -191,17 +219,25 @@ risa_gb_status risa_gb_sweep_create(const risa_gb_sweep_instance* in, int n, ris
    auto tiles = [&](int i) {
       for (int t = 0; t < h->inst[i].tiles; ++t) items.push_back(SweepItem{i, kSweepTile, t});
    };
+   auto sums = [&](int i) {
+      for (int c = 0; c < h->inst[i].combine_items; ++c) items.push_back(SweepItem{i, kSweepSum, c});
+   };
    rows(0);
    for (int i = 0; i < n; ++i) {
       if (i + 1 < n) rows(i + 1);
       tiles(i);
+      if (i > 0) sums(i - 1);
    }
+   sums(n - 1);
    h->n_items = (int)items.size();
    RG_TRY(h->d_items.upload(items));
    RG_TRY(h->d_pairs.alloc(sizeof(float2) * h->pair_total));
+   bool any_sums = false;
+   for (const SweepInst& I : h->inst) any_sums = any_sums || I.n_base > 0;
+   if (any_sums) RG_TRY(h->d_part.alloc(sizeof(float) * 4 * h->img_total));
    const int lens[4] = {512, 1024, 2048, 4096};
    for (int k = 0; k < 4; ++k) RG_TRY(h->d_twp[k].upload(filter_pass_twiddles(lens[k])));
-   RG_TRY(h->d_cnt.alloc(sizeof(int) * (2 + 2 * (size_t)n)));
+   RG_TRY(h->d_cnt.alloc(sizeof(int) * (2 + 3 * (size_t)n)));
    RG_TRY(h->d_times.alloc(sizeof(unsigned long long) * (2 * (size_t)n + 1)));
    RG_CUDA(cudaMemset(h->d_cnt.p, 0, h->d_cnt.bytes));
    *out = h.release();
@@ -231,11 +267,14 @@ risa_gb_status risa_gb_sweep_enqueue(risa_gb_sweep* h, const uint16_t* raw, floa
    a.n_items = h->n_items;
    a.raw = raw;
    a.img = img;
+   a.part = h->d_part.as<float>();
+   a.n_tiles = h->n_tiles;
    a.pairs = h->d_pairs.as<float2>();
    for (int k = 0; k < 4; ++k) a.twp[k] = h->d_twp[k].as<float2>();
    a.next = h->next();
    a.rows_done = h->rows_done();
    a.tiles_done = h->tiles_done();
+   a.sums_done = h->sums_done();
    a.t_first = h->t_first();
    a.t_done = h->t_done();
    a.t_launch = h->t_launch();
