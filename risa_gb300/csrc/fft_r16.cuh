@@ -62,9 +62,9 @@ __device__ __forceinline__ void dft8(float2* v) {
    v[3] = cadd(a3, b3); v[7] = csub(a3, b3);
 }
 
-// ---- register-resident radix-16 path, FFT lengths 512 .. 4096 --------------------
+// ---- register-resident radix-16 path, FFT lengths 256 .. 4096 --------------------
 // One row pair per LEN/16 threads, 16 complex values per thread, three
-// Stockham passes (radix 16; then 8 or 16; then 4, 8 or 16) whose butterflies
+// Stockham passes (radix 16; then 8 or 16; then 4, 8 or 16; two of radix 16 at 256) whose butterflies
 // run in registers. The first forward pass reads the rows straight from global
 // memory and the last inverse pass writes them back; the filter multiply is
 // applied to the registers of the last forward pass. Shared memory is touched
@@ -191,12 +191,14 @@ __device__ __forceinline__ void r16_store(float2* buf, int lt, const float2 (&v)
       }
 }
 
+// Radices of the passes after the first (16): R2, then R3. LEN 256 has no middle
+// pass (R2 = 1).
 template <int LEN>
 struct R16Plan {
-   static constexpr int R2 = LEN >= 2048 ? 16 : 8;
+   static constexpr int R2 = LEN >= 2048 ? 16 : LEN == 256 ? 1 : 8;
    static constexpr int NS3 = 16 * R2;
    static constexpr int R3 = LEN / NS3;
-   static constexpr int TW3 = R2 * 16;  // offset of pass 3's table in the pass-twiddle array
+   static constexpr int TW3 = R2 > 1 ? R2 * 16 : 0;  // offset of pass 3's table in the pass-twiddle array
 };
 
 // Forward FFT of the packed row pair held in v in the first pass's layout
@@ -222,11 +224,13 @@ __device__ __forceinline__ void r16_forward(float2 (&v)[16], float2* buf, int lt
    else r16_compute<LEN, 16, 1>(lt, v, nullptr);
    r16_store<LEN, 16, 1>(buf, lt, v);
    __syncthreads();
-   r16_load<LEN, P::R2>(buf, lt, v);
-   __syncthreads();
-   r16_compute<LEN, P::R2, 16>(lt, v, twp);
-   r16_store<LEN, P::R2, 16>(buf, lt, v);
-   __syncthreads();
+   if constexpr (P::R2 > 1) {
+      r16_load<LEN, P::R2>(buf, lt, v);
+      __syncthreads();
+      r16_compute<LEN, P::R2, 16>(lt, v, twp);
+      r16_store<LEN, P::R2, 16>(buf, lt, v);
+      __syncthreads();
+   }
    r16_load<LEN, P::R3>(buf, lt, v);
    __syncthreads();
    r16_compute<LEN, P::R3, P::NS3>(lt, v, twp + P::TW3);
@@ -262,11 +266,13 @@ __device__ __forceinline__ void r16_filter_core(float2 (&v)[16], float2* buf, in
    r16_compute<LEN, 16, 1>(lt, v, nullptr);
    r16_store<LEN, 16, 1>(buf, lt, v);
    __syncthreads();
-   r16_load<LEN, P::R2>(buf, lt, v);
-   __syncthreads();
-   r16_compute<LEN, P::R2, 16>(lt, v, tw2);
-   r16_store<LEN, P::R2, 16>(buf, lt, v);
-   __syncthreads();
+   if constexpr (P::R2 > 1) {
+      r16_load<LEN, P::R2>(buf, lt, v);
+      __syncthreads();
+      r16_compute<LEN, P::R2, 16>(lt, v, tw2);
+      r16_store<LEN, P::R2, 16>(buf, lt, v);
+      __syncthreads();
+   }
    r16_load<LEN, P::R3>(buf, lt, v);
    r16_compute<LEN, P::R3, P::NS3>(lt, v, tw3);
 }

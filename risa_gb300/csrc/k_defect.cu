@@ -3,12 +3,12 @@
 // The reference runs this on the host with a device->host->device round trip
 // per frame (DetectorInterpolation.cu:113-139) using findDefectDetectors and
 // interpolateDefectDetectors (interpolationFunctions.h:28-97). Here:
-//   1. defect_stats_cluster (detector-major frames): per-column total
+//   1. defect_stats_cluster: per-column total
 //      variation (exact integer sum, so the result does not depend on the
 //      reduction order) and max/min; a cluster of 8 CTAs covers one frame,
 //      one row chunk each, and the chunks are combined through distributed
-//      shared memory (no atomics, no zeroing pass); defect_stats (module-major
-//      frames) reduces its row chunks with integer atomics instead;
+//      shared memory (no atomics, no zeroing pass); defect_stats (frames whose
+//      columns are not in aligned octets) reduces its row chunks with integer atomics instead;
 //   2. defect_flags: one CTA per frame forms var = TV * range^2 in FP64,
 //      applies the 17-tap threshold with the reference's exact operation
 //      order (no FMA contraction) and compiles the ordered list of defect
@@ -69,35 +69,46 @@ __global__ void __launch_bounds__(kStatThreads) defect_stats(const uint16_t* __r
    atomicMin(&s->mn, mn);
 }
 
-// Detector-major frames with D % 8 == 0 and 16-byte aligned rows. A cluster
+// Frames whose 8 adjacent columns are contiguous and 16-byte aligned in every row
+// (D % 8 == 0; module-major with a module width of a multiple of 8). A cluster
 // of kStatCluster CTAs owns one frame and one block of column octets; CTA r
-// of the cluster takes row chunk r. Each thread takes 8 adjacent columns (one
+// of the cluster takes row chunk r, its RY groups of threads a share of the
+// chunk each. Each thread takes 8 adjacent columns (one
 // 16-byte load per row, kStatBatch rows in flight), keeps their max/min as
 // packed 16-bit pairs and their total variation in 32 bits (at most
 // `rows` * 65535 per chunk, rows <= 32768), and leaves them in shared memory;
-// after a cluster barrier CTA 0 sums the chunks in 64 bits, reading the other
+// the groups of a CTA are combined there, and after a cluster barrier CTA 0 sums
+// the chunks in 64 bits, reading the other
 // CTAs' shared memory, and writes the column statistics. Every CTA reaches
 // both cluster barriers (no early return), and a cluster's CTAs are
 // co-scheduled, so the barriers always complete.
+// RY = 1 (a block spans the frame's columns) streams a batch at 0.72 of the HBM
+// rate; RY = 8 (32 octets per block) is for a few frames, which are latency: 2
+// frames of 1000 x 1152 9 us instead of 23.
 constexpr int kStatCluster = 8;
 constexpr int kStatMaxThreads = 256;
 constexpr int kStatBatch = 8;
+template <int RY>
 __global__ void __cluster_dims__(kStatCluster, 1, 1) __launch_bounds__(kStatMaxThreads)
-    defect_stats_cluster(const uint16_t* __restrict__ frames, ColStats* __restrict__ st, int P, int D, int rows) {
+    defect_stats_cluster(const uint16_t* __restrict__ frames, ColStats* __restrict__ st, int P, int D, int rows,
+                         int modules) {
    __shared__ uint32_t part[16][kStatMaxThreads];  // tv[8], mx[4], mn[4] of every thread
    namespace cg = cooperative_groups;
    cg::cluster_group cl = cg::this_cluster();
    const unsigned rank = cl.block_rank();
-   const int t = threadIdx.x;
-   const int o = (blockIdx.x / kStatCluster) * blockDim.x + t;  // column octet
+   const int width = (int)blockDim.x / RY;  // octets of the block
+   const int t = RY == 1 ? (int)threadIdx.x : (int)threadIdx.x % width, ry = RY == 1 ? 0 : (int)threadIdx.x / width;
+   const int o = (blockIdx.x / kStatCluster) * width + t;  // column octet
    const bool act = 8 * o < D;
-   const int r0 = (int)rank * rows;
-   const int r1 = min(r0 + rows, P - 1);  // pairs (p, p+1) with p < r1
+   const int share = (rows + RY - 1) / RY;
+   const int r0 = (int)rank * rows + ry * share;
+   const int r1 = min(min(r0 + share, ((int)rank + 1) * rows), P - 1);  // pairs (p, p+1) with p < r1
    uint32_t mx[4] = {0u, 0u, 0u, 0u}, mn[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
    uint32_t tv[8] = {0, 0, 0, 0, 0, 0, 0, 0};
    if (act && r0 < r1) {
-      const uint4* f = reinterpret_cast<const uint4*>(frames + (size_t)blockIdx.z * P * D) + o;
-      const size_t rs = (size_t)D / 8;
+      const size_t rs = (size_t)(modules > 0 ? D / modules : D) / 8;
+      const uint4* f = reinterpret_cast<const uint4*>(frames + (size_t)blockIdx.z * P * D +
+                                                      raw_offset(0, 8 * o, P, D, modules));
       uint4 prev = __ldg(f + (size_t)r0 * rs);
       for (int p = r0; p < r1; p += kStatBatch) {
          uint4 nx[kStatBatch];
@@ -120,14 +131,26 @@ __global__ void __cluster_dims__(kStatCluster, 1, 1) __launch_bounds__(kStatMaxT
       }
    }
 #pragma unroll
-   for (int k = 0; k < 8; ++k) part[k][t] = tv[k];
+   for (int k = 0; k < 8; ++k) part[k][threadIdx.x] = tv[k];
 #pragma unroll
    for (int j = 0; j < 4; ++j) {
-      part[8 + j][t] = mx[j];
-      part[12 + j][t] = mn[j];
+      part[8 + j][threadIdx.x] = mx[j];
+      part[12 + j][threadIdx.x] = mn[j];
+   }
+   if (RY > 1) {  // the CTA's groups into its first one (its own 32-bit sums: rows * 65535 still fits)
+      __syncthreads();
+      for (int i = threadIdx.x; i < 16 * width; i += blockDim.x) {
+         const int k = i / width, c = i - k * width;
+         uint32_t v = part[k][c];
+         for (int g = 1; g < RY; ++g) {
+            const uint32_t w = part[k][g * width + c];
+            v = k < 8 ? v + w : k < 12 ? __vmaxu2(v, w) : __vminu2(v, w);
+         }
+         part[k][c] = v;
+      }
    }
    cl.sync();
-   if (rank == 0 && act) {
+   if (rank == 0 && act && ry == 0) {
       unsigned long long s64[8] = {0, 0, 0, 0, 0, 0, 0, 0};
       uint32_t MX[4] = {0u, 0u, 0u, 0u}, MN[4] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu};
       for (int q = 0; q < kStatCluster; ++q) {
@@ -303,48 +326,50 @@ __global__ void defect_flags(const ColStats* __restrict__ st, DefectCfg cfg,
       }
       return;
    }
-   if (threadIdx.x != 0) return;
-
-   // RISA mode: ordered run list of the reference's linear scan (single thread,
-   // its continuation rule and unsigned wraps reproduced exactly).
-   int n = 0;
-   // interpolationFunctions.h:76-96: flags[D] reads as 0
-   unsigned det = 0;
-   while (det < uD) {
-      if (flags[det]) {
-         const unsigned det0 = det;
+   // RISA mode: the run list of the reference's linear scan
+   // (interpolationFunctions.h:76-96; flags[D] reads as 0), in its order: a run
+   // starts at a flagged column after a good one or at column 0, and one that
+   // reaches the last column goes on over column 0 where that is flagged (its
+   // unsigned wraps reproduced exactly). The starts are numbered by ballots.
+   __shared__ int s_warp[32];
+   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = (int)blockDim.x >> 5;
+   int before = 0;  // runs that start in earlier blocks of columns
+   for (unsigned base = 0; base < uD; base += blockDim.x) {
+      const unsigned d = base + threadIdx.x;
+      const bool start = d < uD && flags[d] && (d == 0 || !flags[d - 1u]);
+      const unsigned vote = __ballot_sync(~0u, start);
+      if (lane == 0) s_warp[warp] = __popc(vote);
+      __syncthreads();
+      int n = before;
+      for (int w = 0; w < warp; ++w) n += s_warp[w];
+      n += __popc(vote & ((1u << lane) - 1u));
+      if (start && n < cfg.max_runs) {
+         unsigned det = d;
          while (flags[det] && flags[(det + 1u) % uD]) det++;
-         if (n < cfg.max_runs) {
-            DefectRun r;
-            r.start = (uint16_t)det0;
-            r.len = (uint16_t)(det - det0 + 1u);
-            r.left = (uint16_t)((det0 - 1u) % uD);
-            r.right = (uint16_t)((det + 1u) % uD);
-            out[n] = r;
-         }
-         ++n;
+         DefectRun r;
+         r.start = (uint16_t)d;
+         r.len = (uint16_t)(det - d + 1u);
+         r.left = (uint16_t)((d - 1u) % uD);
+         r.right = (uint16_t)((det + 1u) % uD);
+         out[n] = r;
       }
-      det++;
+      for (int w = 0; w < warps; ++w) before += s_warp[w];
+      __syncthreads();  // the counts are rewritten by the next block
    }
-   counts[f] = n < cfg.max_runs ? n : cfg.max_runs;
+   if (threadIdx.x == 0) counts[f] = before < cfg.max_runs ? before : cfg.max_runs;
 }
 
-__global__ void defect_repair(uint16_t* __restrict__ frames, DefectCfg cfg,
-                              const int* __restrict__ counts, const DefectRun* __restrict__ runs) {
-   const int p = blockIdx.x * blockDim.x + threadIdx.x;
+// One warp per row (one thread per row, walking all runs: 12 us for a frame of
+// 500 x 432).
+__global__ void __launch_bounds__(256) defect_repair(uint16_t* __restrict__ frames, DefectCfg cfg,
+                                                     const int* __restrict__ counts,
+                                                     const DefectRun* __restrict__ runs) {
+   const int p = blockIdx.x * 8 + (threadIdx.x >> 5);
    const int f = blockIdx.y;
    if (p >= cfg.P) return;
-   const int n = counts[f];
    uint16_t* fr = frames + (size_t)f * cfg.P * cfg.D;
-   auto at = [&](int x) -> uint16_t& { return fr[raw_offset(p, x, cfg.P, cfg.D, cfg.modules)]; };
-   const DefectRun* rl = runs + (size_t)f * cfg.max_runs;
-   for (int r = 0; r < n; ++r) {
-      const DefectRun run = rl[r];
-      for (int m = 0; m < run.len; ++m) {
-         const int col = (run.start + m) % cfg.D;
-         at(col) = defect_value(at(run.left), at(run.right), m, run.len, cfg.quirk);
-      }
-   }
+   repair_row_warp([&](int x) -> uint16_t& { return fr[raw_offset(p, x, cfg.P, cfg.D, cfg.modules)]; },
+                   runs + (size_t)f * cfg.max_runs, counts[f], cfg.D, cfg.quirk, threadIdx.x & 31);
 }
 }  // namespace
 
@@ -402,14 +427,21 @@ cudaError_t launch_defect_detect(const uint16_t* frames, int batch, const Defect
                                  DefectWorkspace ws, int32_t* flags_out, cudaStream_t st) {
    if (batch <= 0) return cudaSuccess;
    const int n = cfg.D * batch;
-   if (cfg.modules <= 0 && cfg.D % 8 == 0 && ((uintptr_t)frames & 15u) == 0 && cfg.P - 1 <= 8 * 32768) {
+   if (cfg.D % 8 == 0 && (cfg.modules <= 0 || (cfg.D / cfg.modules) % 8 == 0) && ((uintptr_t)frames & 15u) == 0 &&
+       cfg.P - 1 <= 8 * 32768) {
       // one block spans a frame's column octets where it can (D <= 2048);
-      // the cluster's CTAs split the rows
+      // the cluster's CTAs split the rows. A few frames (fewer CTAs of that kind
+      // than keep 152 SMs busy) take blocks of 32 octets with the rows split further.
       const int octets = cfg.D / 8;
-      const int threads = std::min(kStatMaxThreads, (octets + 31) / 32 * 32);
       const int rows = std::max(1, (cfg.P - 1 + kStatCluster - 1) / kStatCluster);
-      dim3 grid(kStatCluster * ((octets + threads - 1) / threads), 1, batch);
-      defect_stats_cluster<<<grid, threads, 0, st>>>(frames, ws.stats, cfg.P, cfg.D, rows);
+      if ((long)batch * kStatCluster < 8 * 152) {
+         dim3 grid(kStatCluster * ((octets + 31) / 32), 1, batch);
+         defect_stats_cluster<8><<<grid, 256, 0, st>>>(frames, ws.stats, cfg.P, cfg.D, rows, cfg.modules);
+      } else {
+         const int threads = std::min(kStatMaxThreads, (octets + 31) / 32 * 32);
+         dim3 grid(kStatCluster * ((octets + threads - 1) / threads), 1, batch);
+         defect_stats_cluster<1><<<grid, threads, 0, st>>>(frames, ws.stats, cfg.P, cfg.D, rows, cfg.modules);
+      }
    } else {
       defect_stats_init<<<(n + 255) / 256, 256, 0, st>>>(ws.stats, n);
       dim3 grid((cfg.D + kStatThreads - 1) / kStatThreads, (cfg.P - 1 + kStatRows - 1) / kStatRows,
@@ -417,7 +449,11 @@ cudaError_t launch_defect_detect(const uint16_t* frames, int batch, const Defect
       defect_stats<<<grid, kStatThreads, 0, st>>>(frames, ws.stats, cfg.P, cfg.D, cfg.modules);
    }
    const size_t smem = sizeof(double) * cfg.D + sizeof(float) * cfg.D + sizeof(int) * (cfg.D + 1);
-   defect_flags<<<batch, 256, smem, st>>>(ws.stats, cfg, flags_out, ws.counts, ws.runs, ws.fix_counts,
+   // up to one frame per SM takes wide blocks (one frame of 432 columns with its run
+   // list 6.9 us; 27 with 256 threads and one of them listing the runs), a batch
+   // fills the SMs with small ones (512 frames of 1152 columns 21 us)
+   const int threads = batch <= 152 ? std::min(1024, (cfg.D + 31) / 32 * 32) : 256;
+   defect_flags<<<batch, threads, smem, st>>>(ws.stats, cfg, flags_out, ws.counts, ws.runs, ws.fix_counts,
                                           ws.fixes);
    return cudaGetLastError();
 }
@@ -425,8 +461,8 @@ cudaError_t launch_defect_detect(const uint16_t* frames, int batch, const Defect
 cudaError_t launch_defect_repair(uint16_t* frames, int batch, const DefectCfg& cfg,
                                  DefectWorkspace ws, cudaStream_t st) {
    if (batch <= 0) return cudaSuccess;
-   dim3 grid((cfg.P + 127) / 128, batch);
-   defect_repair<<<grid, 128, 0, st>>>(frames, cfg, ws.counts, ws.runs);
+   dim3 grid((cfg.P + 7) / 8, batch);
+   defect_repair<<<grid, 256, 0, st>>>(frames, cfg, ws.counts, ws.runs);
    return cudaGetLastError();
 }
 

@@ -582,8 +582,8 @@ cudaError_t launch_filter_taps_grad(const float* x, const float* g, int batch, c
 
 std::vector<float2> filter_pass_twiddles(int len) {
    std::vector<float2> t;
-   if (len != 512 && len != 1024 && len != 2048 && len != 4096) return t;
-   const int r2 = len >= 2048 ? 16 : 8, ns3 = 16 * r2, r3 = len / ns3;
+   if (len != 256 && len != 512 && len != 1024 && len != 2048 && len != 4096) return t;
+   const int r2 = len >= 2048 ? 16 : len == 256 ? 1 : 8, ns3 = 16 * r2, r3 = len / ns3;
    auto add = [&t](int R, int NS) {
       for (int r = 0; r < R; ++r)
          for (int k = 0; k < NS; ++k) {
@@ -591,13 +591,13 @@ std::vector<float2> filter_pass_twiddles(int len) {
             t.push_back(make_float2((float)std::cos(ang), (float)std::sin(ang)));
          }
    };
-   add(r2, 16);
+   if (r2 > 1) add(r2, 16);
    add(r3, ns3);
    return t;
 }
 
 bool filter_pairs_supported(const FilterCfg& cfg) {
-   return cfg.twp && (cfg.len == 512 || cfg.len == 1024 || cfg.len == 2048 || cfg.len == 4096);
+   return cfg.twp && (cfg.len == 256 || cfg.len == 512 || cfg.len == 1024 || cfg.len == 2048 || cfg.len == 4096);
 }
 
 cudaError_t launch_filter_pairs(const float* sino, int batch, const FilterCfg& cfg, const PairsOut& po,
@@ -605,6 +605,7 @@ cudaError_t launch_filter_pairs(const float* sino, int batch, const FilterCfg& c
    if (batch <= 0) return cudaSuccess;
    if (!po.pairs || po.S % 2 || po.S < 0 || (po.S > 0 && po.wp <= 0)) return cudaErrorInvalidValue;
    switch (filter_pairs_supported(cfg) ? cfg.len : 0) {
+      case 256: return launch_r16_pairs<256>(sino, batch, cfg, po, st);
       case 512: return launch_r16_pairs<512>(sino, batch, cfg, po, st);
       case 1024: return launch_r16_pairs<1024>(sino, batch, cfg, po, st);
       case 2048: return launch_r16_pairs<2048>(sino, batch, cfg, po, st);
@@ -618,6 +619,7 @@ cudaError_t launch_filter(float* sino, int batch, const FilterCfg& cfg, cudaStre
    const int total_rows = batch * cfg.rows;
    if (cfg.twp) {
       switch (cfg.len) {
+         case 256: return launch_r16<256>(sino, total_rows, cfg, st);
          case 512: return launch_r16<512>(sino, total_rows, cfg, st);
          case 1024: return launch_r16<1024>(sino, total_rows, cfg, st);
          case 2048: return launch_r16<2048>(sino, total_rows, cfg, st);

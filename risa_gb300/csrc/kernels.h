@@ -77,6 +77,38 @@ template <class Row>
 __device__ __forceinline__ uint16_t repair_value(const Row& row, const DefectRun& run, int m, int quirk) {
    return defect_value(row[run.left], row[run.right], m, run.len, quirk);
 }
+// The defect runs of one row by a whole warp; at(column) is the sample. A run's
+// neighbours are good columns, which no run writes, so the lanes take runs in
+// parallel -- but for two of the reference's unsigned wraps, which its list order
+// decides in RISA mode: a first run from column 0 (its left neighbour is column
+// 2^32 - 1 mod D, defective or not, read before any other run) and a last run
+// that goes on over column 0 (its right neighbour is column 1, repaired by the
+// first run, and it writes column 0 again). Those run first and last.
+template <class At>
+__device__ __forceinline__ void repair_row_warp(const At& at, const DefectRun* __restrict__ runs, int n, int D,
+                                                int quirk, int lane) {
+   auto apply = [&](int i) {
+      const DefectRun run = runs[i];
+      for (int m = 0; m < run.len; ++m) {
+         int col = run.start + m;
+         if (col >= D) col -= D;
+         at(col) = defect_value(at(run.left), at(run.right), m, run.len, quirk);
+      }
+   };
+   int first = 0, last = n;
+   if (quirk == 1 && n > 0) {
+      if (runs[0].start == 0) {
+         if (lane == 0) apply(0);
+         first = 1;
+      }
+      if (n > first && runs[n - 1].start + runs[n - 1].len > D) last = n - 1;
+   }
+   __syncwarp();
+   for (int i = first + lane; i < last; i += 32) apply(i);
+   __syncwarp();
+   if (last < n && lane == 0) apply(last);
+   __syncwarp();
+}
 #endif
 // Workspace layout: [batch*D ColStats][batch int run counts][batch*max_runs DefectRun],
 // with `fixes`: then [batch int fix counts][batch*D DefectFix] (NONE mode only).
@@ -213,9 +245,9 @@ struct FilterCfg {
    const float2* twiddle;  // [len] exp(-2 pi i k / len)
    const float2* h;        // [len] frequency response (Hermitian: the filter taps are real)
    int adjoint;            // multiply by conj(h): the transposed filter
-   const float2* twp = nullptr;  // radix-16 path (len 512..4096): filter_pass_twiddles(len)
+   const float2* twp = nullptr;  // radix-16 path (len 256..4096): filter_pass_twiddles(len)
 };
-// Per-pass twiddles of the radix-16 filter path, built in FP64: pass 2 as
+// Per-pass twiddles of the radix-16 filter path, built in FP64: pass 2 (none at 256) as
 // [R2][16], then pass 3 as [R3][16*R2], entry [r][k] = exp(-2 pi i k r / (NS R)).
 // Empty for lengths the path does not cover.
 std::vector<float2> filter_pass_twiddles(int len);
