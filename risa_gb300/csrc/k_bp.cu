@@ -27,7 +27,8 @@ namespace risa_gb {
 namespace {
 
 // Linear interpolation variants: kernel kind, slices per CTA and angles per
-// chunk. The nearest-neighbour modes always use the plain tile kernel.
+// chunk. The nearest-neighbour modes always use the plain tile kernel, or its split
+// form for a few slices.
 enum VariantKind { kTile, kPairs, kAsync, kAsyncPacked, kPatch };
 struct BPVariant {
    int kind, slices, achunk, ppt;  // ppt: pixels per thread of the staged kernels
@@ -176,6 +177,115 @@ __global__ void __launch_bounds__(TX*(TY / PPT)) bp_tile(const float* __restrict
          out[(size_t)y * N + x] = v;
       }
    }
+}
+
+// ---- nearest-neighbour modes, a few slices ---------------------------------------
+// bp_tile gives a 32 x 32 tile to one CTA, which walks every angle: one slice of
+// 231^2 is 64 CTAs of eight warps, all latency. Here a CTA owns 16 of the tile's rows
+// and G groups of 256 threads take a share of the angles each, PX pixels 8 rows apart
+// per thread (warps of 8 x 4 pixels, whose bins are in one or two lines), and read the
+// sinogram itself: a few slices stay in L1 and L2, and with no windows to stage
+// the loads of several angles are in flight. The coordinate is formed as
+// bp_tile forms it, from the same tile origin, so each pixel takes the same bins;
+// the groups' sums are added in shared memory.
+constexpr int kSplitAngles = 512;  // angles per table of coordinates
+constexpr int kSplitGroups = 4, kSplitStrips = 2;
+template <int INTERP>
+__global__ void __launch_bounds__(256 * kSplitGroups) bp_nearest_split(const float* __restrict__ sino, float* __restrict__ img,
+                                                                       BPCfg cfg) {
+   constexpr int G = kSplitGroups, PX = kSplitStrips;
+   // a, b, coordinate of the tile's origin in its window, window start (less the
+   // bits of 2^23, from whose sum the floor is read)
+   __shared__ float4 tab[kSplitAngles];
+   __shared__ float part[G][PX][256];
+   const int N = cfg.N, Dp = cfg.Dp, Pp = cfg.Pp;
+   const int x0 = blockIdx.x * 32, y0 = (blockIdx.y / (4 / PX)) * 32, r0 = (blockIdx.y % (4 / PX)) * PX;
+   const int g = threadIdx.x >> 8, p = threadIdx.x & 255, warp = p >> 5, lane = p & 31;
+   const int tx = (warp & 3) * 8 + (lane & 7), ty = (warp >> 2) * 4 + (lane >> 3);
+   const int x = x0 + tx, ys = y0 + 8 * r0;
+   const float c = 0.5f * (float)(N - 1);
+   const float lim = (float)N * (float)N * 0.25f;
+   float* out = img + (size_t)blockIdx.z * N * N;
+   if (ys >= N) return;
+   if (cfg.masking) {  // a strip outside the inscribed circle
+      const float nx = fminf(fmaxf(c, (float)x0), (float)(x0 + 31)) - c;
+      const float ny = fminf(fmaxf(c, (float)ys), (float)(ys + 8 * PX - 1)) - c;
+      if (nx * nx + ny * ny > lim) {
+         if (g == 0)
+            for (int i = 0; i < PX; ++i)
+               if (x < N && ys + 8 * i + ty < N) out[(size_t)(ys + 8 * i + ty) * N + x] = cfg.mask_value;
+         return;
+      }
+   }
+   const float* q = sino + (size_t)blockIdx.z * Pp * Dp;
+   const float fx = (float)tx, fy = (float)ty;
+   float acc[PX];
+#pragma unroll
+   for (int i = 0; i < PX; ++i) acc[i] = 0.f;
+   for (int c0 = 0; c0 < Pp; c0 += kSplitAngles) {
+      const int na = min(kSplitAngles, Pp - c0);
+      __syncthreads();
+      for (int i = threadIdx.x; i < na; i += 256 * G) {
+         const int ang = c0 + i;
+         const float a = __ldg(cfg.a + ang), b = __ldg(cfg.b + ang);
+         const double base = __ldg(cfg.t0 + ang) + (double)x0 * __ldg(cfg.ad + ang) +
+                             (double)y0 * __ldg(cfg.bd + ang);
+         const double tmin = base + (double)fminf(0.f, 31.f * a) + (double)fminf(0.f, 31.f * b);
+         const int w0 = (int)floor(tmin) - 2;
+         tab[i] = make_float4(a, b, (float)(base - (double)w0), __uint_as_float((unsigned)w0 - 0x4B000000u));
+      }
+      __syncthreads();
+      const float* row = q + (size_t)(c0 + g) * Dp;
+#pragma unroll 8
+      for (int i = g; i < na; i += G, row += (size_t)G * Dp) {
+         const float4 e = tab[i];
+         const float tb = fmaf(fy, e.y, fmaf(fx, e.x, e.z));
+#pragma unroll
+         for (int j = 0; j < PX; ++j) {
+            const float t = fmaf((float)(r0 + j), 8.f * e.y, tb);  // at least 2
+            const float tt = t + (INTERP == RISA_GB_INTERP_NEAREST ? 0.5f : cfg.trunc_offset);
+            const float fl = __fadd_rd(tt, 8388608.f);  // floor(tt) in the low bits
+            unsigned k = __float_as_uint(fl) + __float_as_uint(e.w);
+            // truncation toward zero, as in bp_tile
+            if (INTERP != RISA_GB_INTERP_NEAREST && k == ~0u && tt != fl - 8388608.f) k = 0u;
+            if (k < (unsigned)Dp) acc[j] += __ldg(row + k);
+         }
+      }
+   }
+   if (G > 1) {
+#pragma unroll
+      for (int j = 0; j < PX; ++j) part[g][j][p] = acc[j];
+      __syncthreads();
+      if (g > 0) return;
+#pragma unroll
+      for (int h = 1; h < G; ++h)
+#pragma unroll
+         for (int j = 0; j < PX; ++j) acc[j] += part[h][j][p];
+   }
+#pragma unroll
+   for (int j = 0; j < PX; ++j) {
+      const int y = ys + 8 * j + ty;
+      if (x < N && y < N) {
+         float v = acc[j] * cfg.norm;
+         if (cfg.masking) {
+            const float dx = (float)x - c, dy = (float)y - c;
+            if (dx * dx + dy * dy > lim) v = cfg.mask_value;
+         }
+         out[(size_t)y * N + x] = v;
+      }
+   }
+}
+// Up to 512 tiles (slices together): 231^2 of 361 angles 63 -> 28 us for one slice,
+// 114 -> 108 for eight; 512^2 of 720 angles 135 -> 122 us for one, 213 -> 205 for
+// two. From there on bp_tile fills the GPU and its windows are cheaper than loads of
+// bins with their bounds (four slices of 512^2 335 against 393 us). One group per
+// strip of 8 rows (one pixel per thread) takes 33 us for the first.
+constexpr long kSplitMaxTiles = 512;
+template <int INTERP>
+cudaError_t launch_nearest_split(const float* sino, float* img, int batch, const BPCfg& cfg, cudaStream_t st) {
+   const int t = (cfg.N + 31) / 32;
+   bp_nearest_split<INTERP><<<dim3(t, t * (4 / kSplitStrips), batch), 256 * kSplitGroups, 0, st>>>(sino, img, cfg);
+   return cudaGetLastError();
 }
 
 // ---- linear interpolation, the hot kernel ---------------------------------------
@@ -1231,6 +1341,11 @@ cudaError_t launch_backprojection(const float* sino, float* img, int batch, cons
       cudaError_t e = cudaEventRecord(cfg.mid_event, st);
       if (e != cudaSuccess) return e;
    }
+   const long t = (cfg.N + 31) / 32;
+   if (cfg.interp != RISA_GB_INTERP_LINEAR && t * t * batch <= kSplitMaxTiles)
+      return cfg.interp == RISA_GB_INTERP_NEAREST
+                 ? launch_nearest_split<RISA_GB_INTERP_NEAREST>(sino, img, batch, cfg, st)
+                 : launch_nearest_split<RISA_GB_INTERP_NEAREST_TRUNC>(sino, img, batch, cfg, st);
    if (cfg.interp != RISA_GB_INTERP_LINEAR || variant < 0 || variant >= kNumVariants ||
        kVariants[variant].kind == kTile)
       return launch_interp<32, 32, 4, 32>(sino, img, batch, cfg, st);
