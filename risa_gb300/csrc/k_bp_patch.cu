@@ -875,6 +875,23 @@ bool bp_patch_plan(const float* a, const float* b, const double* ad, const doubl
    return true;
 }
 
+// Tiles with a pixel inside the inscribed circle (all without a mask), as the
+// kernel's test counts them, row by row.
+static long live_tiles(int N, bool masked) {
+   const int t = (N + kTile - 1) / kTile;
+   if (!masked) return (long)t * t;
+   const double c = 0.5 * (N - 1), lim = 0.25 * (double)N * N;
+   long n = 0;
+   for (int r = 0; r < t; ++r) {
+      const double y0 = (double)r * kTile, ny = std::max({y0 - c, c - (y0 + kTile - 1), 0.0});
+      if (ny * ny > lim) continue;
+      const double w = std::sqrt(lim - ny * ny);  // a tile from x0 on meets it if x0 <= c + w and x0 + 15 >= c - w
+      const long first = std::max(0L, (long)std::ceil((c - w - (kTile - 1)) / kTile));
+      n += std::min((long)t - 1, (long)std::floor((c + w) / kTile)) - first + 1;
+   }
+   return n;
+}
+
 // The rows, then one non-finite flag per quad.
 size_t bp_quads_bytes(int batch, int Pp, int Dp) {
    if (batch <= 0) return 0;
@@ -962,15 +979,38 @@ cudaError_t launch_bp_patch(const float* sino, float* img, int batch, const BPCf
    // phase fall in different banks as they are, so few quads per phase do as
    // well as eight and leave smaller CTAs: 16 slices of 1024^2 at 1 bin per pixel
    // 2.19 ms with (2, 2), 2.77 with (1, 4). Above, patches collide (64 slices at
-   // 1.5: (2, 2) 2.35 ms, (2, 8) 1.72) and a phase takes as many quads as the
-   // batch has. All forms add the same terms in the same order: same bits.
+   // 1.5: (2, 2) 2.35 ms, (2, 8) 1.72) and a phase takes more quads. All forms add
+   // the same terms in the same order: same bits.
    if (nq == 1) return launch_patch<1, 1, 10>(a, pp, cfg.scale, st);
    if (nq == 2) return launch_patch<1, 2, 6>(a, pp, cfg.scale, st);
-   if (cfg.scale <= 1.25f) return launch_patch<2, 2, 3>(a, pp, cfg.scale, st);
+   // The larger forms cost less per slice but leave more of the SMs idle at the end:
+   // the most CTAs that an SM gets, of the tiles that meet the circle where it is
+   // masked, times a form's cost.
+   const long live = live_tiles(cfg.N, cfg.masking != 0);
+   auto rounds = [live, nq](int quads) { return (live * ((nq + quads - 1) / quads) + 151) / 152; };
+   if (cfg.scale <= 1.25f) {
+      // Four quads per thread spread a patch's weights (a fifth of the FP32 work)
+      // over twice the slices: 1.84 times the time of half the slices (32 slices of
+      // 512^2 x 720 angles 773 us against 844, of 256^2 x 512 128 slices 570 against 618;
+      // 64 slices of that, four CTAs per SM for seven halves, 217 against 209), if an SM
+      // has two.
+      if (live * ((nq + 7) / 8) >= 304 && 184 * rounds(8) <= 100 * rounds(4))
+         return launch_patch<4, 2, 2>(a, pp, cfg.scale, st);
+      return launch_patch<2, 2, 3>(a, pp, cfg.scale, st);
+   }
    if (nq <= 4) return launch_patch<1, 4, 3>(a, pp, cfg.scale, st);
-   // 16 quads per CTA share a pixel's weights between twice the slices: 1.69
-   // times the time of 8 quads (2.11 against 1.25 ms, 512^2 x 1024 angles)
-   if (169 * ((nq + 15) / 16) <= 100 * ((nq + 7) / 8)) return launch_patch<2, 8, 1, true>(a, pp, cfg.scale, st);
-   return launch_patch<1, 8, 1>(a, pp, cfg.scale, st);
+   // The CTA of 16 quads shares a pixel's weights between twice the slices of 8 quads:
+   // 1.65 times the time of 8 quads (2.11 against 1.25 ms, 512^2 x 1024 angles; 60
+   // slices of 256^2 x 512, two for four, 398 us against 456, but for three, masked, 397
+   // against 356). That of 4 quads takes 0.6 of it, 0.53 up to 1.5 bins per pixel (30 masked
+   // slices of 256^2: 199 and 220 us at 1.5 and 2 bins, with 8 240 and 242; 64 slices of
+   // 128^2 at 2: one of 8 quads 80 us, two of 4 89, one of 16 119).
+   const long c4 = (cfg.scale <= 1.5f ? 53 : 60) * rounds(4), c8 = 100 * rounds(8), c16 = 165 * rounds(16);
+   if (c16 <= c8 && c16 <= c4) return launch_patch<2, 8, 1, true>(a, pp, cfg.scale, st);
+   if (c4 < c8) return launch_patch<1, 4, 3>(a, pp, cfg.scale, st);
+   // Two CTAs of 8 quads per SM (their registers held to 56, a few spilled) hide each
+   // other's waits, 30 slices of 512^2 1484 us against 1531; a CTA that has its SM to
+   // itself is faster without (20 masked slices of 200^2 129 us against 190).
+   return rounds(8) > 1 ? launch_patch<1, 8, 2>(a, pp, cfg.scale, st) : launch_patch<1, 8, 1>(a, pp, cfg.scale, st);
 }
 }  // namespace risa_gb

@@ -140,3 +140,20 @@ def test_patch_nonfinite_rows(value, n):
     # the flags are per call: a clean call after it is the clean result again
     bp.set_variant(_variant("patch_2x2"))
     np.testing.assert_array_equal(_run(bp, torch.from_numpy(base).cuda(), N, n), clean)
+
+
+@pytest.mark.parametrize("N,Dp,n", [
+    (400, 400, 29), (400, 400, 64), (400, 380, 61), (64, 64, 30), (400, 400, 33),  # four quads per thread, and not
+    (350, 525, 64), (350, 700, 61), (350, 700, 36), (350, 480, 20), (64, 128, 30), (64, 100, 61)])
+def test_shapes_add_the_same_terms(N, Dp, n):
+    """Large batches and images take other shapes than 8 slices do, with the same bits."""
+    g = rg.make_geometry(n_par_proj=37, n_par_det=Dp, n_pixels=N, rotation_offset=11.0)
+    bp = rg.Backprojection(g, rg.make_params(masking=True))
+    bp.reserve(n)
+    sino = torch.from_numpy(np.random.default_rng(Dp).standard_normal((n, 37, Dp)).astype(np.float32)).cuda()
+    got = _run(bp, sino, N, n)
+    for i in range(0, n, 8):
+        m = min(8, n - i)
+        if m <= 2 and n > 2:  # the tail as part of a full group
+            i, m = n - 8, 8
+        np.testing.assert_array_equal(got[i:i + m], _run(bp, sino[i:i + m].contiguous(), N, m))
