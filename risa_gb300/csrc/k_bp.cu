@@ -27,8 +27,8 @@ namespace risa_gb {
 namespace {
 
 // Linear interpolation variants: kernel kind, slices per CTA and angles per
-// chunk. The nearest-neighbour modes always use the plain tile kernel, or its split
-// form for a few slices.
+// chunk. The nearest-neighbour modes always use tile kernels of their own: the plain
+// one, one of several slices, or one that splits the angles for a few slices.
 enum VariantKind { kTile, kPairs, kAsync, kAsyncPacked, kPatch };
 struct BPVariant {
    int kind, slices, achunk, ppt;  // ppt: pixels per thread of the staged kernels
@@ -179,6 +179,137 @@ __global__ void __launch_bounds__(TX*(TY / PPT)) bp_tile(const float* __restrict
    }
 }
 
+// ---- nearest-neighbour modes, slice batches --------------------------------------
+// bp_tile for S slices of one geometry: a bin's S samples are one 16-byte (S = 4) or
+// 8-byte entry of the window, so the coordinate and bin of a pixel are formed once
+// and one load serves S slices -- 4 B of the shared-memory data path and ~2
+// instructions per update, where bp_tile spends ~8. Same bins, same order of
+// the angles: same bits. 16 slices of 512^2 x 720 angles 1145 -> 651 us, four of
+// 1024^2 x 1024 1622 -> 725; chunks of 16 angles 673 and 760.
+template <int S>
+struct NearestVec;
+template <>
+struct NearestVec<4> {
+   using T = float4;
+};
+template <>
+struct NearestVec<2> {
+   using T = float2;
+};
+constexpr int kNearestAngles = 32;  // most angles per chunk
+template <int INTERP, int S>
+__global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__ sino, float* __restrict__ img,
+                                                       BPCfg cfg, int wlen, int ach, int batch) {
+   using V = typename NearestVec<S>::T;
+   extern __shared__ __align__(16) unsigned char smem_raw[];
+   V* win = reinterpret_cast<V*>(smem_raw);  // [ach][wlen]
+   __shared__ float4 s_ang[kNearestAngles];  // a, b, coordinate of the tile's origin in its window, window start
+   const int N = cfg.N, Dp = cfg.Dp, Pp = cfg.Pp;
+   const int x0 = blockIdx.x * 32, y0 = blockIdx.y * 32, s0 = blockIdx.z * S;
+   const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+   const float c = 0.5f * (float)(N - 1);
+   const float lim = (float)N * (float)N * 0.25f;
+   bool live = true;
+   if (cfg.masking) {  // tiles entirely outside the inscribed circle
+      const float nx = fminf(fmaxf(c, (float)x0), (float)(x0 + 31)) - c;
+      const float ny = fminf(fmaxf(c, (float)y0), (float)(y0 + 31)) - c;
+      live = nx * nx + ny * ny <= lim;
+   }
+   float acc[4][S];
+#pragma unroll
+   for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int s = 0; s < S; ++s) acc[r][s] = 0.f;
+   const size_t fs = (size_t)Pp * Dp;
+   const float* q = sino + (size_t)s0 * fs;
+   const int ns = min(S, batch - s0);
+   constexpr uint32_t kFloorBits = 0x4B000000u;  // 2^23: floor(v) is in the low bits of v + 2^23 rounded down
+   const uint32_t top = kFloorBits + (uint32_t)wlen - 1u;
+
+   for (int c0 = 0; live && c0 < Pp; c0 += ach) {
+      const int na = min(ach, Pp - c0);
+      if (threadIdx.x < na) {
+         const int ang = c0 + threadIdx.x;
+         const float a = __ldg(cfg.a + ang), b = __ldg(cfg.b + ang);
+         const double base = __ldg(cfg.t0 + ang) + (double)x0 * __ldg(cfg.ad + ang) +
+                             (double)y0 * __ldg(cfg.bd + ang);
+         const double tmin = base + (double)fminf(0.f, 31.f * a) + (double)fminf(0.f, 31.f * b);
+         const int w0 = (int)floor(tmin) - 2;
+         s_ang[threadIdx.x] = make_float4(a, b, (float)(base - (double)w0), __int_as_float(w0));
+      }
+      __syncthreads();
+      for (int ai = ty; ai < na; ai += 8) {
+         const int w0 = __float_as_int(s_ang[ai].w);
+         const float* row = q + (size_t)(c0 + ai) * Dp;
+         for (int m = tx; m < wlen; m += 32) {
+            const int k = w0 + m;
+            const bool in = k >= 0 && k < Dp;
+            float v[S];
+#pragma unroll
+            for (int s = 0; s < S; ++s) v[s] = in && s < ns ? __ldg(row + (size_t)s * fs + k) : 0.f;
+            if constexpr (S == 4) win[ai * wlen + m] = make_float4(v[0], v[1], v[2], v[3]);
+            else win[ai * wlen + m] = make_float2(v[0], v[1]);
+         }
+      }
+      __syncthreads();
+#pragma unroll 2
+      for (int ai = 0; ai < na; ++ai) {
+         const float4 e = s_ang[ai];
+         const float tb = fmaf((float)ty, e.y, fmaf((float)tx, e.x, e.z));
+         const float bstep = 8.f * e.y;
+         const V* w = win + ai * wlen;
+#pragma unroll
+         for (int r = 0; r < 4; ++r) {
+            const float t = fmaf((float)r, bstep, tb);  // at least 2
+            const float tt = t + (INTERP == RISA_GB_INTERP_NEAREST ? 0.5f : cfg.trunc_offset);
+            const float fl = __fadd_rd(tt, 8388608.f);
+            uint32_t k = __float_as_uint(fl);
+            // truncation toward zero, as in bp_tile
+            if (INTERP != RISA_GB_INTERP_NEAREST && (int)(k - kFloorBits) + __float_as_int(e.w) == -1 &&
+                tt != fl - 8388608.f)
+               k += 1u;
+            const V u = w[min(k, top) - kFloorBits];
+            acc[r][0] += u.x;
+            acc[r][1] += u.y;
+            if constexpr (S == 4) {
+               acc[r][2] += u.z;
+               acc[r][3] += u.w;
+            }
+         }
+      }
+      __syncthreads();
+   }
+#pragma unroll
+   for (int r = 0; r < 4; ++r) {
+      const int x = x0 + tx, y = y0 + ty + 8 * r;
+      if (x >= N || y >= N) continue;
+      bool out = !live;
+      if (cfg.masking) {
+         const float dx = (float)x - c, dy = (float)y - c;
+         out = out || dx * dx + dy * dy > lim;
+      }
+#pragma unroll
+      for (int s = 0; s < S; ++s)
+         if (s < ns) img[((size_t)(s0 + s) * N + y) * N + x] = out ? cfg.mask_value : acc[r][s] * cfg.norm;
+   }
+}
+template <int INTERP, int S>
+cudaError_t launch_nearest_tile(const float* sino, float* img, int batch, const BPCfg& cfg, cudaStream_t st) {
+   const int wlen = window_len(cfg.scale, 32, 32);
+   // half the angles where the windows are wide (256^2 x 512 angles at 4 bins per pixel,
+   // 30 slices: 412 us, 503 with 32)
+   const int ach = cfg.scale <= 2.f ? kNearestAngles : kNearestAngles / 2;
+   const size_t smem = sizeof(float) * S * (size_t)ach * wlen;
+   auto kern = bp_nearest_tile<INTERP, S>;
+   if (smem > 47 * 1024) {
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+   }
+   const int t = (cfg.N + 31) / 32;
+   kern<<<dim3(t, t, (batch + S - 1) / S), 256, smem, st>>>(sino, img, cfg, wlen, ach, batch);
+   return cudaGetLastError();
+}
+
 // ---- nearest-neighbour modes, a few slices ---------------------------------------
 // bp_tile gives a 32 x 32 tile to one CTA, which walks every angle: one slice of
 // 231^2 is 64 CTAs of eight warps, all latency. Here a CTA owns 16 of the tile's rows
@@ -276,9 +407,9 @@ __global__ void __launch_bounds__(256 * kSplitGroups) bp_nearest_split(const flo
    }
 }
 // Up to 512 tiles (slices together): 231^2 of 361 angles 63 -> 28 us for one slice,
-// 114 -> 108 for eight; 512^2 of 720 angles 135 -> 122 us for one, 213 -> 205 for
-// two. From there on bp_tile fills the GPU and its windows are cheaper than loads of
-// bins with their bounds (four slices of 512^2 335 against 393 us). One group per
+// 74 -> 67 for four; 512^2 of 720 angles 135 -> 122 us for one. From there on the
+// tiles fill the GPU and their windows are cheaper than loads of bins with their
+// bounds (one slice of 1024^2 x 1024 468 against 556 us). One group per
 // strip of 8 rows (one pixel per thread) takes 33 us for the first.
 constexpr long kSplitMaxTiles = 512;
 template <int INTERP>
@@ -1341,11 +1472,25 @@ cudaError_t launch_backprojection(const float* sino, float* img, int batch, cons
       cudaError_t e = cudaEventRecord(cfg.mid_event, st);
       if (e != cudaSuccess) return e;
    }
-   const long t = (cfg.N + 31) / 32;
-   if (cfg.interp != RISA_GB_INTERP_LINEAR && t * t * batch <= kSplitMaxTiles)
-      return cfg.interp == RISA_GB_INTERP_NEAREST
-                 ? launch_nearest_split<RISA_GB_INTERP_NEAREST>(sino, img, batch, cfg, st)
-                 : launch_nearest_split<RISA_GB_INTERP_NEAREST_TRUNC>(sino, img, batch, cfg, st);
+   if (cfg.interp != RISA_GB_INTERP_LINEAR) {
+      const bool plain = cfg.interp == RISA_GB_INTERP_NEAREST;
+      const long t = (cfg.N + 31) / 32, tiles = t * t;
+      // Several slices per thread where that leaves 256 CTAs and the windows of 32
+      // angles fit a few CTAs per SM (512^2 x 720 angles, bp_tile / 2 / 4 slices: two
+      // slices 213 / 175 / 240 us, three 294 / 250 / 242, sixteen 1145 / 752 / 651; at 4
+      // bins per pixel 468 / 415 / 412, at 16 1333 / 1772 / 2197)
+      const int s = cfg.scale > 4.f ? 1 : batch >= 3 && tiles * ((batch + 3) / 4) >= 256 ? 4
+                    : batch >= 2 && tiles * ((batch + 1) / 2) >= 256 ? 2 : 1;
+      if (s == 4)
+         return plain ? launch_nearest_tile<RISA_GB_INTERP_NEAREST, 4>(sino, img, batch, cfg, st)
+                      : launch_nearest_tile<RISA_GB_INTERP_NEAREST_TRUNC, 4>(sino, img, batch, cfg, st);
+      if (s == 2)
+         return plain ? launch_nearest_tile<RISA_GB_INTERP_NEAREST, 2>(sino, img, batch, cfg, st)
+                      : launch_nearest_tile<RISA_GB_INTERP_NEAREST_TRUNC, 2>(sino, img, batch, cfg, st);
+      if (tiles * batch <= kSplitMaxTiles)
+         return plain ? launch_nearest_split<RISA_GB_INTERP_NEAREST>(sino, img, batch, cfg, st)
+                      : launch_nearest_split<RISA_GB_INTERP_NEAREST_TRUNC>(sino, img, batch, cfg, st);
+   }
    if (cfg.interp != RISA_GB_INTERP_LINEAR || variant < 0 || variant >= kNumVariants ||
        kVariants[variant].kind == kTile)
       return launch_interp<32, 32, 4, 32>(sino, img, batch, cfg, st);

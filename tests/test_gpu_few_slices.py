@@ -36,6 +36,25 @@ def test_nearest_split_picks_the_same_bins(Pp, Dp, N, rot, masking, interp, quir
         np.testing.assert_array_equal(got.cpu().numpy(), exp[:n].cpu().numpy())
 
 
+@pytest.mark.parametrize("quirk", [rg.QUIRKS_RISA, rg.QUIRKS_NONE])
+@pytest.mark.parametrize("interp", [rg.INTERP_NEAREST, rg.INTERP_NEAREST_TRUNC])
+@pytest.mark.parametrize("Dp,N,n,masking", [(600, 750, 2, True), (601, 737, 3, False), (1100, 750, 7, True),
+                                            (2990, 750, 5, False), (33, 740, 4, False)])
+def test_nearest_batches_match_single_slices(Dp, N, n, masking, interp, quirk):
+    """Two or four slices per thread against the one-slice tiles that one slice of more than 512
+    tiles takes, bit for bit; angles that are no multiple of a chunk, partial groups of slices."""
+    Pp = 45
+    g = rg.make_geometry(n_par_proj=Pp, n_par_det=Dp, n_pixels=N, rotation_offset=-33.0)
+    bp = rg.Backprojection(g, rg.make_params(quirks=quirk, interp=interp, masking=masking, masking_value=7.0))
+    sino = torch.from_numpy(np.random.default_rng(N).standard_normal((n, Pp, Dp)).astype(np.float32)).cuda()
+    got = torch.full((n, N, N), float("nan"), dtype=torch.float32, device="cuda")
+    bp.enqueue(sino, got, n)
+    for i in range(n):
+        exp = torch.full((1, N, N), float("nan"), dtype=torch.float32, device="cuda")
+        bp.enqueue(sino[i:i + 1].contiguous(), exp, 1)
+        np.testing.assert_array_equal(got[i].cpu().numpy(), exp[0].cpu().numpy())
+
+
 @pytest.mark.parametrize("N,n", [(16, 1), (17, 3), (90, 1), (91, 2), (181, 5), (512, 1)])
 def test_normalisation_range(N, n):
     g = rg.make_geometry(n_pixels=N)
