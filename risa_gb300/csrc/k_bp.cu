@@ -1199,8 +1199,9 @@ __device__ __forceinline__ ulonglong2 ldg_if(const ulonglong2* ptr, bool p) {
 // for steep angles). A warp is 32 consecutive bins of one angle; the warps of a
 // CTA are `apc` consecutive angles over the same bins, whose rays cross a row at
 // nearly the same pixels, so the image passes from L2 to L1 once per CTA and not
-// once per angle; `rs` warps share an angle's rows where the bins alone leave
-// the GPU idle, and their sums are added in a fixed order.
+// once per angle. Each sum runs over the rows in bp_adjoint's order, with the same
+// terms: the same bits (shares of the rows per warp, added at the end, were faster
+// for small geometries but rounded differently).
 // What bounds it is L1 wavefronts: per row and warp, two candidate pixels of NH
 // 16-byte loads (4.5 wavefronts each; 82% of the data path). 16 slices of 512^2
 // -> 720 x 768: 1.77 ms with 32-byte pixel records and one angle per CTA (7
@@ -1209,21 +1210,21 @@ __device__ __forceinline__ ulonglong2 ldg_if(const ulonglong2* ptr, bool p) {
 template <int NH>
 __global__ void __launch_bounds__(256) bp_adjoint_rows(const float4* __restrict__ P, const float4* __restrict__ PT,
                                                        float* __restrict__ sino, BPCfg cfg, int batch, int apc,
-                                                       int rs) {
-   extern __shared__ float2 s_line[];  // the angles' line starts [apc][N]; then the partial sums
+                                                       int halves) {
+   extern __shared__ float2 s_line[];  // the angles' line starts [apc][N]
    const int N = cfg.N, Dp = cfg.Dp;
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   const int sub = warp % apc, part = warp / apc;  // angle of the CTA, share of the rows
    const int k = blockIdx.x * 32 + lane;
-   const int i = blockIdx.y * apc + sub, g = blockIdx.z;
-   for (int w = warp; w < apc; w += apc * rs) {
-      const int iw = blockIdx.y * apc + w;
-      if (iw >= cfg.Pp) continue;
-      const bool ax = fabsf(__ldg(cfg.a + iw)) >= fabsf(__ldg(cfg.b + iw));
-      const float2* line = (ax ? cfg.rowbase : cfg.colbase) + (size_t)iw * N;
-      for (int r = lane; r < N; r += 32) s_line[w * N + r] = __ldg(line + r);
+   const int i = blockIdx.y * apc + warp;
+   const int g = NH == 1 && halves > 1 ? blockIdx.z >> 1 : blockIdx.z, half = NH == 1 && halves > 1 ? blockIdx.z & 1 : 0;
+   const int first = 8 * g + 4 * half;  // first slice
+   if (first >= batch) return;
+   if (i < cfg.Pp) {
+      const bool ax = fabsf(__ldg(cfg.a + i)) >= fabsf(__ldg(cfg.b + i));
+      const float2* line = (ax ? cfg.rowbase : cfg.colbase) + (size_t)i * N;
+      for (int r = lane; r < N; r += 32) s_line[warp * N + r] = __ldg(line + r);
    }
-   __syncthreads();
+   __syncthreads();  // the warps set out together, over the same pixels
    unsigned long long acc2[2 * NH];
 #pragma unroll
    for (int q = 0; q < 2 * NH; ++q) acc2[q] = 0ull;
@@ -1234,8 +1235,8 @@ __global__ void __launch_bounds__(256) bp_adjoint_rows(const float4* __restrict_
       const float s_lo = (float)((along_x ? __ldg(cfg.ad + i) : __ldg(cfg.bd + i)) - (double)s_hi);
       const float inv = 1.0f / s_hi;  // |s_hi| >= scale / sqrt(2) > 0
       const size_t plane = (size_t)N * N;
-      const ulonglong2* im = reinterpret_cast<const ulonglong2*>((along_x ? P : PT) + (size_t)g * plane * 2);
-      const float2* lines = s_line + sub * N;
+      const ulonglong2* im = reinterpret_cast<const ulonglong2*>((along_x ? P : PT) + (size_t)(2 * g + half) * plane);
+      const float2* lines = s_line + warp * N;
       const float kf = (float)k;
       // Rows whose candidates can lie in the image, for any bin of the warp: the
       // ray of bin k crosses row r near j = c0 + slope r (margin 3 pixels, the
@@ -1254,11 +1255,6 @@ __global__ void __launch_bounds__(256) bp_adjoint_rows(const float4* __restrict_
          if (k >= Dp || r1 <= r0) r0 = N, r1 = 0;
          r0 = __reduce_min_sync(~0u, r0);
          r1 = __reduce_max_sync(~0u, r1);
-      }
-      if (rs > 1 && r1 > r0) {
-         const int len = (r1 - r0 + rs - 1) / rs, first = r0 + part * len;
-         r1 = min(r1, first + len);
-         r0 = first;
       }
       // The pixels of a row within one bin of k lie in the open interval from
       // jlo = (-/+1 - t0) / s of length 2 / |s|; the candidates are the
@@ -1338,25 +1334,13 @@ __global__ void __launch_bounds__(256) bp_adjoint_rows(const float4* __restrict_
          }
       }
    }
-   if (rs > 1) {  // sum the row shares of an angle in their order
-      __syncthreads();
-      unsigned long long* part_sums = reinterpret_cast<unsigned long long*>(s_line);  // [warp][2 NH][32]
-#pragma unroll
-      for (int q = 0; q < 2 * NH; ++q) part_sums[(warp * 2 * NH + q) * 32 + lane] = acc2[q];
-      __syncthreads();
-      if (part > 0) return;
-      for (int p = 1; p < rs; ++p)
-#pragma unroll
-         for (int q = 0; q < 2 * NH; ++q)
-            acc2[q] = f2_add(acc2[q], part_sums[((p * apc + sub) * 2 * NH + q) * 32 + lane]);
-   }
    if (i >= cfg.Pp || k >= Dp) return;
    float acc[4 * NH];
 #pragma unroll
    for (int q = 0; q < 2 * NH; ++q) f2_unpack(acc2[q], acc[2 * q], acc[2 * q + 1]);
 #pragma unroll
    for (int s = 0; s < 4 * NH; ++s)
-      if (8 * g + s < batch) sino[((size_t)(8 * g + s) * cfg.Pp + i) * Dp + k] = acc[s] * cfg.norm;
+      if (first + s < batch) sino[((size_t)(first + s) * cfg.Pp + i) * Dp + k] = acc[s] * cfg.norm;
 }
 }  // namespace
 
@@ -1539,18 +1523,19 @@ cudaError_t launch_backprojection_adjoint(const float* img, float* sino, int bat
       float4* PT = P + (size_t)groups * cfg.N * cfg.N * 2;
       dim3 lg((cfg.N + 31) / 32, (cfg.N + 31) / 32, groups);
       bp_adjoint_layout<<<lg, 256, 0, st>>>(img, P, PT, cfg.N, batch);
-      // 8 warps per CTA; row shares so that small geometries still fill the GPU
-      // (about 32 warps on each of 152 SMs)
-      const long warps = (long)((cfg.Dp + 31) / 32) * cfg.Pp * groups;
-      const int rs = warps >= 4864 ? 1 : warps >= 2432 ? 2 : 4;
-      int apc = 8 / rs;
+      // Eight angles per CTA share the image rows in L1, fewer where that leaves fewer
+      // than two CTAs per SM; below 32 warps per SM a group of 8 slices goes to two
+      // warps (8 slices of 290^2 -> 161 x 372 112 us, 132 with one warp, 221 without the
+      // layout; one of 96^2 -> 90 x 96 43, 48 with eight angles per CTA, 85 without).
+      const int columns = (cfg.Dp + 31) / 32;
+      const int halves = batch > 4 && (long)columns * cfg.Pp * groups < 4864 ? 2 : 1;
+      int apc = 8;
+      while (apc > 1 && (long)columns * ((cfg.Pp + apc - 1) / apc) * groups * halves < 304) apc /= 2;
       while (apc > 1 && sizeof(float2) * (size_t)apc * cfg.N > 48 * 1024) apc /= 2;
-      const bool one = batch <= 4;
-      const size_t sums = rs > 1 ? sizeof(float2) * 32 * (one ? 2 : 4) * (size_t)(apc * rs) : 0;
-      const size_t lines = std::max(sizeof(float2) * (size_t)apc * cfg.N, sums);
-      dim3 grid((cfg.Dp + 31) / 32, (cfg.Pp + apc - 1) / apc, groups);
-      if (one) bp_adjoint_rows<1><<<grid, 32 * apc * rs, lines, st>>>(P, PT, sino, cfg, batch, apc, rs);
-      else bp_adjoint_rows<2><<<grid, 32 * apc * rs, lines, st>>>(P, PT, sino, cfg, batch, apc, rs);
+      const size_t lines = sizeof(float2) * (size_t)apc * cfg.N;
+      dim3 grid(columns, (cfg.Pp + apc - 1) / apc, groups * halves);
+      if (batch <= 4 || halves > 1) bp_adjoint_rows<1><<<grid, 32 * apc, lines, st>>>(P, PT, sino, cfg, batch, apc, halves);
+      else bp_adjoint_rows<2><<<grid, 32 * apc, lines, st>>>(P, PT, sino, cfg, batch, apc, halves);
       return cudaGetLastError();
    }
    if (batch >= 8) {
