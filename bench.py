@@ -39,13 +39,11 @@ WORKLOAD = dict(n_planes=2, n_fan_det=1152, n_fan_proj=1000, n_par_proj=1024, n_
                 delta_x=[0.0, 0.0], delta_z=[1417.0, 1430.0], source_angle=[360.0, 360.0])
 FRAMES_PER_PLANE = 2000
 FLOPS_PER_UPDATE = 6  # ray coordinate FMA (2) + weight add (1) + interpolation FMA (2) + accumulate (1)
-SMEM_BYTES_PER_UPDATE = 8  # one FP32 (midpoint, difference) pair per pixel x angle and slice
 SMEM_BYTES_PER_CLK_SM = 128  # nominal shared-memory bandwidth per SM
-# dram__bytes_read.sum + dram__bytes_write.sum of a 64-slice launch of the autotuned
-# backprojection variant (staged_cp_s4_a8_p4, profiles/bp_staged_fbp512_ncu.txt):
-# the pair records read once and the images written, both proportional to the
-# slices, so a launch of B slices moves B/64 of it
-BP_DRAM_BYTES_PER_SLICE = 722.1e6 / 64
+# dram__bytes_read.sum + dram__bytes_write.sum of a 64-slice launch of patch_2x2
+# (profiles/bp_patch_fbp512_ncu.txt): the slice quads read once and the images
+# written, both proportional to the slices, so a launch of B slices moves B/64 of it
+BP_DRAM_BYTES_PER_SLICE = 336e6 / 64
 WORKLOAD_NAME = ("full-rate streaming: 2 planes x 2000 frames of 1000x1152 uint16 fan sinograms, 1% defective "
                  "detectors -> 1024x1024 parallel (pad 2048, Shepp-Logan) -> 512^2 FP32, circular mask")
 
@@ -339,6 +337,19 @@ def timed(torch, stream, fn, reps: int) -> float:
     return e0.elapsed_time(e1) / reps
 
 
+def bp_smem_bytes_per_update(variant_name):
+    """Shared-memory bytes per pixel x angle update and slice of the workload's
+    backprojection: a 2 x 2 patch reads floor(|a| + |b|) + 3 bins of 4 B per slice
+    for its 4 pixels (a, b: bins per pixel along x and y); the record variants
+    read one FP32 (midpoint, difference) pair per pixel."""
+    if variant_name != "patch_2x2":
+        return 8.0
+    scale = WORKLOAD["n_par_det"] / WORKLOAD["n_pixels"]
+    th = np.arange(WORKLOAD["n_par_proj"]) * np.pi / WORKLOAD["n_par_proj"]
+    span = scale * (np.abs(np.cos(th)) + np.abs(np.sin(th)))
+    return float(np.mean(np.minimum(np.floor(span), 2) + 3))
+
+
 def measure_e2e(args, sc, fbp, torch, rg):
     """Seconds per step through risa_gb_fbp_run_host: pinned host frames in,
     pinned host images out, the copies inside the timed region. Each step is
@@ -388,33 +399,34 @@ def measure_extras(args, sc, fbp, raw, img, stream, B, variant, torch, rg, g, p)
     fs, ps = Pf * Df, Pp * Dp
     att_bytes = B * fs * (2 + 4) + L * fs * 4
     f2p_bytes = B * (fs * 4 + ps * 4) + L * ps * 4 * 12
-    # the filter reads the rebinned sinogram; fused with the staging pass it
-    # writes the padded pair records (8 B per window bin, angle and slice)
-    win_lo, win_len = bp.window(True)
-    # with a staged variant the filter writes the pair records itself and no
+    # with a staged variant the filter writes its rows itself (slice quads, 4 B
+    # per bin, angle and slice, or the padded records, 8 B per window bin) and no
     # staging pass runs (its event interval is then only the events' own
     # overhead, a few microseconds against ~1 ms for a real staging pass)
+    vname = rg.Backprojection.variant_name(variant)
+    win_lo, win_len = bp.window(True)
     prefilled = t_stage < 0.05 * t_filt
-    filt_bytes = B * ps * 4 + (B * Pp * win_len * 8 if prefilled else B * ps * 4)
+    records = prefilled and vname != "patch_2x2"
+    filt_bytes = B * ps * 4 + (B * Pp * win_len * 8 if records else B * ps * 4)
     yy, xx = np.mgrid[:N, :N]
     inside = int(((xx - (N - 1) / 2) ** 2 + (yy - (N - 1) / 2) ** 2 <= N * N / 4).sum())
     updates = B * inside * Pp
-    # The backprojection kernel is bound by shared-memory bandwidth: every
-    # update reads one FP32 (midpoint, difference) pair of its slice (8 B).
+    # The backprojection kernel is bound by shared-memory bandwidth.
     # Denominators measured on this GPU (risa_gb_measure_peak), nominal beside.
     smem_meas = rg.measure_peak(rg.PEAK_SMEM_READ, 5, stream)
     fma_meas = rg.measure_peak(rg.PEAK_FP32_FMA, 5, stream)
     smem_nominal = SMEM_BYTES_PER_CLK_SM * sms * sm_mhz * 1e6 / 1e9  # GB/s
     smem_peak = smem_meas["value"]
     fp32_peak_meas = fma_meas["value"]
-    smem_gbs = updates * SMEM_BYTES_PER_UPDATE / (t_kern / 1e3) / 1e9
+    smem_bytes = bp_smem_bytes_per_update(vname)
+    smem_gbs = updates * smem_bytes / (t_kern / 1e3) / 1e9
     bp_tflops = updates * FLOPS_PER_UPDATE / (t_kern / 1e3) / 1e12
     out["roofline"] = {
-        "kernel": f"bp_linear_async ({rg.Backprojection.variant_name(variant)})", "bound": "smem",
+        "kernel": f"{'bp_patch' if vname == 'patch_2x2' else 'bp_linear_async'} ({vname})", "bound": "smem",
         "achieved": smem_gbs, "peak": smem_peak, "unit": "GB/s", "frac": smem_gbs / smem_peak,
         "traffic": BP_DRAM_BYTES_PER_SLICE * B,
         "traffic_source": "ncu capture of a 64-slice launch, scaled by slices per launch",
-        "work": f"{SMEM_BYTES_PER_UPDATE} B of shared-memory reads per pixel x angle update and slice, "
+        "work": f"{smem_bytes:.2f} B of shared-memory reads per pixel x angle update and slice, "
                 f"{inside} in-circle pixels x {Pp} angles x {B} slices per launch",
         "peak_source": "measured: risa_gb_measure_peak(RISA_GB_PEAK_SMEM_READ), conflict-free 128-bit "
                        f"shared loads on all {sms} SMs, {smem_meas['per_sm_per_clk']:.1f} B/clk/SM at "
@@ -440,8 +452,8 @@ def measure_extras(args, sc, fbp, raw, img, stream, B, variant, torch, rg, g, p)
                      "frac_hbm": f2p_bytes / (t_f2p / 1e3) / 1e9 / hbm},
         "filter": {"ms": t_filt, "gbs": filt_bytes / (t_filt / 1e3) / 1e9,
                    "frac_hbm": filt_bytes / (t_filt / 1e3) / 1e9 / hbm,
-                   "writes": "pair records, %d bins per angle and slice" % win_len if prefilled
-                             else "filtered sinogram"},
+                   "writes": "pair records, %d bins per angle and slice" % win_len if records
+                             else "slice quads" if prefilled else "filtered sinogram"},
         "backprojection": {"ms": t_bp},
         "defect_detect": {"ms": t_def, "gbs": B * fs * 2 / (t_def / 1e3) / 1e9},
         "hbm_peak_gbs": hbm, "batch": B,

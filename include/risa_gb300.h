@@ -316,11 +316,12 @@ risa_gb_status risa_gb_backprojection_set_variant(risa_gb_backprojection* h, int
 int risa_gb_backprojection_variant_count(void);
 /* Static name of a variant ("invalid" when out of range). */
 const char* risa_gb_backprojection_variant_name(int variant);
-/* Allocates the device buffer the asynchronous variants stage from (a padded
- * (midpoint, difference) copy of the sinogram) for batches up to max_batch.
- * Set-up call: may allocate and synchronise. Autotune and the FBP engine
- * reserve for their batch themselves; an enqueue whose batch exceeds the
- * reservation runs a variant that stages windows from the sinogram itself. */
+/* Allocates the device buffer the staged variants read from (slice quads of the
+ * sinogram, or its padded (midpoint, difference) records) for batches up to
+ * max_batch. Set-up call: may allocate and synchronise. Autotune and the FBP engine
+ * reserve for their batch themselves, and a new handle holds four slices (where
+ * that is at most 64 MB); an enqueue whose batch exceeds the reservation runs a
+ * variant that stages windows from the sinogram itself. */
 risa_gb_status risa_gb_backprojection_reserve(risa_gb_backprojection* h, int max_batch);
 /* Measurement: runs `reps` enqueues (after one warm-up) with CUDA events on
  * `stream` around the staging pass and around the backprojection kernel, and
@@ -333,8 +334,7 @@ risa_gb_status risa_gb_backprojection_time(risa_gb_backprojection* h, const floa
  * one transposed, 8 N^2 floats per group of 8 slices) for batches up to
  * max_batch. Set-up call: may allocate and synchronise. An adjoint enqueue
  * whose batch exceeds the reservation gathers from the image directly (same
- * results within FP32 rounding, several times slower). No reference
- * counterpart. */
+ * results, several times slower). No reference counterpart. */
 risa_gb_status risa_gb_backprojection_reserve_adjoint(risa_gb_backprojection* h, int max_batch);
 /* Padded pair-sinogram window of the staged variants: per angle, window bin u
  * holds detector bin u - win_lo, u < win_len (fused_mask 0: every tile; 1: the
@@ -410,15 +410,15 @@ risa_gb_status risa_gb_fbp_set_lanes(risa_gb_fbp* h, int lanes);
  * side, [quad][n_fan_proj][n_fan_det][4] float, quads of plane k before those of
  * plane k+1 -- and parallel sinograms per frame, [batch][n_par_proj][n_par_det]
  * (rebinned; with a staged backprojection variant and a radix-16 filter length
- * the filter writes the backprojection's pair records directly and the
- * filtered sinogram is not stored). The fan buffer holds at least max_batch
+ * the filter writes the backprojection's rows directly and the filtered
+ * sinogram is not stored). The fan buffer holds at least max_batch
  * frames. */
 risa_gb_status risa_gb_fbp_intermediates(risa_gb_fbp* h, float** fan, float** par);
 /* Measurement: runs the engine's stages on one batch `reps` times (after a
  * warm-up) with CUDA events on `stream` between them; ms[6] receives the mean
  * durations of defect detection, attenuation (+ repair), rebinning, filter,
  * backprojection staging and the backprojection kernel (staging 0 where the
- * filter writes the pair records itself). Synchronises. */
+ * filter writes its rows itself). Synchronises. */
 risa_gb_status risa_gb_fbp_time_stages(risa_gb_fbp* h, const uint16_t* raw, float* img, int plane, int batch,
                                        int reps, void* stream, float* ms);
 risa_gb_backprojection* risa_gb_fbp_backprojection(risa_gb_fbp* h);
