@@ -41,9 +41,10 @@ FRAMES_PER_PLANE = 2000
 FLOPS_PER_UPDATE = 6  # ray coordinate FMA (2) + weight add (1) + interpolation FMA (2) + accumulate (1)
 SMEM_BYTES_PER_CLK_SM = 128  # nominal shared-memory bandwidth per SM
 # dram__bytes_read.sum + dram__bytes_write.sum of a 64-slice launch of patch_2x2
-# (profiles/bp_patch_fbp512_ncu.txt): the slice quads read once and the images
-# written, both proportional to the slices, so a launch of B slices moves B/64 of it
-BP_DRAM_BYTES_PER_SLICE = 336e6 / 64
+# (profiles/bp_patch_fbp512_ncu.txt): the slice quads (268 MB, twice L2, read 6 times
+# over by the tiles) and the images, proportional to the slices, so a launch of B
+# slices moves B/64 of it
+BP_DRAM_BYTES_PER_SLICE = 1756e6 / 64
 WORKLOAD_NAME = ("full-rate streaming: 2 planes x 2000 frames of 1000x1152 uint16 fan sinograms, 1% defective "
                  "detectors -> 1024x1024 parallel (pad 2048, Shepp-Logan) -> 512^2 FP32, circular mask")
 
