@@ -287,10 +287,13 @@ struct risa_gb_backprojection {
       RG_CUDA(cudaDeviceSynchronize());
       return pairs.alloc(need);
    }
-   int variant_for(int batch, bool fused_mask) const {
+   int variant_for(const BPCfg& c, const float* sino, int batch) const {
       const int v = variant == kAutoVariant ? bp_patch_variant() : variant;
-      if (v == bp_patch_variant() && patch.angles.empty()) return 0;  // outside its range of angles or bins per pixel
-      return bp_pairs_bytes(v, batch, g.Pp, g.Dp, win_len[fused_mask ? 1 : 0]) > pairs.bytes ? 0 : v;
+      if (v == bp_patch_variant()) {
+         if (patch.angles.empty()) return 0;  // outside its range of angles or bins per pixel
+         if (bp_patch_rows_ok(c, sino, batch)) return v;  // stages no rows
+      }
+      return bp_pairs_bytes(v, batch, g.Pp, g.Dp, c.win_len) > c.pairs_bytes ? 0 : v;
    }
 };
 
@@ -852,8 +855,8 @@ risa_gb_status risa_gb_backprojection_create(const risa_gb_geometry* gi, const r
 
 static risa_gb_status bp_run(risa_gb_backprojection* h, const float* sino, float* img, int batch,
                              bool fused_mask, void* stream) {
-   RG_CUDA(launch_backprojection(sino, img, batch, h->cfg(fused_mask), h->variant_for(batch, fused_mask),
-                                 S(stream)));
+   const BPCfg c = h->cfg(fused_mask);
+   RG_CUDA(launch_backprojection(sino, img, batch, c, h->variant_for(c, sino, batch), S(stream)));
    return RISA_GB_OK;
 }
 
@@ -871,7 +874,7 @@ risa_gb_status risa_gb_backprojection_time(risa_gb_backprojection* h, const floa
       BPCfg c = h->cfg(fused);
       c.mid_event = ev[1];
       cudaError_t e = cudaEventRecord(ev[0], st);
-      if (e == cudaSuccess) e = launch_backprojection(sino, img, batch, c, h->variant_for(batch, fused), st);
+      if (e == cudaSuccess) e = launch_backprojection(sino, img, batch, c, h->variant_for(c, sino, batch), st);
       if (e == cudaSuccess) e = cudaEventRecord(ev[2], st);
       if (e == cudaSuccess) e = cudaEventSynchronize(ev[2]);
       float a = 0.f, b = 0.f;
@@ -1093,8 +1096,8 @@ static AttenuationCfg engine_atten_cfg(const risa_gb_fbp* h, int plane) {
 static cudaError_t engine_filter_bp(risa_gb_fbp* h, float* par, float* img, int batch, bool fused, cudaStream_t st,
                                     cudaEvent_t ev_filtered, cudaEvent_t ev_staged) {
    const FilterCfg fc = h->filt->cfg();
-   const int v = h->bp->variant_for(batch, fused);
    BPCfg c = h->bp->cfg(fused);
+   const int v = h->bp->variant_for(c, par, batch);
    cudaError_t e;
    const bool rows = v == bp_patch_variant() && bp_patch_rows_ok(c, par, batch);
    if (!rows && bp_variant_layout(v) != kLayoutNone && filter_pairs_supported(fc)) {
@@ -1135,8 +1138,9 @@ static cudaError_t engine_streaming(risa_gb_fbp* h, const uint16_t* raw, int pla
 static bool two_lanes(const risa_gb_fbp* h, int batch) {
    if (h->lanes < 2 || h->p.normalize || h->p.interp != RISA_GB_INTERP_LINEAR) return false;
    const bool fused = h->p.masking && !h->p.normalize;
-   const int v = h->bp->variant_for(batch, fused);
-   if (v == bp_patch_variant() && bp_patch_rows_ok(h->bp->cfg(fused), h->par.as<float>(), batch)) return false;
+   const BPCfg c = h->bp->cfg(fused);
+   const int v = h->bp->variant_for(c, h->par.as<float>(), batch);
+   if (v == bp_patch_variant() && bp_patch_rows_ok(c, h->par.as<float>(), batch)) return false;
    return bp_variant_layout(v) != kLayoutNone && filter_pairs_supported(h->filt->cfg());
 }
 
@@ -1168,8 +1172,8 @@ static cudaError_t engine_lane_prefix(risa_gb_fbp* h, const uint16_t* raw, int p
    cudaError_t e = engine_streaming(h, raw, plane, batch, st);
    if (e != cudaSuccess) return e;
    const bool fused = h->p.masking && !h->p.normalize;
-   const int v = h->bp->variant_for(batch, fused);
    const BPCfg c = h->bp->cfg(fused);
+   const int v = h->bp->variant_for(c, h->par.as<float>(), batch);
    return launch_filter_pairs(h->par.as<float>(), batch, h->filt->cfg(),
                               PairsOut{pairs, bp_variant_pair_slices(v), c.win_lo, c.win_len}, st);
 }
@@ -1178,8 +1182,8 @@ static cudaError_t engine_lane_prefix(risa_gb_fbp* h, const uint16_t* raw, int p
 // pair buffers hold at least the backprojection's reservation).
 static cudaError_t engine_lane_bp(risa_gb_fbp* h, float* img, int batch, void* pairs, cudaStream_t st) {
    const bool fused = h->p.masking && !h->p.normalize;
-   const int v = h->bp->variant_for(batch, fused);
    BPCfg c = h->bp->cfg(fused);
+   const int v = h->bp->variant_for(c, h->par.as<float>(), batch);
    c.pairs = pairs;
    c.prefilled = true;
    return launch_backprojection(h->par.as<float>(), img, batch, c, v, st);
