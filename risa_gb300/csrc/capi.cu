@@ -279,13 +279,20 @@ struct risa_gb_backprojection {
    // that the calls of one handle give the same bits however a job is cut.
    int reserved_batch = 0;
    risa_gb_status reserve(int batch) {
-      reserved_batch = std::max(reserved_batch, batch);
       size_t need = 0;
       for (int v = 0; v < bp_variant_count(); ++v)
          need = std::max(need, bp_pairs_bytes(v, batch, g.Pp, g.Dp, std::max(win_len[0], win_len[1])));
-      if (need <= pairs.bytes) return RISA_GB_OK;
-      RG_CUDA(cudaDeviceSynchronize());
-      return pairs.alloc(need);
+      if (need > pairs.bytes) {
+         RG_CUDA(cudaDeviceSynchronize());
+         const size_t had = pairs.bytes;
+         const risa_gb_status s = pairs.alloc(need);  // gives the present buffer back first
+         if (s != RISA_GB_OK) {
+            if (had > 0) pairs.alloc(had);
+            return s;
+         }
+      }
+      reserved_batch = std::max(reserved_batch, batch);
+      return RISA_GB_OK;
    }
    int variant_for(const BPCfg& c, const float* sino, int batch) const {
       const int v = variant == kAutoVariant ? bp_patch_variant() : variant;

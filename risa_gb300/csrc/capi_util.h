@@ -42,6 +42,7 @@ struct DevBuf {
       if (n == 0) return RISA_GB_OK;
       cudaError_t e = cudaMalloc(&p, n);
       if (e != cudaSuccess) {
+         cudaGetLastError();  // returned here, not by the next launch's check
          p = nullptr;
          return fail(RISA_GB_ENOMEM, std::string("cudaMalloc(") + std::to_string(n) + "): " + cudaGetErrorString(e));
       }
