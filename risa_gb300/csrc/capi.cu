@@ -847,14 +847,15 @@ risa_gb_status risa_gb_backprojection_create(const risa_gb_geometry* gi, const r
          std::vector<BPPatchAngle> all = h->patch.angles;
          all.insert(all.end(), h->patch.sym_angles.begin(), h->patch.sym_angles.end());
          RG_TRY(h->patch_angles.upload(all));
-         const size_t part = bp_part_bytes(2, h->g.N);  // single frames (8 MB at 512^2)
-         if (!h->patch.sym_angles.empty() && part <= ((size_t)64 << 20)) RG_TRY(h->part.alloc(part));
       }
-      // frame-by-frame callers need no reserve(): one slice quad (16 MB at 1024 x 1024)
-      const size_t quad = bp_quads_bytes(4, h->g.Pp, h->g.Dp);
-      if (!h->patch.angles.empty() && quad <= ((size_t)64 << 20)) RG_TRY(h->pairs.alloc(quad));
       RG_TRY(h->rowbase.upload(bp_line_starts(t.t0.data(), t.bd.data(), h->g.Pp, h->g.N)));
       RG_TRY(h->colbase.upload(bp_line_starts(t.t0.data(), t.ad.data(), h->g.Pp, h->g.N)));
+      // The patch kernels' buffers for callers that make no reservation, up to 64 MB each:
+      // two slices' partial images (8 MB at 512^2), one slice quad (16 MB at
+      // 1024 x 1024). A handle that cannot have them takes the forms that need none.
+      const size_t part = bp_part_bytes(2, h->g.N), quad = bp_quads_bytes(4, h->g.Pp, h->g.Dp);
+      if (!h->patch.sym_angles.empty() && part <= ((size_t)64 << 20)) h->part.alloc(part);
+      if (!h->patch.angles.empty() && quad <= ((size_t)64 << 20)) h->pairs.alloc(quad);
    }
    *out = h.release();
    return RISA_GB_OK;
@@ -1084,6 +1085,7 @@ risa_gb_status risa_gb_fbp_create(const risa_gb_geometry* gi, const risa_gb_para
       RG_TRY(h->dws.alloc(defects_workspace_bytes(h->defects->cfg.D, max_batch, h->defects->cfg.max_runs, true)));
    RG_TRY(h->mm.alloc(sizeof(unsigned int) * 2 * (size_t)max_batch));
    if (h->p.interp == RISA_GB_INTERP_LINEAR) RG_TRY(h->bp->reserve(max_batch));
+   if (max_batch > 2) h->bp->part.release();  // for handles of one or two slices
    *out = h.release();
    return RISA_GB_OK;
 }

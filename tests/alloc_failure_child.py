@@ -69,6 +69,23 @@ def reserve():
         np.testing.assert_array_equal(backproject(bp, sino), before, err_msg=f"{first} {n}")
 
 
+def create():
+    """A new handle does without its optional buffers (here 4 MB of partial images and
+    2 MB of staged rows; its tables are below 1.5 MB each)."""
+    pp, dp, n_pix = 512, 256, 360
+    with Refused(2 << 20):
+        bp = handle(pp, dp, n_pix)
+    plenty = handle(pp, dp, n_pix)
+    for n in (1, 2, 3, 5):
+        sino = sinograms(n, pp, dp)
+        got, exp = backproject(bp, sino, n_pix), backproject(plenty, sino, n_pix)
+        assert np.abs(got - exp).max() < 1e-5 * np.abs(exp).max(), n
+    bp.reserve(8)
+    plenty.reserve(8)
+    sino = sinograms(8, pp, dp)
+    np.testing.assert_array_equal(backproject(bp, sino, n_pix), backproject(plenty, sino, n_pix))
+
+
 def main():
     rt.RT = rt.cudart()
     rt.ck(rt.RT.cudaSetDevice(0), "cudaSetDevice")
