@@ -351,7 +351,7 @@ __device__ __forceinline__ bool sweep_tile(const SweepArgs& A, const SweepInst& 
       for (int r = 0; r < PPT; ++r) {
          const int x = x0 + xo, y = y0 + yo + RS * r;
          if (SYM && x < N && y < N) {
-            float* part = A.part + 4 * I.img_off;
+            float* part = A.part + I.part_off;
             const size_t plane = (size_t)N * N;
             part[(size_t)y * N + x] = acc[0][r];
             part[plane + (size_t)y * N + (N - 1 - x)] = acc[R > 1 ? 1 : 0][r];
@@ -397,7 +397,7 @@ __device__ __forceinline__ bool sweep_sum(const SweepArgs& A, const SweepInst& I
    const int N = I.N;
    const size_t plane = (size_t)N * N;
    const float c = 0.5f * (float)(N - 1), lim = (float)N * (float)N * 0.25f;
-   const float* part = A.part + 4 * I.img_off;
+   const float* part = A.part + I.part_off;
    const float2* prow = A.pairs + I.pair_off;
    const size_t end = min(plane, (size_t)(index + 1) * I.combine_px);
    for (size_t at = (size_t)index * I.combine_px + threadIdx.x; at < end; at += kNT) {

@@ -50,6 +50,7 @@ struct SweepInst {
    float norm, mask_value;
    float dark, logden;          // flat field: dark level, log(max(ref - dark, 1e-5))
    size_t raw_off, img_off, pair_off;  // element offsets: uint16, float, float2 (pair_off even)
+   size_t part_off;                    // of the partial images (n_base > 0)
    const float* a;              // [Pp] per-angle ray-coordinate steps (FP32)
    const float* b;
    const double* ad;            // [Pp] FP64 copies and the offset of the tile origin
@@ -73,7 +74,7 @@ struct SweepArgs {
    int n_items;
    const uint16_t* raw;
    float* img;
-   float* part;                   // partial images, [4][N][N] at 4 img_off
+   float* part;                   // partial images, [4][N][N] at part_off
    float2* pairs;
    const float2* twp[4];          // radix-16 pass twiddles for len 512, 1024, 2048, 4096
    int* next;                     // work counter, zero at launch
@@ -99,6 +100,9 @@ constexpr int kSweepACH = 64;
 // sets, 779 with; 24 of up to 1024^2 (5215) 1167 and 1140; 64 of up to 1024^2
 // (13 thousand) 4.58 and 4.16 ms.
 constexpr int kSweepManyTiles = 2000, kSweepSetTiles = 5000;
+// Partial images that a sweep keeps at most (four times the images: 256 instances of
+// up to 1024^2 take 0.9 GB); the instances after that take their angles singly.
+constexpr size_t kSweepPartBytes = (size_t)4 << 30;
 
 // Staged window length (bins, even) for a given bins-per-pixel scale.
 int sweep_window_len(float scale);

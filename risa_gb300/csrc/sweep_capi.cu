@@ -76,12 +76,7 @@ bool any_flag(const uint8_t* flags, int D) {
 
 }  // namespace
 
-extern "C" {
-
-risa_gb_status risa_gb_sweep_create(const risa_gb_sweep_instance* in, int n, risa_gb_sweep** out) {
-   if (!out) return fail(RISA_GB_EINVAL, "out is NULL");
-   *out = nullptr;
-   if (!in || n < 1) return fail(RISA_GB_EINVAL, "sweep needs at least one instance");
+static risa_gb_status sweep_create(const risa_gb_sweep_instance* in, int n, bool allow_sets, risa_gb_sweep** out) {
    std::unique_ptr<risa_gb_sweep> h(new (std::nothrow) risa_gb_sweep());
    if (!h) return fail(RISA_GB_ENOMEM, "host allocation failed");
    h->n = n;
@@ -94,13 +89,13 @@ risa_gb_status risa_gb_sweep_create(const risa_gb_sweep_instance* in, int n, ris
    std::vector<SweepRepair> reps;
    std::vector<size_t> o_f32(n), o_f64(n), o_h(n), o_rep(n, (size_t)-1), o_win(n, (size_t)-1);
    std::vector<int2> win;
-   size_t n_tiles = 0;
+   size_t n_tiles = 0, part_total = 0;
    for (int i = 0; i < n; ++i) {
       const size_t t = in[i].n_pixels > 0 ? ((size_t)in[i].n_pixels + 31) / 32 : 0;
       n_tiles += t * t;
    }
    h->n_tiles = (int)std::min<size_t>(n_tiles, 1u << 30);
-   const bool sets = h->n_tiles >= kSweepSetTiles;
+   const bool sets = allow_sets && h->n_tiles >= kSweepSetTiles;
    for (int i = 0; i < n; ++i) {
       const risa_gb_sweep_instance& s = in[i];
       if (s.n_pixels < 16 || s.n_par_proj < 1 || s.n_par_det < 2 || s.n_par_det > 65535 ||
@@ -154,7 +149,11 @@ risa_gb_status risa_gb_sweep_create(const risa_gb_sweep_instance* in, int n, ris
       h->img_total += (size_t)g.N * g.N;
       h->pair_total += (size_t)g.Pp * I.win_len;
       I.n_base = I.combine_items = I.combine_px = I.n_extra = 0;
-      if (sets && g.rotation_offset == 0.0 && g.Pp % 2 == 0 && g.Pp >= 8) {
+      I.part_off = part_total;
+      const size_t part = 4 * (size_t)g.N * g.N;
+      if (sets && g.rotation_offset == 0.0 && g.Pp % 2 == 0 && g.Pp >= 8 &&
+          sizeof(float) * (part_total + part) <= kSweepPartBytes) {
+         part_total += part;
          I.n_base = (g.Pp - 1) / 4;  // 0 < i < Pp / 4
          I.extra[I.n_extra++] = 0;
          I.extra[I.n_extra++] = g.Pp / 2;
@@ -232,9 +231,7 @@ risa_gb_status risa_gb_sweep_create(const risa_gb_sweep_instance* in, int n, ris
    h->n_items = (int)items.size();
    RG_TRY(h->d_items.upload(items));
    RG_TRY(h->d_pairs.alloc(sizeof(float2) * h->pair_total));
-   bool any_sums = false;
-   for (const SweepInst& I : h->inst) any_sums = any_sums || I.n_base > 0;
-   if (any_sums) RG_TRY(h->d_part.alloc(sizeof(float) * 4 * h->img_total));
+   RG_TRY(h->d_part.alloc(sizeof(float) * part_total));
    const int lens[4] = {512, 1024, 2048, 4096};
    for (int k = 0; k < 4; ++k) RG_TRY(h->d_twp[k].upload(filter_pass_twiddles(lens[k])));
    RG_TRY(h->d_cnt.alloc(sizeof(int) * (2 + 3 * (size_t)n)));
@@ -242,6 +239,17 @@ risa_gb_status risa_gb_sweep_create(const risa_gb_sweep_instance* in, int n, ris
    RG_CUDA(cudaMemset(h->d_cnt.p, 0, h->d_cnt.bytes));
    *out = h.release();
    return RISA_GB_OK;
+}
+
+extern "C" {
+
+risa_gb_status risa_gb_sweep_create(const risa_gb_sweep_instance* in, int n, risa_gb_sweep** out) {
+   if (!out) return fail(RISA_GB_EINVAL, "out is NULL");
+   *out = nullptr;
+   if (!in || n < 1) return fail(RISA_GB_EINVAL, "sweep needs at least one instance");
+   const risa_gb_status s = sweep_create(in, n, true, out);
+   // without symmetric sets where their partial images cannot be had
+   return s == RISA_GB_ENOMEM ? sweep_create(in, n, false, out) : s;
 }
 
 risa_gb_status risa_gb_sweep_layout(const risa_gb_sweep* h, size_t* raw_offsets, size_t* img_offsets,

@@ -86,6 +86,26 @@ def create():
     np.testing.assert_array_equal(backproject(bp, sino, n_pix), backproject(plenty, sino, n_pix))
 
 
+def sweep():
+    """A large sweep does without the partial images of its symmetric sets (80 MB here)."""
+    inst = [dict(n_pixels=1024, n_par_proj=pp, n_par_det=160, filter_type="ramp", ref_level=40200.0, dark_level=200.0,
+                 masking=True) for pp in (8, 10, 12, 8, 9)]
+    out = []
+    for refuse in (True, False):
+        if refuse:
+            with Refused(64 << 20):
+                sw = rg.Sweep(inst)
+        else:
+            sw = rg.Sweep(inst)
+        raw_total, img_total = sw.layout()[2:]
+        raw = np.random.default_rng(3).integers(300, 40000, raw_total).astype(np.uint16)
+        d, img = rt.upload(raw), rt.upload(np.full(img_total, np.nan, np.float32))
+        sw.enqueue(d, img)
+        sw.check()
+        out.append(rt.download(img, (img_total,), np.float32))
+    assert np.abs(out[0] - out[1]).max() < 1e-5 * np.abs(out[1]).max()
+
+
 def main():
     rt.RT = rt.cudart()
     rt.ck(rt.RT.cudaSetDevice(0), "cudaSetDevice")

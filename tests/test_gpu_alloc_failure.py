@@ -45,7 +45,7 @@ def fake(tmp_path_factory):
     return str(so)
 
 
-@pytest.mark.parametrize("what", ["reserve", "create"])
+@pytest.mark.parametrize("what", ["reserve", "create", "sweep"])
 def test_refused_allocation(fake, what):
     env = dict(os.environ, LD_PRELOAD=fake)
     res = subprocess.run([sys.executable, os.path.join(HERE, "alloc_failure_child.py"), what, fake],
