@@ -298,7 +298,14 @@ risa_gb_status risa_gb_filter_design_host(const risa_gb_geometry* g, const risa_
 typedef struct risa_gb_backprojection risa_gb_backprojection;
 risa_gb_status risa_gb_backprojection_create(const risa_gb_geometry* g, const risa_gb_params* p,
                                              risa_gb_backprojection** out);
-/* sino: [batch][Pp][Dp] float -> img: [batch][N][N] float. */
+/* sino: [batch][Pp][Dp] float -> img: [batch][N][N] float.
+ * A call that the program captures into a graph of its own takes a kernel that
+ * holds none of the handle's buffers (its sums may round differently from those of a
+ * direct call): the graph may be replayed on any stream while the handle lives, and
+ * stays valid after reserve. After set_variant or autotune a captured call
+ * runs that variant: with a staged one (patch_2x2, staged_*) the graph uses the
+ * handle's buffers, so do not replay it beside other calls of the handle, and
+ * capture again after reserve or autotune. */
 risa_gb_status risa_gb_backprojection_enqueue(risa_gb_backprojection* h, const float* sino,
                                               float* img, int batch, void* stream);
 /* Adjoint: img [batch][N][N] -> sino [batch][Pp][Dp] (ray-driven forward projector,

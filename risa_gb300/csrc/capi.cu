@@ -241,7 +241,8 @@ struct risa_gb_backprojection {
    BPPatchPlan patch;        // the patch variant's angle order
    DevBuf patch_angles, part;
    std::vector<float> a_host, b_host;  // the staged variants' kernel-parameter copies of a and b
-   BPCfg cfg(bool fused_mask) const {
+   // scratch: whether the call may use the handle's buffers (pairs, part)
+   BPCfg cfg(bool fused_mask, bool scratch = true) const {
       BPCfg c;
       c.Pp = g.Pp; c.Dp = g.Dp; c.N = g.N;
       c.a = a.as<float>(); c.b = b.as<float>(); c.t0 = t0.as<double>();
@@ -255,8 +256,8 @@ struct risa_gb_backprojection {
       // t' = t + shift; the texture variant truncates t + Dp/2
       const double shift = p.quirks == RISA_GB_QUIRKS_RISA ? (double)(int)(g.Dp * 0.5) : g.Dp * 0.5 - 0.5;
       c.trunc_offset = (float)(g.Dp * 0.5 - shift);
-      c.pairs = pairs.p;
-      c.pairs_bytes = pairs.bytes;
+      c.pairs = scratch ? pairs.p : nullptr;
+      c.pairs_bytes = scratch ? pairs.bytes : 0;
       c.win_lo = win_lo[fused_mask ? 1 : 0];
       c.win_len = win_len[fused_mask ? 1 : 0];
       c.err = err.as<int>();
@@ -265,7 +266,7 @@ struct risa_gb_backprojection {
       c.tile_win = tile_win.as<int2>();
       c.patch = &patch;
       c.few = reserved_batch <= 2;
-      c.part = part.as<float>();
+      c.part = scratch ? part.as<float>() : nullptr;
       c.patch_angles = patch_angles.as<BPPatchAngle>();
       c.adj_scratch = adj.p;
       c.adj_scratch_bytes = adj.bytes;
@@ -863,7 +864,13 @@ risa_gb_status risa_gb_backprojection_create(const risa_gb_geometry* gi, const r
 
 static risa_gb_status bp_run(risa_gb_backprojection* h, const float* sino, float* img, int batch,
                              bool fused_mask, void* stream) {
-   const BPCfg c = h->cfg(fused_mask);
+   // A graph that a program captures is replayed on any stream and may outlive a
+   // reservation, so unless a variant was chosen (set_variant, autotune) a
+   // captured call takes the forms that hold none of the handle's buffers.
+   cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+   if (h->variant == kAutoVariant && h->p.interp == RISA_GB_INTERP_LINEAR)
+      RG_CUDA(cudaStreamIsCapturing(S(stream), &capture));
+   const BPCfg c = h->cfg(fused_mask, capture == cudaStreamCaptureStatusNone);
    RG_CUDA(launch_backprojection(sino, img, batch, c, h->variant_for(c, sino, batch), S(stream)));
    return RISA_GB_OK;
 }

@@ -2,7 +2,9 @@
 import numpy as np
 import pytest
 
+import oracle
 import risa_gb300 as rg
+from tests.helpers import rel_err
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -43,3 +45,67 @@ def test_single_frames_need_no_staged_rows(n):
     reserved = _handle(Pp, Dp, N)
     reserved.reserve(2)
     np.testing.assert_array_equal(_run(_handle(Pp, Dp, N), sino, N), _run(reserved, sino, N))
+
+
+def _capture(bp, sino, img, stream):
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        bp.enqueue(sino, img, sino.shape[0], stream)
+    return graph
+
+
+def _images(n, N):
+    return torch.full((n, N, N), float("nan"), dtype=torch.float32, device="cuda")
+
+
+@pytest.mark.parametrize("reserved", [0, 2, 8])
+@pytest.mark.parametrize("n", [1, 2, 4, 8])
+def test_captured_enqueue_outlives_a_reservation(n, reserved):
+    Pp, Dp, N = 64, 128, 128
+    bp = _handle(Pp, Dp, N)
+    if reserved:
+        bp.reserve(reserved)
+    sino, img = _sino(n, Pp, Dp, n), _images(n, N)
+    exp = [oracle.mask(oracle.backproject(s, N), 0.0) for s in sino.cpu().numpy()]
+    graph = _capture(bp, sino, img, torch.cuda.Stream())
+    bp.reserve(64)  # the staged rows move
+    many = _sino(64, Pp, Dp, 5)
+    other = _run(bp, many, N)
+    for _ in range(2):
+        img.fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        for b in range(n):
+            mr, _ = rel_err(img[b].cpu().numpy(), exp[b])
+            assert mr < MAX_REL, (b, mr)
+        np.testing.assert_array_equal(_run(bp, many, N), other)
+
+
+@pytest.mark.parametrize("n", [1, 4])
+def test_captured_enqueue_beside_other_calls(n):
+    """Replays on one stream, calls of the same handle on another: the bits of each alone."""
+    Pp, Dp, N = 180, 256, 256
+    bp = _handle(Pp, Dp, N)
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    sino, img = _sino(n, Pp, Dp, 1), _images(n, N)
+    graph = _capture(bp, sino, img, a)
+    with torch.cuda.stream(a):
+        graph.replay()
+    torch.cuda.synchronize()
+    alone = img.cpu().numpy()
+    sino2, img2 = _sino(n, Pp, Dp, 2), _images(n, N)
+    alone2 = _run(bp, sino2, N)
+    for _ in range(20):
+        img.fill_(float("nan"))
+        img2.fill_(float("nan"))
+        torch.cuda.synchronize()
+        with torch.cuda.stream(a):
+            graph.replay()
+        bp.enqueue(sino2, img2, n, b)
+        with torch.cuda.stream(a):
+            graph.replay()
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(img.cpu().numpy(), alone)
+        np.testing.assert_array_equal(img2.cpu().numpy(), alone2)
+    bp.check()
