@@ -298,7 +298,9 @@ risa_gb_status risa_gb_filter_design_host(const risa_gb_geometry* g, const risa_
 typedef struct risa_gb_backprojection risa_gb_backprojection;
 risa_gb_status risa_gb_backprojection_create(const risa_gb_geometry* g, const risa_gb_params* p,
                                              risa_gb_backprojection** out);
-/* sino: [batch][Pp][Dp] float -> img: [batch][N][N] float.
+/* sino: [batch][Pp][Dp] float -> img: [batch][N][N] float. Any number of threads
+ * and streams may enqueue on one handle: calls that use its buffers run one after the
+ * other on the device.
  * A call that the program captures into a graph of its own takes a kernel that
  * holds none of the handle's buffers (its sums may round differently from those of a
  * direct call): the graph may be replayed on any stream while the handle lives, and

@@ -14,6 +14,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -224,6 +225,45 @@ std::vector<float> twiddles(int len) {
 // Before set_variant or autotune: the patch kernel where it covers the geometry.
 constexpr int kAutoVariant = -1;
 
+// Orders the calls that use a handle's buffers, whatever threads and streams
+// they come from: one thread at a time launches, and a call on another stream
+// than the last one's first waits for the event recorded after that.
+struct BufferOrder {
+   std::mutex lock;
+   cudaEvent_t done = nullptr;     // after the last use
+   unsigned long long stream = 0;  // where that was
+   bool used = false;
+   ~BufferOrder() {
+      if (done) cudaEventDestroy(done);
+   }
+};
+class BufferUse {
+  public:
+   explicit BufferUse(BufferOrder& o) : o_(o), hold_(o.lock) {}
+   // Before the call's first launch on `st`; the destructor follows its last one.
+   cudaError_t begin(cudaStream_t st) {
+      cudaError_t e = cudaSuccess;
+      if (!o_.done && (e = cudaEventCreateWithFlags(&o_.done, cudaEventDisableTiming)) != cudaSuccess) return e;
+      if ((e = cudaStreamGetId(st, &id_)) != cudaSuccess) return e;
+      if (o_.used && id_ != o_.stream && (e = cudaStreamWaitEvent(st, o_.done, 0)) != cudaSuccess) return e;
+      st_ = st;
+      begun_ = true;
+      return e;
+   }
+   ~BufferUse() {
+      if (!begun_ || cudaEventRecord(o_.done, st_) != cudaSuccess) return;
+      o_.used = true;
+      o_.stream = id_;
+   }
+
+  private:
+   BufferOrder& o_;
+   std::lock_guard<std::mutex> hold_;
+   bool begun_ = false;
+   cudaStream_t st_ = nullptr;
+   unsigned long long id_ = 0;
+};
+
 struct risa_gb_backprojection {
    Geometry g;
    Params p;
@@ -240,6 +280,7 @@ struct risa_gb_backprojection {
    DevBuf tile_win;          // staged variants: window start + origin per tile and angle
    BPPatchPlan patch;        // the patch variant's angle order
    DevBuf patch_angles, part;
+   BufferOrder order;        // of the calls that use pairs or part
    std::vector<float> a_host, b_host;  // the staged variants' kernel-parameter copies of a and b
    // scratch: whether the call may use the handle's buffers (pairs, part)
    BPCfg cfg(bool fused_mask, bool scratch = true) const {
@@ -283,6 +324,7 @@ struct risa_gb_backprojection {
       size_t need = 0;
       for (int v = 0; v < bp_variant_count(); ++v)
          need = std::max(need, bp_pairs_bytes(v, batch, g.Pp, g.Dp, std::max(win_len[0], win_len[1])));
+      std::lock_guard<std::mutex> hold(order.lock);
       if (need > pairs.bytes) {
          RG_CUDA(cudaDeviceSynchronize());
          const size_t had = pairs.bytes;
@@ -302,6 +344,10 @@ struct risa_gb_backprojection {
          if (bp_patch_rows_ok(c, sino, batch)) return v;  // stages no rows
       }
       return bp_pairs_bytes(v, batch, g.Pp, g.Dp, c.win_len) > c.pairs_bytes ? 0 : v;
+   }
+   bool uses_buffers(int v, const BPCfg& c, const float* sino, int batch) const {
+      if (v == bp_patch_variant() && bp_patch_rows_ok(c, sino, batch)) return c.part && !patch.sym_angles.empty();
+      return p.interp == RISA_GB_INTERP_LINEAR && bp_variant_layout(v) != kLayoutNone;
    }
 };
 
@@ -868,10 +914,13 @@ static risa_gb_status bp_run(risa_gb_backprojection* h, const float* sino, float
    // reservation, so unless a variant was chosen (set_variant, autotune) a
    // captured call takes the forms that hold none of the handle's buffers.
    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-   if (h->variant == kAutoVariant && h->p.interp == RISA_GB_INTERP_LINEAR)
-      RG_CUDA(cudaStreamIsCapturing(S(stream), &capture));
-   const BPCfg c = h->cfg(fused_mask, capture == cudaStreamCaptureStatusNone);
-   RG_CUDA(launch_backprojection(sino, img, batch, c, h->variant_for(c, sino, batch), S(stream)));
+   if (h->p.interp == RISA_GB_INTERP_LINEAR) RG_CUDA(cudaStreamIsCapturing(S(stream), &capture));
+   const bool direct = capture == cudaStreamCaptureStatusNone;
+   BufferUse use(h->order);
+   const BPCfg c = h->cfg(fused_mask, direct || h->variant != kAutoVariant);
+   const int v = h->variant_for(c, sino, batch);
+   if (direct && h->uses_buffers(v, c, sino, batch)) RG_CUDA(use.begin(S(stream)));
+   RG_CUDA(launch_backprojection(sino, img, batch, c, v, S(stream)));
    return RISA_GB_OK;
 }
 
@@ -886,9 +935,11 @@ risa_gb_status risa_gb_backprojection_time(risa_gb_backprojection* h, const floa
    float sum_stage = 0.f, sum_kernel = 0.f;
    risa_gb_status rc = RISA_GB_OK;
    for (int r = 0; r < reps && rc == RISA_GB_OK; ++r) {
+      BufferUse use(h->order);
       BPCfg c = h->cfg(fused);
       c.mid_event = ev[1];
-      cudaError_t e = cudaEventRecord(ev[0], st);
+      cudaError_t e = use.begin(st);
+      if (e == cudaSuccess) e = cudaEventRecord(ev[0], st);
       if (e == cudaSuccess) e = launch_backprojection(sino, img, batch, c, h->variant_for(c, sino, batch), st);
       if (e == cudaSuccess) e = cudaEventRecord(ev[2], st);
       if (e == cudaSuccess) e = cudaEventSynchronize(ev[2]);

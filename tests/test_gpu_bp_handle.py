@@ -1,4 +1,6 @@
 """A backprojection handle's own buffers, and the kernels that do without them."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -109,3 +111,43 @@ def test_captured_enqueue_beside_other_calls(n):
         np.testing.assert_array_equal(img.cpu().numpy(), alone)
         np.testing.assert_array_equal(img2.cpu().numpy(), alone2)
     bp.check()
+
+
+@pytest.mark.parametrize("threads", [False, True])
+@pytest.mark.parametrize("n,reserved,aligned", [(1, 0, True), (2, 0, True), (2, 0, False), (4, 0, True), (6, 0, True),
+                                                (1, 2, True), (16, 16, True)])
+def test_two_streams(n, reserved, aligned, threads):
+    """Two streams, from one host thread and from two: the bits of each call alone."""
+    Pp, Dp, N = 180, 256, 256
+    bp = _handle(Pp, Dp, N)
+    if reserved:
+        bp.reserve(reserved)
+    sinos = []
+    for seed in (1, 2):
+        t = torch.empty(n * Pp * Dp + 1, dtype=torch.float32, device="cuda")[0 if aligned else 1:][:n * Pp * Dp]
+        t = t.view(n, Pp, Dp)
+        t.copy_(_sino(n, Pp, Dp, seed))
+        sinos.append(t)
+    alone = [_run(bp, s, N) for s in sinos]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    imgs = [[_images(n, N) for _ in range(12)] for _ in sinos]
+    torch.cuda.synchronize()
+
+    def calls(i):
+        for img in imgs[i]:
+            bp.enqueue(sinos[i], img, n, streams[i])
+
+    if threads:
+        work = [threading.Thread(target=calls, args=(i,)) for i in range(2)]
+        for w in work:
+            w.start()
+        for w in work:
+            w.join()
+    else:
+        for a, b in zip(*imgs):
+            bp.enqueue(sinos[0], a, n, streams[0])
+            bp.enqueue(sinos[1], b, n, streams[1])
+    bp.check()
+    for i in range(2):
+        for img in imgs[i]:
+            np.testing.assert_array_equal(img.cpu().numpy(), alone[i])
