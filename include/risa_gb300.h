@@ -430,6 +430,9 @@ risa_gb_status risa_gb_fbp_intermediates(risa_gb_fbp* h, float** fan, float** pa
  * filter writes its rows itself). Synchronises. */
 risa_gb_status risa_gb_fbp_time_stages(risa_gb_fbp* h, const uint16_t* raw, float* img, int plane, int batch,
                                        int reps, void* stream, float* ms);
+/* The engine's backprojection, for autotune, set_variant and the measurements. Its
+ * enqueue may run beside the engine's own runs unless a staged variant was chosen,
+ * whose buffers both then use. */
 risa_gb_backprojection* risa_gb_fbp_backprojection(risa_gb_fbp* h);
 risa_gb_status risa_gb_fbp_destroy(risa_gb_fbp* h);
 

@@ -281,6 +281,7 @@ struct risa_gb_backprojection {
    BPPatchPlan patch;        // the patch variant's angle order
    DevBuf patch_angles, part;
    BufferOrder order;        // of the calls that use pairs or part
+   bool engine = false;      // an engine's, whose runs and graphs use them
    std::vector<float> a_host, b_host;  // the staged variants' kernel-parameter copies of a and b
    // scratch: whether the call may use the handle's buffers (pairs, part)
    BPCfg cfg(bool fused_mask, bool scratch = true) const {
@@ -911,13 +912,14 @@ risa_gb_status risa_gb_backprojection_create(const risa_gb_geometry* gi, const r
 static risa_gb_status bp_run(risa_gb_backprojection* h, const float* sino, float* img, int batch,
                              bool fused_mask, void* stream) {
    // A graph that a program captures is replayed on any stream and may outlive a
-   // reservation, so unless a variant was chosen (set_variant, autotune) a
-   // captured call takes the forms that hold none of the handle's buffers.
+   // reservation, and an engine's graphs use the buffers of its handle at any time.
+   // So unless a variant was chosen (set_variant, autotune) captured calls, and all
+   // calls of an engine's handle, take the forms that hold none of the buffers.
    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
    if (h->p.interp == RISA_GB_INTERP_LINEAR) RG_CUDA(cudaStreamIsCapturing(S(stream), &capture));
    const bool direct = capture == cudaStreamCaptureStatusNone;
    BufferUse use(h->order);
-   const BPCfg c = h->cfg(fused_mask, direct || h->variant != kAutoVariant);
+   const BPCfg c = h->cfg(fused_mask, (direct && !h->engine) || h->variant != kAutoVariant);
    const int v = h->variant_for(c, sino, batch);
    if (direct && h->uses_buffers(v, c, sino, batch)) RG_CUDA(use.begin(S(stream)));
    RG_CUDA(launch_backprojection(sino, img, batch, c, v, S(stream)));
@@ -1132,6 +1134,7 @@ risa_gb_status risa_gb_fbp_create(const risa_gb_geometry* gi, const risa_gb_para
    RG_TRY(prepare_f2p_staged(h->f2p));
    RG_TRY(risa_gb_filter_create(gi, pi, &h->filt));
    RG_TRY(risa_gb_backprojection_create(gi, pi, &h->bp));
+   h->bp->engine = true;
    RG_TRY(risa_gb_masking_create(gi, pi, &h->mask));
    // attenuated frames are kept as frame quads (see QuadMap): room for the
    // padded quads of a batch with interleaved or with fixed planes

@@ -6,7 +6,8 @@ import pytest
 
 import oracle
 import risa_gb300 as rg
-from tests.helpers import rel_err
+from risa_gb300 import phantom
+from tests.helpers import SMALL, geom, rel_err
 
 torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
@@ -151,3 +152,34 @@ def test_two_streams(n, reserved, aligned, threads):
     for i in range(2):
         for img in imgs[i]:
             np.testing.assert_array_equal(img.cpu().numpy(), alone[i])
+
+
+@pytest.mark.parametrize("batch", [1, 4])
+def test_engine_beside_its_own_handle(batch):
+    """An engine's runs and replays on one stream, direct calls of its backprojection on another."""
+    d = dict(SMALL, n_par_proj=128, n_par_det=256, n_pixels=256)
+    sc = phantom.make_scan(batch, 1, 500, 432, 215.0, 240.0, seed=3, distinct=batch)
+    p = rg.make_params(masking=True)
+    fbp = rg.FBP(geom(d), p, sc.ref, 1, sc.dark, 1, max_batch=batch)
+    bp = fbp.backprojection()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    raw = torch.from_numpy(sc.raw.view(np.int16)).cuda()
+    img, img2 = _images(batch, 256), _images(batch, 256)
+    sino = _sino(batch, 128, 256, 9)
+    torch.cuda.synchronize()
+    graph = fbp.graph_capture(raw, img, 0, batch, a)
+    graph.replay(a)
+    torch.cuda.synchronize()
+    alone = img.cpu().numpy()
+    alone2 = _run(bp, sino, 256)
+    for _ in range(20):
+        img.fill_(float("nan"))
+        img2.fill_(float("nan"))
+        torch.cuda.synchronize()
+        graph.replay(a)
+        bp.enqueue(sino, img2, batch, b)
+        fbp.enqueue(raw, img, 0, batch, a)
+        bp.enqueue(sino, img2, batch, b)
+        bp.check()
+        np.testing.assert_array_equal(img.cpu().numpy(), alone)
+        np.testing.assert_array_equal(img2.cpu().numpy(), alone2)
