@@ -330,7 +330,10 @@ const char* risa_gb_backprojection_variant_name(int variant);
  * max_batch. Set-up call: may allocate and synchronise. Autotune and the FBP engine
  * reserve for their batch themselves, and a new handle holds four slices (where
  * that is at most 64 MB); an enqueue whose batch exceeds the reservation runs a
- * variant that stages windows from the sinogram itself. */
+ * variant that stages windows from the sinogram itself. Calls up to the largest
+ * reservation give the same bits however a job's slices are cut into batches (of
+ * sinograms aligned alike, to 16 bytes or not); a linear handle without one takes its
+ * kernel by the call's batch (up to 2, up to 4, more), and these round differently. */
 risa_gb_status risa_gb_backprojection_reserve(risa_gb_backprojection* h, int max_batch);
 /* Measurement: runs `reps` enqueues (after one warm-up) with CUDA events on
  * `stream` around the staging pass and around the backprojection kernel, and

@@ -308,6 +308,8 @@ struct risa_gb_backprojection {
       c.tile_win = tile_win.as<int2>();
       c.patch = &patch;
       c.few = reserved_batch <= 2;
+      const long tiles = (long)((g.N + 31) / 32) * ((g.N + 31) / 32);
+      c.split = tiles * std::max(reserved_batch, 1) <= kSplitMaxTiles;
       c.part = scratch ? part.as<float>() : nullptr;
       c.patch_angles = patch_angles.as<BPPatchAngle>();
       c.adj_scratch = adj.p;
@@ -317,13 +319,16 @@ struct risa_gb_backprojection {
    // Pair buffer for `batch` slices under every variant. Only set-up calls
    // (create of the engine, reserve, autotune) allocate; an enqueue whose
    // batch exceeds the reservation runs a variant that needs no pair buffer.
-   // The largest reservation also says how the handle is used: up to two slices
-   // take the patch kernel's form for single frames, whatever a call's batch, so
-   // that the calls of one handle give the same bits however a job is cut.
+   // The largest reservation also says how the handle is used, so that its calls up to
+   // that batch give the same bits however a job is cut: up to two slices always take
+   // the patch kernel's form for single frames, larger ones the staged form, and
+   // nearest-neighbour calls of any batch add their angles in one order. Without
+   // a reservation a linear call takes its form by its own batch (one or two slices,
+   // four, more), which round differently.
    int reserved_batch = 0;
    risa_gb_status reserve(int batch) {
       size_t need = 0;
-      for (int v = 0; v < bp_variant_count(); ++v)
+      for (int v = 0; p.interp == RISA_GB_INTERP_LINEAR && v < bp_variant_count(); ++v)  // the others stage nothing
          need = std::max(need, bp_pairs_bytes(v, batch, g.Pp, g.Dp, std::max(win_len[0], win_len[1])));
       std::lock_guard<std::mutex> hold(order.lock);
       if (need > pairs.bytes) {
@@ -1145,7 +1150,7 @@ risa_gb_status risa_gb_fbp_create(const risa_gb_geometry* gi, const risa_gb_para
    if (h->defects)
       RG_TRY(h->dws.alloc(defects_workspace_bytes(h->defects->cfg.D, max_batch, h->defects->cfg.max_runs, true)));
    RG_TRY(h->mm.alloc(sizeof(unsigned int) * 2 * (size_t)max_batch));
-   if (h->p.interp == RISA_GB_INTERP_LINEAR) RG_TRY(h->bp->reserve(max_batch));
+   RG_TRY(h->bp->reserve(max_batch));
    if (max_batch > 2) h->bp->part.release();  // for handles of one or two slices
    *out = h.release();
    return RISA_GB_OK;

@@ -69,7 +69,15 @@ __host__ __device__ inline int window_len(float scale, int tx, int ty) {
    return ((int)ceilf(scale * 1.41421357f * (float)(tx > ty ? tx : ty)) + 6 + 3) & ~3;
 }
 
-template <int TX, int TY, int PPT, int ACH, int INTERP>
+// Groups of angles of the nearest-neighbour modes. Where a handle's largest batch may
+// run as bp_nearest_split, whose four groups of threads take the angles in turn,
+// every kernel adds a pixel's angles in four groups (angle mod 4) and the groups in
+// order; other handles add them in one. So the calls of a handle give the same
+// bits however a job is cut. Four groups leave fewer warps on an SM (16 slices of 512^2 x
+// 720 angles 753 us, 645 in one group; 231^2 x 361 107 and 118).
+constexpr int kSplitGroups = 4;
+
+template <int TX, int TY, int PPT, int ACH, int INTERP, int G = 1>
 __global__ void __launch_bounds__(TX*(TY / PPT)) bp_tile(const float* __restrict__ sino,
                                                         float* __restrict__ img, BPCfg cfg,
                                                         int wlen) {
@@ -103,9 +111,12 @@ __global__ void __launch_bounds__(TX*(TY / PPT)) bp_tile(const float* __restrict
       }
    }
 
-   float acc[PPT];
+   static_assert(ACH % G == 0, "chunks start with the first group");
+   float acc[G][PPT];
 #pragma unroll
-   for (int r = 0; r < PPT; ++r) acc[r] = 0.f;
+   for (int g = 0; g < G; ++g)
+#pragma unroll
+      for (int r = 0; r < PPT; ++r) acc[g][r] = 0.f;
    const float* q = sino + (size_t)slice * Pp * Dp;
 
    for (int c0 = 0; c0 < Pp; c0 += ACH) {
@@ -133,8 +144,7 @@ __global__ void __launch_bounds__(TX*(TY / PPT)) bp_tile(const float* __restrict
          }
       }
       __syncthreads();
-#pragma unroll 4
-      for (int ai = 0; ai < na; ++ai) {
+      auto angle = [&](int ai, int g) {
          const float a = s_a[ai], b = s_b[ai];
          const float tb = s_rel[ai] + (float)tx * a + (float)ty * b;
          const float bstep = (float)ROWS * b;
@@ -147,11 +157,11 @@ __global__ void __launch_bounds__(TX*(TY / PPT)) bp_tile(const float* __restrict
                k = min(max(k, 0), wlen - 2);
                const float f = t - (float)k;
                const float q0 = w[k], q1 = w[k + 1];
-               acc[r] += q0 + f * (q1 - q0);
+               acc[g][r] += q0 + f * (q1 - q0);
             } else if (INTERP == RISA_GB_INTERP_NEAREST) {
                int k = __float2int_rd(t + 0.5f);
                k = min(max(k, 0), wlen - 1);
-               acc[r] += w[k];
+               acc[g][r] += w[k];
             } else {
                // truncation toward zero of t + Dp/2 (texture variant, Backprojection.cu:294)
                const float tt = t + cfg.trunc_offset;
@@ -159,9 +169,22 @@ __global__ void __launch_bounds__(TX*(TY / PPT)) bp_tile(const float* __restrict
                const int kg = k + s_w0[ai];
                if (kg == -1 && tt != (float)k) k += 1;
                k = min(max(k, 0), wlen - 1);
-               acc[r] += w[k];
+               acc[g][r] += w[k];
             }
          }
+      };
+      if constexpr (G == 1) {
+#pragma unroll 4
+         for (int ai = 0; ai < na; ++ai) angle(ai, 0);
+      } else {
+         int ai = 0;
+         for (; ai + G <= na; ai += G) {
+#pragma unroll
+            for (int u = 0; u < G; ++u) angle(ai + u, u);
+         }
+#pragma unroll
+         for (int u = 0; u < G - 1; ++u)
+            if (ai + u < na) angle(ai + u, u);
       }
       __syncthreads();
    }
@@ -169,7 +192,10 @@ __global__ void __launch_bounds__(TX*(TY / PPT)) bp_tile(const float* __restrict
    for (int r = 0; r < PPT; ++r) {
       const int x = x0 + tx, y = y0 + ty + ROWS * r;
       if (x < N && y < N) {
-         float v = acc[r] * cfg.norm;
+         float v = acc[0][r];
+#pragma unroll
+         for (int g = 1; g < G; ++g) v += acc[g][r];
+         v *= cfg.norm;
          if (cfg.masking) {
             const float dx = (float)x - c, dy = (float)y - c;
             if (dx * dx + dy * dy > lim) v = cfg.mask_value;
@@ -197,7 +223,7 @@ struct NearestVec<2> {
    using T = float2;
 };
 constexpr int kNearestAngles = 32;  // most angles per chunk
-template <int INTERP, int S>
+template <int INTERP, int S, int G>
 __global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__ sino, float* __restrict__ img,
                                                        BPCfg cfg, int wlen, int ach, int batch) {
    using V = typename NearestVec<S>::T;
@@ -215,11 +241,13 @@ __global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__
       const float ny = fminf(fmaxf(c, (float)y0), (float)(y0 + 31)) - c;
       live = nx * nx + ny * ny <= lim;
    }
-   float acc[4][S];
+   float acc[G][4][S];
 #pragma unroll
-   for (int r = 0; r < 4; ++r)
+   for (int g = 0; g < G; ++g)
 #pragma unroll
-      for (int s = 0; s < S; ++s) acc[r][s] = 0.f;
+      for (int r = 0; r < 4; ++r)
+#pragma unroll
+         for (int s = 0; s < S; ++s) acc[g][r][s] = 0.f;
    const size_t fs = (size_t)Pp * Dp;
    const float* q = sino + (size_t)s0 * fs;
    const int ns = min(S, batch - s0);
@@ -252,8 +280,7 @@ __global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__
          }
       }
       __syncthreads();
-#pragma unroll 2
-      for (int ai = 0; ai < na; ++ai) {
+      auto angle = [&](int ai, int g) {
          const float4 e = s_ang[ai];
          const float tb = fmaf((float)ty, e.y, fmaf((float)tx, e.x, e.z));
          const float bstep = 8.f * e.y;
@@ -269,13 +296,26 @@ __global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__
                 tt != fl - 8388608.f)
                k += 1u;
             const V u = w[min(k, top) - kFloorBits];
-            acc[r][0] += u.x;
-            acc[r][1] += u.y;
+            acc[g][r][0] += u.x;
+            acc[g][r][1] += u.y;
             if constexpr (S == 4) {
-               acc[r][2] += u.z;
-               acc[r][3] += u.w;
+               acc[g][r][2] += u.z;
+               acc[g][r][3] += u.w;
             }
          }
+      };
+      if constexpr (G == 1) {
+#pragma unroll 2
+         for (int ai = 0; ai < na; ++ai) angle(ai, 0);
+      } else {
+         int ai = 0;
+         for (; ai + G <= na; ai += G) {
+#pragma unroll
+            for (int u = 0; u < G; ++u) angle(ai + u, u);
+         }
+#pragma unroll
+         for (int u = 0; u < G - 1; ++u)
+            if (ai + u < na) angle(ai + u, u);
       }
       __syncthreads();
    }
@@ -289,18 +329,22 @@ __global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__
          out = out || dx * dx + dy * dy > lim;
       }
 #pragma unroll
-      for (int s = 0; s < S; ++s)
-         if (s < ns) img[((size_t)(s0 + s) * N + y) * N + x] = out ? cfg.mask_value : acc[r][s] * cfg.norm;
+      for (int s = 0; s < S; ++s) {
+         float v = acc[0][r][s];
+#pragma unroll
+         for (int g = 1; g < G; ++g) v += acc[g][r][s];
+         if (s < ns) img[((size_t)(s0 + s) * N + y) * N + x] = out ? cfg.mask_value : v * cfg.norm;
+      }
    }
 }
-template <int INTERP, int S>
-cudaError_t launch_nearest_tile(const float* sino, float* img, int batch, const BPCfg& cfg, cudaStream_t st) {
+template <int INTERP, int S, int G>
+cudaError_t launch_nearest_tile_as(const float* sino, float* img, int batch, const BPCfg& cfg, cudaStream_t st) {
    const int wlen = window_len(cfg.scale, 32, 32);
    // half the angles where the windows are wide (256^2 x 512 angles at 4 bins per pixel,
    // 30 slices: 412 us, 503 with 32)
    const int ach = cfg.scale <= 2.f ? kNearestAngles : kNearestAngles / 2;
    const size_t smem = sizeof(float) * S * (size_t)ach * wlen;
-   auto kern = bp_nearest_tile<INTERP, S>;
+   auto kern = bp_nearest_tile<INTERP, S, G>;
    if (smem > 47 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
@@ -308,6 +352,11 @@ cudaError_t launch_nearest_tile(const float* sino, float* img, int batch, const 
    const int t = (cfg.N + 31) / 32;
    kern<<<dim3(t, t, (batch + S - 1) / S), 256, smem, st>>>(sino, img, cfg, wlen, ach, batch);
    return cudaGetLastError();
+}
+template <int INTERP, int S>
+cudaError_t launch_nearest_tile(const float* sino, float* img, int batch, const BPCfg& cfg, cudaStream_t st) {
+   return cfg.split ? launch_nearest_tile_as<INTERP, S, kSplitGroups>(sino, img, batch, cfg, st)
+                    : launch_nearest_tile_as<INTERP, S, 1>(sino, img, batch, cfg, st);
 }
 
 // ---- nearest-neighbour modes, a few slices ---------------------------------------
@@ -318,9 +367,9 @@ cudaError_t launch_nearest_tile(const float* sino, float* img, int batch, const 
 // sinogram itself: a few slices stay in L1 and L2, and with no windows to stage
 // the loads of several angles are in flight. The coordinate is formed as
 // bp_tile forms it, from the same tile origin, so each pixel takes the same bins;
-// the groups' sums are added in shared memory.
+// the groups' sums are added in shared memory, in order.
 constexpr int kSplitAngles = 512;  // angles per table of coordinates
-constexpr int kSplitGroups = 4, kSplitStrips = 2;
+constexpr int kSplitStrips = 2;
 template <int INTERP>
 __global__ void __launch_bounds__(256 * kSplitGroups) bp_nearest_split(const float* __restrict__ sino, float* __restrict__ img,
                                                                        BPCfg cfg) {
@@ -406,12 +455,11 @@ __global__ void __launch_bounds__(256 * kSplitGroups) bp_nearest_split(const flo
       }
    }
 }
-// Up to 512 tiles (slices together): 231^2 of 361 angles 63 -> 28 us for one slice,
+// Up to kSplitMaxTiles tiles (slices together): 231^2 of 361 angles 63 -> 28 us for one slice,
 // 74 -> 67 for four; 512^2 of 720 angles 135 -> 122 us for one. From there on the
 // tiles fill the GPU and their windows are cheaper than loads of bins with their
 // bounds (one slice of 1024^2 x 1024 468 against 556 us). One group per
 // strip of 8 rows (one pixel per thread) takes 33 us for the first.
-constexpr long kSplitMaxTiles = 512;
 template <int INTERP>
 cudaError_t launch_nearest_split(const float* sino, float* img, int batch, const BPCfg& cfg, cudaStream_t st) {
    const int t = (cfg.N + 31) / 32;
@@ -1056,12 +1104,12 @@ cudaError_t launch_async_fit(const float* sino, float* img, int batch, const BPC
    }
 }
 
-template <int TX, int TY, int PPT, int ACH, int INTERP>
+template <int TX, int TY, int PPT, int ACH, int INTERP, int G = 1>
 cudaError_t launch_variant(const float* sino, float* img, int batch, const BPCfg& cfg,
                            cudaStream_t st) {
    const int wlen = window_len(cfg.scale, TX, TY);
    const size_t smem = sizeof(float) * ((size_t)ACH * wlen + 4 * ACH);
-   auto kern = bp_tile<TX, TY, PPT, ACH, INTERP>;
+   auto kern = bp_tile<TX, TY, PPT, ACH, INTERP, G>;
    if (smem > 48 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
@@ -1074,11 +1122,14 @@ cudaError_t launch_variant(const float* sino, float* img, int batch, const BPCfg
 template <int TX, int TY, int PPT, int ACH>
 cudaError_t launch_interp(const float* sino, float* img, int batch, const BPCfg& cfg,
                           cudaStream_t st) {
+   constexpr int G = kSplitGroups;
    switch (cfg.interp) {
       case RISA_GB_INTERP_NEAREST:
-         return launch_variant<TX, TY, PPT, ACH, RISA_GB_INTERP_NEAREST>(sino, img, batch, cfg, st);
+         return cfg.split ? launch_variant<TX, TY, PPT, ACH, RISA_GB_INTERP_NEAREST, G>(sino, img, batch, cfg, st)
+                          : launch_variant<TX, TY, PPT, ACH, RISA_GB_INTERP_NEAREST>(sino, img, batch, cfg, st);
       case RISA_GB_INTERP_NEAREST_TRUNC:
-         return launch_variant<TX, TY, PPT, ACH, RISA_GB_INTERP_NEAREST_TRUNC>(sino, img, batch, cfg, st);
+         return cfg.split ? launch_variant<TX, TY, PPT, ACH, RISA_GB_INTERP_NEAREST_TRUNC, G>(sino, img, batch, cfg, st)
+                          : launch_variant<TX, TY, PPT, ACH, RISA_GB_INTERP_NEAREST_TRUNC>(sino, img, batch, cfg, st);
       default:
          return launch_variant<TX, TY, PPT, ACH, RISA_GB_INTERP_LINEAR>(sino, img, batch, cfg, st);
    }
@@ -1471,7 +1522,7 @@ cudaError_t launch_backprojection(const float* sino, float* img, int batch, cons
       if (s == 2)
          return plain ? launch_nearest_tile<RISA_GB_INTERP_NEAREST, 2>(sino, img, batch, cfg, st)
                       : launch_nearest_tile<RISA_GB_INTERP_NEAREST_TRUNC, 2>(sino, img, batch, cfg, st);
-      if (tiles * batch <= kSplitMaxTiles)
+      if (cfg.split && tiles * batch <= kSplitMaxTiles)
          return plain ? launch_nearest_split<RISA_GB_INTERP_NEAREST>(sino, img, batch, cfg, st)
                       : launch_nearest_split<RISA_GB_INTERP_NEAREST_TRUNC>(sino, img, batch, cfg, st);
    }

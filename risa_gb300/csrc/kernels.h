@@ -301,6 +301,8 @@ inline size_t bp_part_bytes(int batch, int N) { return sizeof(float) * 4 * (size
 // Device bytes of the staged rows [quad of slices][angle][bin][4] of `batch` slices
 // and the quads' non-finite flags.
 size_t bp_quads_bytes(int batch, int Pp, int Dp);
+// Most 32 x 32 tiles of a nearest-neighbour call that splits its angles over thread groups
+constexpr long kSplitMaxTiles = 512;
 struct BPCfg {
    int Pp, Dp, N;
    const float* a;      // [Pp]
@@ -329,6 +331,7 @@ struct BPCfg {
                                     // coordinate of the tile origin in it), bp_tile_windows; else FP64 on device
    const BPPatchPlan* patch = nullptr;  // host side
    bool few = false;  // a caller of one or two slices at a time: the patch kernel over the sinogram itself
+   bool split = true;  // nearest-neighbour modes: a few slices may split their angles (kSplitMaxTiles)
    const BPPatchAngle* patch_angles = nullptr;  // the plan's angles, then its sym_angles
    float* part = nullptr;  // partial images of the symmetric form (bp_part_bytes)
    void* adj_scratch = nullptr;  // adjoint: slice-interleaved image copies (bp_adjoint_scratch_bytes)

@@ -183,3 +183,32 @@ def test_engine_beside_its_own_handle(batch):
         bp.check()
         np.testing.assert_array_equal(img.cpu().numpy(), alone)
         np.testing.assert_array_equal(img2.cpu().numpy(), alone2)
+
+
+@pytest.mark.parametrize("rot", [0.0, 21.0])
+@pytest.mark.parametrize("reserved,n,cuts", [(2, 2, [1]), (5, 5, [1, 2, 4]), (40, 40, [1, 2, 4, 5, 17])])
+def test_cuts_of_a_reserved_handle(reserved, n, cuts, rot):
+    """A linear handle reserved for a job's largest batch gives the same bits however the job is cut."""
+    Pp, Dp, N = 60, 96, 90
+    bp = _handle(Pp, Dp, N, rot)
+    bp.reserve(reserved)
+    sino = _sino(n, Pp, Dp, n)
+    whole = _run(bp, sino, N)
+    for m in cuts:
+        for first in sorted({0, (n - m) // 2, n - m}):
+            np.testing.assert_array_equal(_run(bp, sino[first:first + m].contiguous(), N), whole[first:first + m])
+
+
+@pytest.mark.parametrize("rot", [0.0, 21.0])
+def test_batches_of_an_unreserved_handle(rot):
+    """Two, four, five and more slices take different kernels without a reservation."""
+    Pp, Dp, N = 60, 96, 90
+    bp = _handle(Pp, Dp, N, rot)
+    sino = _sino(9, Pp, Dp, 3)
+    exp = [oracle.mask(oracle.backproject(s, N, rot), 0.0) for s in sino.cpu().numpy()]
+    for n in (1, 2, 3, 4, 5, 9):
+        got = _run(bp, sino[:n].contiguous(), N)
+        np.testing.assert_array_equal(_run(bp, sino[:n].contiguous(), N), got)
+        for b in range(n):
+            mr, _ = rel_err(got[b], exp[b])
+            assert mr < MAX_REL, (n, b, mr)
