@@ -161,26 +161,25 @@ __device__ __forceinline__ void flip(u64 (&acc)[SQ][2][4], bool x, bool y) {
 // The slices of a CTA's tile whose rows hold an infinity or a NaN (bit j of the
 // quad's flag: slice j), by the general two-bin rule: the patches also multiply a
 // third bin by a zero weight, which would carry it one pixel further. The CTA's
-// other slices have their pixels from the patches. A flagged quad at a time, one to
+// other slices have their pixels from the patches. A flagged slice at a time, one to
 // three pixels per thread, the windows of C angles in the copies' stages (16 rows of
-// every quad); all threads of the CTA, before the first copy (after the last patch
-// the call alone cost the finite CTAs 0.8%). 64 slices of 512^2 x 1024 angles 2.2 ms,
-// with one flagged quad 3.5 ms (108 with all quads of the CTA by scalar loads and FP64
-// coordinates).
+// 16-byte entries for every quad); all threads of the CTA, before the first copy (after
+// the last patch the call alone cost the finite CTAs 0.8%). 64 slices of 512^2 x 1024 angles 2.2 ms, with
+// one bad sample 3.3; 108 with every quad of the CTA
+// by scalar loads and FP64 coordinates, 3.5 with the flagged quad's four slices at once.
 template <int Q, int NT>
 __device__ __noinline__ void patch_general_tile(const PatchArgs& g) {
-   constexpr int C = Q < 3 ? 12 * Q : 32, PX = (kTile * kTile + NT - 1) / NT;  // angles per chunk, pixels per thread
+   constexpr int C = Q == 1 ? 40 : 64, PX = (kTile * kTile + NT - 1) / NT;  // angles per chunk, pixels per thread
    extern __shared__ __align__(128) unsigned char smem_raw[];
-   const int N = g.N, Dp = g.Dp, wlen = g.wlen, x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile, q0 = blockIdx.z * Q;
+   const int N = g.N, Dp = g.Dp, wlen = g.wlen, x0 = blockIdx.x * kTile, y0 = blockIdx.y * kTile;
    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-   float4* win = reinterpret_cast<float4*>(smem_raw);  // [C][wlen]
-   float4* tab = win + (size_t)C * wlen;               // a, b, window-relative coordinate, first bin
-   for (int q = q0; q < min(q0 + Q, g.n_quads); ++q) {
-      const int flags = __ldg(g.nonfinite + q);
-      if (!flags) continue;
-      float acc[PX][4];
+   float4* tab = reinterpret_cast<float4*>(smem_raw);  // a, b, window-relative coordinate, first bin
+   float* win = reinterpret_cast<float*>(tab + C);     // [C][wlen]
+   for (int sl = 4 * blockIdx.z * Q; sl < min(4 * (int)(blockIdx.z + 1) * Q, g.batch); ++sl) {
+      if (!(__ldg(g.nonfinite + (sl >> 2)) >> (sl & 3) & 1)) continue;
+      float acc[PX];
 #pragma unroll
-      for (int r = 0; r < PX; ++r) acc[r][0] = acc[r][1] = acc[r][2] = acc[r][3] = 0.f;
+      for (int r = 0; r < PX; ++r) acc[r] = 0.f;
       for (int c0 = 0; c0 < g.Pp; c0 += C) {
          const int na = min(C, g.Pp - c0);
          __syncthreads();
@@ -193,13 +192,14 @@ __device__ __noinline__ void patch_general_tile(const PatchArgs& g) {
          }
          __syncthreads();
          for (int ai = warp; ai < na; ai += NT / 32) {
-            const float4* row = g.quads + ((size_t)q * g.Pp + __ldg(&g.ang[c0 + ai].index)) * Dp;
+            const float* row = reinterpret_cast<const float*>(
+                                   g.quads + ((size_t)(sl >> 2) * g.Pp + __ldg(&g.ang[c0 + ai].index)) * Dp) + (sl & 3);
             const int w0 = __float_as_int(tab[ai].w);
             for (int m = lane; m < wlen; m += 32)
-               win[ai * wlen + m] = (unsigned)(w0 + m) < (unsigned)Dp ? __ldg(row + w0 + m) : make_float4(0.f, 0.f, 0.f, 0.f);
+               win[ai * wlen + m] = (unsigned)(w0 + m) < (unsigned)Dp ? __ldg(row + 4 * (w0 + m)) : 0.f;
          }
          __syncthreads();
-#pragma unroll 1
+#pragma unroll 2
          for (int ai = 0; ai < na; ++ai) {
             const float4 e = tab[ai];
 #pragma unroll
@@ -209,12 +209,9 @@ __device__ __noinline__ void patch_general_tile(const PatchArgs& g) {
                const float fx = (float)(e.x < 0.f ? kTile - 1 - px : px), fy = (float)(e.y < 0.f ? kTile - 1 - py : py);
                const float t = fmaf(fy, fabsf(e.y), fmaf(fx, fabsf(e.x), e.z));
                const float fl = floorf(t), f = (t - fl) - 0.5f;
-               const float4* w = win + ai * wlen + min((int)fl, wlen - 2);  // the patches of this tile reach as many bins
-               const float4 u = w[0], v = w[1];
-               acc[r][0] = fmaf(f, v.x - u.x, acc[r][0] + 0.5f * (u.x + v.x));
-               acc[r][1] = fmaf(f, v.y - u.y, acc[r][1] + 0.5f * (u.y + v.y));
-               acc[r][2] = fmaf(f, v.z - u.z, acc[r][2] + 0.5f * (u.z + v.z));
-               acc[r][3] = fmaf(f, v.w - u.w, acc[r][3] + 0.5f * (u.w + v.w));
+               const float* w = win + ai * wlen + min((int)fl, wlen - 2);  // the patches of this tile reach as many bins
+               const float u = w[0], v = w[1];
+               acc[r] = fmaf(f, v - u, acc[r] + 0.5f * (u + v));
             }
          }
       }
@@ -225,9 +222,7 @@ __device__ __noinline__ void patch_general_tile(const PatchArgs& g) {
          if (p >= kTile * kTile || x >= N || y >= N) continue;
          const float dx = (float)x - c, dy = (float)y - c;
          const bool out = g.masking && dx * dx + dy * dy > lim;
-         for (int j = 0; j < 4; ++j)
-            if ((flags >> j & 1) && 4 * q + j < g.batch)
-               g.img[((size_t)(4 * q + j) * N + y) * N + x] = out ? g.mask_value : acc[r][j] * g.norm;
+         g.img[((size_t)sl * N + y) * N + x] = out ? g.mask_value : acc[r] * g.norm;
       }
    }
 }
