@@ -340,15 +340,19 @@ def timed(torch, stream, fn, reps: int) -> float:
 
 def bp_smem_bytes_per_update(variant_name):
     """Shared-memory bytes per pixel x angle update and slice of the workload's
-    backprojection: a 2 x 2 patch reads floor(|a| + |b|) + 3 bins of 4 B per slice
-    for its 4 pixels (a, b: bins per pixel along x and y); the record variants
-    read one FP32 (midpoint, difference) pair per pixel."""
+    backprojection, as the kernel issues them: a 2 x 2 patch at span |a| + |b|
+    (bins per pixel along x and y) and m = floor(span) reads m + 2 bins of 4 B per slice
+    for its 4 pixels, and the next one where its far pixel lies beyond the middle
+    of its three (the kernel of large batches leaves that load out elsewhere: span - m of the
+    patches); the record variants read one FP32 (midpoint, difference) pair per
+    pixel."""
     if variant_name != "patch_2x2":
         return 8.0
     scale = WORKLOAD["n_par_det"] / WORKLOAD["n_pixels"]
     th = np.arange(WORKLOAD["n_par_proj"]) * np.pi / WORKLOAD["n_par_proj"]
     span = scale * (np.abs(np.cos(th)) + np.abs(np.sin(th)))
-    return float(np.mean(np.minimum(np.floor(span), 2) + 3))
+    m = np.minimum(np.floor(span), 2)
+    return float(np.mean(m + 2 + (span - m)))
 
 
 def measure_e2e(args, sc, fbp, torch, rg):
