@@ -463,7 +463,10 @@ typedef struct risa_gb_sweep_instance {
    const uint8_t* defect_map; /* host [n_par_det], nonzero = defective column; NULL = none */
 } risa_gb_sweep_instance;
 typedef struct risa_gb_sweep risa_gb_sweep;
-/* Builds every instance's tables (FP64 on the host) and the work list. */
+/* Builds every instance's tables (FP64 on the host) and the work list. A sweep of 5000
+ * tiles of 32 x 32 pixels and more takes the angles of unrotated instances in sets of
+ * four, which needs four more copies of their images (up to 4 GiB in all; without where
+ * that cannot be had) and rounds an instance's sums differently than a small sweep does. */
 risa_gb_status risa_gb_sweep_create(const risa_gb_sweep_instance* inst, int n, risa_gb_sweep** out);
 /* Packed layouts of the inputs (uint16 [Pp][Dp] per instance) and outputs
  * (float [N][N]): element offsets of each instance and the totals. Any
@@ -479,7 +482,7 @@ risa_gb_status risa_gb_sweep_enqueue(risa_gb_sweep* h, const uint16_t* raw, floa
 risa_gb_status risa_gb_sweep_graph_capture(risa_gb_sweep* h, const uint16_t* raw, float* img, void* stream,
                                           risa_gb_graph** out);
 /* Synchronises; per instance the %globaltimer time (ns) its first row group
- * started and its last tile finished in the last enqueue, and the launch's
+ * started and its last tile (or sum, in a large sweep) finished in the last enqueue, and the launch's
  * earliest CTA start. Any pointer may be NULL. */
 risa_gb_status risa_gb_sweep_times(risa_gb_sweep* h, uint64_t* first_ns, uint64_t* done_ns,
                                    uint64_t* launch_ns);

@@ -1579,9 +1579,9 @@ cudaError_t launch_backprojection_adjoint(const float* img, float* sino, int bat
       // warps (8 slices of 290^2 -> 161 x 372 112 us, 132 with one warp, 221 without the
       // layout; one of 96^2 -> 90 x 96 43, 48 with eight angles per CTA, 85 without).
       const int columns = (cfg.Dp + 31) / 32;
-      const int halves = batch > 4 && (long)columns * cfg.Pp * groups < 4864 ? 2 : 1;
+      const int halves = batch > 4 && (long)columns * cfg.Pp * groups < 32 * kSMs ? 2 : 1;
       int apc = 8;
-      while (apc > 1 && (long)columns * ((cfg.Pp + apc - 1) / apc) * groups * halves < 304) apc /= 2;
+      while (apc > 1 && (long)columns * ((cfg.Pp + apc - 1) / apc) * groups * halves < 2 * kSMs) apc /= 2;
       while (apc > 1 && sizeof(float2) * (size_t)apc * cfg.N > 48 * 1024) apc /= 2;
       const size_t lines = sizeof(float2) * (size_t)apc * cfg.N;
       dim3 grid(columns, (cfg.Pp + apc - 1) / apc, groups * halves);

@@ -4,11 +4,13 @@
 // What bounds a linear backprojection is the shared-memory data path: a
 // (midpoint, difference) record per pixel, angle and slice is 8 B of every
 // 128 B/clk (bp_linear_async, k_bp.cu: 23.8 ms per 512 slices of 1024 x 1024
-// -> 512^2, 0.90 of that bound). Here a thread owns a 2 x 2 pixel patch of 4
-// (or 8) slices and reads each detector bin its patch touches once: with
+// -> 512^2, 0.90 of that bound). Here a thread owns a 2 x 2 pixel patch of 4, 8
+// or 16 slices and reads each detector bin its patch touches once: with
 // A = |a|, B = |b| (bins per pixel along x and y) the patch spans A + B bins,
 // so floor(A + B) + 3 bins serve 4 pixels -- 5 loads of 16 B at 2 bins per
-// pixel and 4 at 1, where the records took 8.
+// pixel and 4 at 1, where the records took 8. The form for large batches leaves the last
+// out where its weight is 0: 4.55 B per update and slice at 2 bins per pixel, 15.7 ms
+// for the launch above, 0.78 of the measured 40 TB/s counting the pixels in the circle alone.
 //
 //   * A pixel at offset o from the patch's lowest coordinate k + g (g in [0, 1])
 //     reads the three bins m .. m + 2 around g + o, m = floor(o), with the hat
@@ -46,6 +48,7 @@
 #include "kernels.h"
 #include "patch_window.cuh"
 #include "risa_gb300.h"
+#include "tensor_map.h"
 
 namespace risa_gb {
 
@@ -746,23 +749,6 @@ __global__ void __launch_bounds__(256) bp_quads_fill(const float* __restrict__ s
    if (flags && (flags & ~*reinterpret_cast<volatile int*>(nonfinite + q))) atomicOr(nonfinite + q, flags);
 }
 
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encode_fn() {
-   static const EncodeTiled fn = [] {
-      void* p = nullptr;
-      cudaDriverEntryPointQueryResult q;
-      if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-              cudaSuccess &&
-          q == cudaDriverEntryPointSuccess)
-         return reinterpret_cast<EncodeTiled>(p);
-      return EncodeTiled(nullptr);
-   }();
-   return fn;
-}
-
 // Staged row of one angle and quad, in 16-byte entries: the bins a 16-pixel
 // tile reaches, rounded up so that the rows of the QL quads of a load phase
 // start in different banks (QL rows 8 / QL entries apart modulo a bank row) and
@@ -1030,14 +1016,14 @@ cudaError_t launch_bp_patch(const float* sino, float* img, int batch, const BPCf
    // the most CTAs that an SM gets, of the tiles that meet the circle where it is
    // masked, times a form's cost.
    const long live = live_tiles(cfg.N, cfg.masking != 0);
-   auto rounds = [live, nq](int quads) { return (live * ((nq + quads - 1) / quads) + 151) / 152; };
+   auto rounds = [live, nq](int quads) { return (live * ((nq + quads - 1) / quads) + kSMs - 1) / kSMs; };
    if (cfg.scale <= 1.25f) {
       // Four quads per thread spread a patch's weights (a fifth of the FP32 work)
       // over twice the slices: 1.84 times the time of half the slices (32 slices of
       // 512^2 x 720 angles 773 us against 844, of 256^2 x 512 128 slices 570 against 618;
       // 64 slices of that, four CTAs per SM for seven halves, 217 against 209), if an SM
       // has two.
-      if (live * ((nq + 7) / 8) >= 304 && 184 * rounds(8) <= 100 * rounds(4))
+      if (live * ((nq + 7) / 8) >= 2 * kSMs && 184 * rounds(8) <= 100 * rounds(4))
          return launch_patch<4, 2, 2>(a, pp, cfg.scale, st);
       return launch_patch<2, 2, 3>(a, pp, cfg.scale, st);
    }

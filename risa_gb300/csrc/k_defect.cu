@@ -431,10 +431,10 @@ cudaError_t launch_defect_detect(const uint16_t* frames, int batch, const Defect
        cfg.P - 1 <= 8 * 32768) {
       // one block spans a frame's column octets where it can (D <= 2048);
       // the cluster's CTAs split the rows. A few frames (fewer CTAs of that kind
-      // than keep 152 SMs busy) take blocks of 32 octets with the rows split further.
+      // than keep the SMs busy) take blocks of 32 octets with the rows split further.
       const int octets = cfg.D / 8;
       const int rows = std::max(1, (cfg.P - 1 + kStatCluster - 1) / kStatCluster);
-      if ((long)batch * kStatCluster < 8 * 152) {
+      if ((long)batch * kStatCluster < 8 * kSMs) {
          dim3 grid(kStatCluster * ((octets + 31) / 32), 1, batch);
          defect_stats_cluster<8><<<grid, 256, 0, st>>>(frames, ws.stats, cfg.P, cfg.D, rows, cfg.modules);
       } else {
@@ -452,7 +452,7 @@ cudaError_t launch_defect_detect(const uint16_t* frames, int batch, const Defect
    // up to one frame per SM takes wide blocks (one frame of 432 columns with its run
    // list 6.9 us; 27 with 256 threads and one of them listing the runs), a batch
    // fills the SMs with small ones (512 frames of 1152 columns 21 us)
-   const int threads = batch <= 152 ? std::min(1024, (cfg.D + 31) / 32 * 32) : 256;
+   const int threads = batch <= kSMs ? std::min(1024, (cfg.D + 31) / 32 * 32) : 256;
    defect_flags<<<batch, threads, smem, st>>>(ws.stats, cfg, flags_out, ws.counts, ws.runs, ws.fix_counts,
                                           ws.fixes);
    return cudaGetLastError();

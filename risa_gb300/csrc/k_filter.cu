@@ -423,7 +423,8 @@ __global__ void __launch_bounds__(r16_threads<LEN>(), 512 / r16_threads<LEN>())
 // patch backprojection's slice quads, quads[s / 4][angle][bin][s % 4]: the
 // values go straight from the last pass's registers (8 bytes per bin; the two
 // row pairs of a quad and angle are neighbouring groups, whose halves of each
-// entry meet in L2).
+// entry meet in L2). Two slices share a transform, so a slice's low bits depend on its
+// partner, as in filter_rows_r16_pairs.
 template <int LEN, bool HALF>
 __global__ void __launch_bounds__(r16_threads<LEN>(), 512 / r16_threads<LEN>())
     filter_rows_r16_quads(const float* __restrict__ sino, int batch, FilterCfg cfg, float* __restrict__ quads) {

@@ -32,6 +32,7 @@
 
 #include "async_copy.h"
 #include "kernels.h"
+#include "tensor_map.h"
 #include "toeplitz.h"
 
 namespace risa_gb {
@@ -488,24 +489,6 @@ __global__ void split_f16_rows(const float* __restrict__ x, __half* __restrict__
       }
    }
    if (lane == 0) row_inv[row] = inv;
-}
-
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encode_fn() {
-   static EncodeTiled fn = nullptr;
-   if (!fn) {
-      void* p = nullptr;
-      cudaDriverEntryPointQueryResult q;
-      // the driver API's cuTensorMapEncodeTiled as introduced in CUDA 12.0
-      if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000, cudaEnableDefault, &q) ==
-              cudaSuccess &&
-          q == cudaDriverEntryPointSuccess)
-         fn = reinterpret_cast<EncodeTiled>(p);
-   }
-   return fn;
 }
 
 // 16-bit matrix [rows][cols] (cols contiguous), boxes of 64 columns x box_rows rows.

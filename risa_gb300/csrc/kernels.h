@@ -9,6 +9,10 @@
 
 namespace risa_gb {
 
+// SMs of a GB300, where the lines of the launch rules were measured. Another count
+// moves the lines, not the results.
+constexpr int kSMs = 152;
+
 // ---------------------------------------------------------------- defects
 // Per-column statistics of one frame (interpolationFunctions.h:36-47):
 // total variation over consecutive projections (exact integer sum) and the
