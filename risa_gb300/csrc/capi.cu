@@ -230,7 +230,7 @@ constexpr int kAutoVariant = -1;
 // than the last one's first waits for the event recorded after that.
 struct BufferOrder {
    std::mutex lock;
-   cudaEvent_t done = nullptr;     // after the last use
+   cudaEvent_t done = nullptr;     // after the last use (linear handles have one)
    unsigned long long stream = 0;  // where that was
    bool used = false;
    ~BufferOrder() {
@@ -242,9 +242,8 @@ class BufferUse {
    explicit BufferUse(BufferOrder& o) : o_(o), hold_(o.lock) {}
    // Before the call's first launch on `st`; the destructor follows its last one.
    cudaError_t begin(cudaStream_t st) {
-      cudaError_t e = cudaSuccess;
-      if (!o_.done && (e = cudaEventCreateWithFlags(&o_.done, cudaEventDisableTiming)) != cudaSuccess) return e;
-      if ((e = cudaStreamGetId(st, &id_)) != cudaSuccess) return e;
+      cudaError_t e = cudaStreamGetId(st, &id_);
+      if (e != cudaSuccess) return e;
       if (o_.used && id_ != o_.stream && (e = cudaStreamWaitEvent(st, o_.done, 0)) != cudaSuccess) return e;
       st_ = st;
       begun_ = true;
@@ -888,6 +887,7 @@ risa_gb_status risa_gb_backprojection_create(const risa_gb_geometry* gi, const r
    RG_TRY(h->err.alloc(sizeof(int)));
    RG_CUDA(cudaMemset(h->err.p, 0, sizeof(int)));
    if (h->p.interp == RISA_GB_INTERP_LINEAR) {
+      RG_CUDA(cudaEventCreateWithFlags(&h->order.done, cudaEventDisableTiming));
       // 8 B per tile and angle (2 MB for 512^2 x 1024 angles); very large
       // geometries keep computing the window starts on the device instead
       const size_t tiles = (size_t)((h->g.N + 31) / 32) * ((h->g.N + 31) / 32);
@@ -945,7 +945,7 @@ risa_gb_status risa_gb_backprojection_time(risa_gb_backprojection* h, const floa
       BufferUse use(h->order);
       BPCfg c = h->cfg(fused);
       c.mid_event = ev[1];
-      cudaError_t e = use.begin(st);
+      cudaError_t e = h->p.interp == RISA_GB_INTERP_LINEAR ? use.begin(st) : cudaSuccess;
       if (e == cudaSuccess) e = cudaEventRecord(ev[0], st);
       if (e == cudaSuccess) e = launch_backprojection(sino, img, batch, c, h->variant_for(c, sino, batch), st);
       if (e == cudaSuccess) e = cudaEventRecord(ev[2], st);
