@@ -1254,10 +1254,10 @@ __device__ __forceinline__ ulonglong2 ldg_if(const ulonglong2* ptr, bool p) {
 // terms: the same bits (shares of the rows per warp, added at the end, were faster
 // for small geometries but rounded differently).
 // What bounds it is L1 wavefronts: per row and warp, two candidate pixels of NH
-// 16-byte loads (4.5 wavefronts each; 82% of the data path). 16 slices of 512^2
+// 16-byte loads (4.5 wavefronts each; 75% of the data path) and their latency. 16 slices of 512^2
 // -> 720 x 768: 1.77 ms with 32-byte pixel records and one angle per CTA (7
-// wavefronts a load, 6.8 TB/s from L2), 1.24 ms in this layout, 1.13 ms with the
-// loads of two rows issued before their multiply-adds (four rows: 1.16).
+// wavefronts a load, 6.8 TB/s from L2), 1.24 ms in this layout, 1.16 ms with the
+// loads of two rows issued before their multiply-adds (1.18 with the layout pass).
 template <int NH>
 __global__ void __launch_bounds__(256) bp_adjoint_rows(const float4* __restrict__ P, const float4* __restrict__ PT,
                                                        float* __restrict__ sino, BPCfg cfg, int batch, int apc,
