@@ -308,7 +308,7 @@ struct risa_gb_backprojection {
       c.patch = &patch;
       c.few = reserved_batch <= 2;
       const long tiles = (long)((g.N + 31) / 32) * ((g.N + 31) / 32);
-      c.split = tiles * std::max(reserved_batch, 1) <= kSplitMaxTiles;
+      c.split = tiles * (reserved_batch > 0 ? reserved_batch : 2) <= kSplitMaxTiles;
       c.part = scratch ? part.as<float>() : nullptr;
       c.patch_angles = patch_angles.as<BPPatchAngle>();
       c.adj_scratch = adj.p;

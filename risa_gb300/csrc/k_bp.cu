@@ -74,7 +74,9 @@ __host__ __device__ inline int window_len(float scale, int tx, int ty) {
 // every kernel adds a pixel's angles in four groups (angle mod 4) and the groups in
 // order; other handles add them in one. So the calls of a handle give the same
 // bits however a job is cut. Four groups leave fewer warps on an SM (16 slices of 512^2 x
-// 720 angles 753 us, 645 in one group; 231^2 x 361 107 and 118).
+// 720 angles 753 us, 645 in one group; 231^2 x 361 107 and 118), so a handle without a
+// reservation counts as one of two slices: three and four slices of 513^2 to 736^2 lost up
+// to a fifth in groups, while one of 640^2 takes 150 us unsplit and 168 split (600^2 150, 143).
 constexpr int kSplitGroups = 4;
 
 template <int TX, int TY, int PPT, int ACH, int INTERP, int G = 1>
