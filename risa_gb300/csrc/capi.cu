@@ -307,8 +307,9 @@ struct risa_gb_backprojection {
       c.tile_win = tile_win.as<int2>();
       c.patch = &patch;
       c.few = reserved_batch <= 2;
+      // the grouped kernels' CTAs (four slices, two on an SM) all run at once
       const long tiles = (long)((g.N + 31) / 32) * ((g.N + 31) / 32);
-      c.split = tiles * (reserved_batch > 0 ? reserved_batch : 2) <= kSplitMaxTiles;
+      c.split = tiles * ((reserved_batch + 3) / 4 + (reserved_batch == 0)) <= 2 * kSMs;
       c.part = scratch ? part.as<float>() : nullptr;
       c.patch_angles = patch_angles.as<BPPatchAngle>();
       c.adj_scratch = adj.p;

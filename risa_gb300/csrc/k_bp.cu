@@ -69,14 +69,16 @@ __host__ __device__ inline int window_len(float scale, int tx, int ty) {
    return ((int)ceilf(scale * 1.41421357f * (float)(tx > ty ? tx : ty)) + 6 + 3) & ~3;
 }
 
-// Groups of angles of the nearest-neighbour modes. Where a handle's largest batch may
-// run as bp_nearest_split, whose four groups of threads take the angles in turn,
-// every kernel adds a pixel's angles in four groups (angle mod 4) and the groups in
-// order; other handles add them in one. So the calls of a handle give the same
-// bits however a job is cut. Four groups leave fewer warps on an SM (16 slices of 512^2 x
-// 720 angles 753 us, 645 in one group; 231^2 x 361 107 and 118), so a handle without a
-// reservation counts as one of two slices: three and four slices of 513^2 to 736^2 lost up
-// to a fifth in groups, while one of 640^2 takes 150 us unsplit and 168 split (600^2 150, 143).
+// Groups of angles of the nearest-neighbour modes. Small handles (BPCfg::split) run a few
+// slices as bp_nearest_split, whose four groups of threads take the angles in turn, so
+// every kernel of theirs adds a pixel's angles in four groups (angle mod 4) and the
+// groups in order; the others never split and add them in one. So the calls of a handle
+// give the same bits however a job is cut. With four groups two CTAs of four slices fit
+// an SM, with one five: a handle is small while its largest batch (up to four slices
+// without a reservation) is one such wave. 720 angles, four groups and one: three slices of 512^2
+// 181 and 200 us, of 600^2 293 and 249, of 704^2 353 and 318, 16 of 512^2 753 and 645; 16
+// of 231^2 x 361 107 and 118. One slice, split and not: 512^2 115 and 135, 600^2 143 and
+// 150, 640^2 168 and 150.
 constexpr int kSplitGroups = 4;
 
 template <int TX, int TY, int PPT, int ACH, int INTERP, int G = 1>

@@ -335,7 +335,7 @@ struct BPCfg {
                                     // coordinate of the tile origin in it), bp_tile_windows; else FP64 on device
    const BPPatchPlan* patch = nullptr;  // host side
    bool few = false;  // a caller of one or two slices at a time: the patch kernel over the sinogram itself
-   bool split = true;  // nearest-neighbour modes: a few slices may split their angles (kSplitMaxTiles)
+   bool split = true;  // nearest-neighbour modes: a few slices split their angles (kSplitMaxTiles)
    const BPPatchAngle* patch_angles = nullptr;  // the plan's angles, then its sym_angles
    float* part = nullptr;  // partial images of the symmetric form (bp_part_bytes)
    void* adj_scratch = nullptr;  // adjoint: slice-interleaved image copies (bp_adjoint_scratch_bytes)
