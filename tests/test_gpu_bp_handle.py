@@ -212,3 +212,21 @@ def test_batches_of_an_unreserved_handle(rot):
         for b in range(n):
             mr, _ = rel_err(got[b], exp[b])
             assert mr < MAX_REL, (n, b, mr)
+
+
+@pytest.mark.parametrize("n", [1, 4])
+def test_default_and_other_streams_in_turn(n):
+    """The legacy stream, whose use is recorded only when another stream follows, and two others."""
+    Pp, Dp, N = 180, 256, 256
+    bp = _handle(Pp, Dp, N)
+    streams = [None, torch.cuda.Stream(), torch.cuda.Stream()]
+    sinos = [_sino(n, Pp, Dp, seed) for seed in range(3)]
+    alone = [_run(bp, s, N) for s in sinos]
+    order = [0, 1, 0, 0, 2, 1, 1, 0, 2, 2, 0, 1] * 3
+    imgs = [_images(n, N) for _ in order]
+    torch.cuda.synchronize()
+    for i, img in zip(order, imgs):
+        bp.enqueue(sinos[i], img, n, streams[i])
+    bp.check()
+    for i, img in zip(order, imgs):
+        np.testing.assert_array_equal(img.cpu().numpy(), alone[i])
