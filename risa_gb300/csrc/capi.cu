@@ -316,7 +316,7 @@ struct risa_gb_backprojection {
       c.tile_win = tile_win.as<int2>();
       c.patch = &patch;
       c.few = reserved_batch <= 2;
-      // the grouped kernels' CTAs (four slices, two on an SM) all run at once
+      // small enough to split: up to two CTAs of four slices per SM (one slice up to 557^2)
       const long tiles = (long)((g.N + 31) / 32) * ((g.N + 31) / 32);
       c.split = tiles * ((reserved_batch + 3) / 4 + (reserved_batch == 0)) <= 2 * kSMs;
       c.part = scratch ? part.as<float>() : nullptr;

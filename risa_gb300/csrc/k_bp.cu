@@ -71,15 +71,36 @@ __host__ __device__ inline int window_len(float scale, int tx, int ty) {
 
 // Groups of angles of the nearest-neighbour modes. Small handles (BPCfg::split) run a few
 // slices as bp_nearest_split, whose four groups of threads take the angles in turn, so
-// every kernel of theirs adds a pixel's angles in four groups (angle mod 4) and the
+// every kernel of theirs adds a pixel's angles group by group (angle mod 4), and the
 // groups in order; the others never split and add them in one. So the calls of a handle
-// give the same bits however a job is cut. With four groups two CTAs of four slices fit
-// an SM, with one five: a handle is small while its largest batch (up to four slices
-// without a reservation) is one such wave. 720 angles, four groups and one: three slices of 512^2
-// 181 and 200 us, of 600^2 293 and 249, of 704^2 353 and 318, 16 of 512^2 753 and 645; 16
-// of 231^2 x 361 107 and 118. One slice, split and not: 512^2 115 and 135, 600^2 143 and
-// 150, 640^2 168 and 150.
+// give the same bits however a job is cut. A thread that walks all groups takes them one
+// after the other and needs one more sum per pixel: 16 slices of 512^2 x 720 662 us (645 in
+// one group), of 231^2 x 361 121 (118), eight of 423^2 x 300 111 (113). The split form
+// saves a few slices more than that where their tiles are few: one slice of 512^2 115 us
+// (135 unsplit), of 600^2 143 (150), of 640^2 168 (150). (With the angles in their order
+// and a sum for each group, 16 slices of 512^2 took 753 us; groups of consecutive angles
+// leave the split form's unbalanced, whose loads spread with the angle: 231^2 25 us for 18.6.)
 constexpr int kSplitGroups = 4;
+// The angles of G groups one after the other: position p holds the angle at(p), and
+// group g ends at position end(g).
+template <int G>
+struct GroupedAngles {
+   int Pp;
+   __device__ __forceinline__ int end(int g) const {
+      if (G == 1) return Pp;
+      int e = 0;
+#pragma unroll
+      for (int k = 0; k < G; ++k) e += k <= g ? (Pp - k + G - 1) / G : 0;
+      return e;
+   }
+   __device__ __forceinline__ int at(int p) const {
+      if (G == 1) return p;
+      int g = 0;
+#pragma unroll
+      for (int k = 0; k < G - 1; ++k) g += p >= end(k) ? 1 : 0;
+      return (p - (g > 0 ? end(g - 1) : 0)) * G + g;
+   }
+};
 
 template <int TX, int TY, int PPT, int ACH, int INTERP, int G = 1>
 __global__ void __launch_bounds__(TX*(TY / PPT)) bp_tile(const float* __restrict__ sino,
@@ -115,18 +136,17 @@ __global__ void __launch_bounds__(TX*(TY / PPT)) bp_tile(const float* __restrict
       }
    }
 
-   static_assert(ACH % G == 0, "chunks start with the first group");
-   float acc[G][PPT];
+   float acc[PPT], sum[PPT];  // sum: the groups before this one
 #pragma unroll
-   for (int g = 0; g < G; ++g)
-#pragma unroll
-      for (int r = 0; r < PPT; ++r) acc[g][r] = 0.f;
+   for (int r = 0; r < PPT; ++r) acc[r] = sum[r] = 0.f;
    const float* q = sino + (size_t)slice * Pp * Dp;
 
+   const GroupedAngles<G> angles{Pp};
+   int g = 0, end = angles.end(0);  // the group at hand
    for (int c0 = 0; c0 < Pp; c0 += ACH) {
       const int na = min(ACH, Pp - c0);
       if (threadIdx.x < na) {
-         const int ang = c0 + threadIdx.x;
+         const int ang = angles.at(c0 + threadIdx.x);
          const float a = __ldg(cfg.a + ang), b = __ldg(cfg.b + ang);
          const double base = __ldg(cfg.t0 + ang) + (double)x0 * __ldg(cfg.ad + ang) +
                              (double)y0 * __ldg(cfg.bd + ang);
@@ -141,65 +161,62 @@ __global__ void __launch_bounds__(TX*(TY / PPT)) bp_tile(const float* __restrict
       __syncthreads();
       for (int ai = threadIdx.x / 32; ai < na; ai += NT / 32) {
          const int w0 = s_w0[ai];
-         const float* row = q + (size_t)(c0 + ai) * Dp;
+         const float* row = q + (size_t)angles.at(c0 + ai) * Dp;
          for (int m = threadIdx.x % 32; m < wlen; m += 32) {
             const int k = w0 + m;
             win[ai * wlen + m] = (k >= 0 && k < Dp) ? __ldg(row + k) : 0.f;
          }
       }
       __syncthreads();
-      auto angle = [&](int ai, int g) {
-         const float a = s_a[ai], b = s_b[ai];
-         const float tb = s_rel[ai] + (float)tx * a + (float)ty * b;
-         const float bstep = (float)ROWS * b;
-         const float* w = win + ai * wlen;
+      int ai = 0;
+      do {  // the part of the chunk in each group
+         const int stop = G > 1 ? min(na, end - c0) : na;
+#pragma unroll 4
+         for (; ai < stop; ++ai) {
+            const float a = s_a[ai], b = s_b[ai];
+            const float tb = s_rel[ai] + (float)tx * a + (float)ty * b;
+            const float bstep = (float)ROWS * b;
+            const float* w = win + ai * wlen;
 #pragma unroll
-         for (int r = 0; r < PPT; ++r) {
-            const float t = tb + (float)r * bstep;
-            if (INTERP == RISA_GB_INTERP_LINEAR) {
-               int k = __float2int_rd(t);
-               k = min(max(k, 0), wlen - 2);
-               const float f = t - (float)k;
-               const float q0 = w[k], q1 = w[k + 1];
-               acc[g][r] += q0 + f * (q1 - q0);
-            } else if (INTERP == RISA_GB_INTERP_NEAREST) {
-               int k = __float2int_rd(t + 0.5f);
-               k = min(max(k, 0), wlen - 1);
-               acc[g][r] += w[k];
-            } else {
-               // truncation toward zero of t + Dp/2 (texture variant, Backprojection.cu:294)
-               const float tt = t + cfg.trunc_offset;
-               int k = __float2int_rd(tt);
-               const int kg = k + s_w0[ai];
-               if (kg == -1 && tt != (float)k) k += 1;
-               k = min(max(k, 0), wlen - 1);
-               acc[g][r] += w[k];
+            for (int r = 0; r < PPT; ++r) {
+               const float t = tb + (float)r * bstep;
+               if (INTERP == RISA_GB_INTERP_LINEAR) {
+                  int k = __float2int_rd(t);
+                  k = min(max(k, 0), wlen - 2);
+                  const float f = t - (float)k;
+                  const float q0 = w[k], q1 = w[k + 1];
+                  acc[r] += q0 + f * (q1 - q0);
+               } else if (INTERP == RISA_GB_INTERP_NEAREST) {
+                  int k = __float2int_rd(t + 0.5f);
+                  k = min(max(k, 0), wlen - 1);
+                  acc[r] += w[k];
+               } else {
+                  // truncation toward zero of t + Dp/2 (texture variant, Backprojection.cu:294)
+                  const float tt = t + cfg.trunc_offset;
+                  int k = __float2int_rd(tt);
+                  const int kg = k + s_w0[ai];
+                  if (kg == -1 && tt != (float)k) k += 1;
+                  k = min(max(k, 0), wlen - 1);
+                  acc[r] += w[k];
+               }
             }
          }
-      };
-      if constexpr (G == 1) {
-#pragma unroll 4
-         for (int ai = 0; ai < na; ++ai) angle(ai, 0);
-      } else {
-         int ai = 0;
-         for (; ai + G <= na; ai += G) {
+         if (G > 1 && c0 + ai == end) {  // a group ends
 #pragma unroll
-            for (int u = 0; u < G; ++u) angle(ai + u, u);
+            for (int r = 0; r < PPT; ++r) {
+               sum[r] += acc[r];
+               acc[r] = 0.f;
+            }
+            end = angles.end(++g);
          }
-#pragma unroll
-         for (int u = 0; u < G - 1; ++u)
-            if (ai + u < na) angle(ai + u, u);
-      }
+      } while (G > 1 && ai < na);
       __syncthreads();
    }
 #pragma unroll
    for (int r = 0; r < PPT; ++r) {
       const int x = x0 + tx, y = y0 + ty + ROWS * r;
       if (x < N && y < N) {
-         float v = acc[0][r];
-#pragma unroll
-         for (int g = 1; g < G; ++g) v += acc[g][r];
-         v *= cfg.norm;
+         float v = (G > 1 ? sum[r] : acc[r]) * cfg.norm;
          if (cfg.masking) {
             const float dx = (float)x - c, dy = (float)y - c;
             if (dx * dx + dy * dy > lim) v = cfg.mask_value;
@@ -228,8 +245,8 @@ struct NearestVec<2> {
 };
 constexpr int kNearestAngles = 32;  // most angles per chunk
 template <int INTERP, int S, int G>
-__global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__ sino, float* __restrict__ img,
-                                                       BPCfg cfg, int wlen, int ach, int batch) {
+__device__ __forceinline__ void nearest_tile(const float* __restrict__ sino, float* __restrict__ img, const BPCfg& cfg,
+                                             int wlen, int ach, int batch) {
    using V = typename NearestVec<S>::T;
    extern __shared__ __align__(16) unsigned char smem_raw[];
    V* win = reinterpret_cast<V*>(smem_raw);  // [ach][wlen]
@@ -245,23 +262,23 @@ __global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__
       const float ny = fminf(fmaxf(c, (float)y0), (float)(y0 + 31)) - c;
       live = nx * nx + ny * ny <= lim;
    }
-   float acc[G][4][S];
+   float acc[4][S], sum[4][S];  // sum: the groups before this one
 #pragma unroll
-   for (int g = 0; g < G; ++g)
+   for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int r = 0; r < 4; ++r)
-#pragma unroll
-         for (int s = 0; s < S; ++s) acc[g][r][s] = 0.f;
+      for (int s = 0; s < S; ++s) acc[r][s] = sum[r][s] = 0.f;
    const size_t fs = (size_t)Pp * Dp;
    const float* q = sino + (size_t)s0 * fs;
    const int ns = min(S, batch - s0);
    constexpr uint32_t kFloorBits = 0x4B000000u;  // 2^23: floor(v) is in the low bits of v + 2^23 rounded down
    const uint32_t top = kFloorBits + (uint32_t)wlen - 1u;
 
+   const GroupedAngles<G> angles{Pp};
+   int g = 0, end = angles.end(0);  // the group at hand
    for (int c0 = 0; live && c0 < Pp; c0 += ach) {
       const int na = min(ach, Pp - c0);
       if (threadIdx.x < na) {
-         const int ang = c0 + threadIdx.x;
+         const int ang = angles.at(c0 + threadIdx.x);
          const float a = __ldg(cfg.a + ang), b = __ldg(cfg.b + ang);
          const double base = __ldg(cfg.t0 + ang) + (double)x0 * __ldg(cfg.ad + ang) +
                              (double)y0 * __ldg(cfg.bd + ang);
@@ -272,7 +289,7 @@ __global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__
       __syncthreads();
       for (int ai = ty; ai < na; ai += 8) {
          const int w0 = __float_as_int(s_ang[ai].w);
-         const float* row = q + (size_t)(c0 + ai) * Dp;
+         const float* row = q + (size_t)angles.at(c0 + ai) * Dp;
          for (int m = tx; m < wlen; m += 32) {
             const int k = w0 + m;
             const bool in = k >= 0 && k < Dp;
@@ -284,7 +301,7 @@ __global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__
          }
       }
       __syncthreads();
-      auto angle = [&](int ai, int g) {
+      auto angle = [&](int ai) {
          const float4 e = s_ang[ai];
          const float tb = fmaf((float)ty, e.y, fmaf((float)tx, e.x, e.z));
          const float bstep = 8.f * e.y;
@@ -300,26 +317,34 @@ __global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__
                 tt != fl - 8388608.f)
                k += 1u;
             const V u = w[min(k, top) - kFloorBits];
-            acc[g][r][0] += u.x;
-            acc[g][r][1] += u.y;
+            acc[r][0] += u.x;
+            acc[r][1] += u.y;
             if constexpr (S == 4) {
-               acc[g][r][2] += u.z;
-               acc[g][r][3] += u.w;
+               acc[r][2] += u.z;
+               acc[r][3] += u.w;
             }
          }
       };
       if constexpr (G == 1) {
 #pragma unroll 2
-         for (int ai = 0; ai < na; ++ai) angle(ai, 0);
+         for (int ai = 0; ai < na; ++ai) angle(ai);
       } else {
          int ai = 0;
-         for (; ai + G <= na; ai += G) {
+         do {  // the part of the chunk in each group
+            const int stop = min(na, end - c0);
+#pragma unroll 2
+            for (; ai < stop; ++ai) angle(ai);
+            if (c0 + ai == end) {  // a group ends
 #pragma unroll
-            for (int u = 0; u < G; ++u) angle(ai + u, u);
-         }
+               for (int r = 0; r < 4; ++r)
 #pragma unroll
-         for (int u = 0; u < G - 1; ++u)
-            if (ai + u < na) angle(ai + u, u);
+                  for (int s = 0; s < S; ++s) {
+                     sum[r][s] += acc[r][s];
+                     acc[r][s] = 0.f;
+                  }
+               end = angles.end(++g);
+            }
+         } while (ai < na);
       }
       __syncthreads();
    }
@@ -333,13 +358,21 @@ __global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__
          out = out || dx * dx + dy * dy > lim;
       }
 #pragma unroll
-      for (int s = 0; s < S; ++s) {
-         float v = acc[0][r][s];
-#pragma unroll
-         for (int g = 1; g < G; ++g) v += acc[g][r][s];
-         if (s < ns) img[((size_t)(s0 + s) * N + y) * N + x] = out ? cfg.mask_value : v * cfg.norm;
-      }
+      for (int s = 0; s < S; ++s)
+         if (s < ns)
+            img[((size_t)(s0 + s) * N + y) * N + x] = out ? cfg.mask_value : (G > 1 ? sum[r][s] : acc[r][s]) * cfg.norm;
    }
+}
+template <int INTERP, int S, int G>
+__global__ void __launch_bounds__(256) bp_nearest_tile(const float* __restrict__ sino, float* __restrict__ img, BPCfg cfg,
+                                                       int wlen, int ach, int batch) {
+   nearest_tile<INTERP, S, G>(sino, img, cfg, wlen, ach, batch);
+}
+// Four slices in groups: registers for four CTAs on an SM.
+template <int INTERP>
+__global__ void __launch_bounds__(256, 4) bp_nearest_tile_groups(const float* __restrict__ sino, float* __restrict__ img,
+                                                                 BPCfg cfg, int wlen, int ach, int batch) {
+   nearest_tile<INTERP, 4, kSplitGroups>(sino, img, cfg, wlen, ach, batch);
 }
 template <int INTERP, int S, int G>
 cudaError_t launch_nearest_tile_as(const float* sino, float* img, int batch, const BPCfg& cfg, cudaStream_t st) {
@@ -348,7 +381,9 @@ cudaError_t launch_nearest_tile_as(const float* sino, float* img, int batch, con
    // 30 slices: 412 us, 503 with 32)
    const int ach = cfg.scale <= 2.f ? kNearestAngles : kNearestAngles / 2;
    const size_t smem = sizeof(float) * S * (size_t)ach * wlen;
-   auto kern = bp_nearest_tile<INTERP, S, G>;
+   void (*kern)(const float*, float*, BPCfg, int, int, int);
+   if constexpr (S == 4 && G > 1) kern = bp_nearest_tile_groups<INTERP>;
+   else kern = bp_nearest_tile<INTERP, S, G>;
    if (smem > 47 * 1024) {
       cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
