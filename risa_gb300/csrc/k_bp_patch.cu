@@ -167,9 +167,9 @@ __device__ __forceinline__ void flip(u64 (&acc)[SQ][2][4], bool x, bool y) {
 // other slices have their pixels from the patches. A flagged slice at a time, one to
 // three pixels per thread, the windows of C angles in the copies' stages (16 rows of
 // 16-byte entries for every quad); all threads of the CTA, before the first copy (after
-// the last patch the call alone cost the finite CTAs 0.8%). 64 slices of 512^2 x 1024 angles 2.2 ms, with
-// one bad sample 3.3; 108 with every quad of the CTA
-// by scalar loads and FP64 coordinates, 3.5 with the flagged quad's four slices at once.
+// the last patch the call alone cost the finite CTAs 0.8%). 64 slices of 512^2 x 1024
+// angles 2.2 ms, with one bad sample 3.3; 108 with every quad of the CTA by scalar loads and
+// FP64 coordinates, 3.5 with the flagged quad's four slices at once.
 template <int Q, int NT>
 __device__ __noinline__ void patch_general_tile(const PatchArgs& g) {
    constexpr int C = Q == 1 ? 40 : 64, PX = (kTile * kTile + NT - 1) / NT;  // angles per chunk, pixels per thread
